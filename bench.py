@@ -718,10 +718,12 @@ def eigh_sizes(ctx, results):
 
 
 def panel_roofline(ctx, kst, sizes):
-    """Householder panel kernel: each reduced column reads its trailing
-    matrix once for p = A22 v, 8*(m-j-1)^2 bytes for an eigensolve of order
-    m; summed over the columns of every eigensolve of the timed region
-    (sizes) and divided by the panel kernel's total time there."""
+    """Householder reduction: each reduced column reads its trailing matrix
+    once for p = A22 v, 8*(m-j-1)^2 bytes for an eigensolve of order m; summed
+    over the columns of every eigensolve of the timed region (sizes) and
+    divided by the reduction kernels' total time there.  launches_expected
+    counts panels of 32 columns; a reduction that ends in shared memory or
+    registers (order 2048 and below) takes the rest in one launch."""
     st = kst["tridiag_panel"]
     if st["launches"] == 0 or not sizes:
         return None
@@ -732,7 +734,7 @@ def panel_roofline(ctx, kst, sizes):
     peak = peaks.get("hbm_gbs", 6650.0)
     ach = algo_total / (st["total_ms"] * 1e-3) / 1e9
     n = ctx.norbs
-    return {"kernel": "tridiag_panel (Householder panel: column updates, reflectors, p = A22 v)",
+    return {"kernel": "tridiag_panel, tridiag_grid, tridiag_cluster (Householder reduction: column updates, reflectors, p = A22 v)",
             "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
             "traffic": PANEL_DRAM_BYTES * (algo_total / st["launches"]) / PANEL_ALGO_BYTES_3072,
             "ms_per_launch": ms, "algorithmic_bytes": algo_total / st["launches"],

@@ -3,538 +3,32 @@
 // :53-121, cuda_wrappers.cu:469-505).
 //
 //   1. i*1e-10 added to diagonal element i of the packed input (the
-//      reference's parity-critical perturbation, eigenvectors_LAPACK.F90:53-55),
-//      then unpacked to a full column-major matrix.
-//   2. Householder tridiagonalisation, blocked: a cooperative kernel forms each
-//      panel of NB reflectors (three grid barriers per column: column update,
-//      reflector + symmetric matrix-vector product, correction), and the
-//      trailing matrix gets the rank-2*NB update A -= V W^T + W V^T as FP64 GEMM.
-//   3. Eigenvalues of the tridiagonal matrix by bisection on Sturm counts, one
-//      thread per eigenvalue.
+//      reference's parity-critical perturbation, eigenvectors_LAPACK.F90:53-55).
+//   2. Householder tridiagonalisation.  Up to order 608 and up to 2048 the
+//      matrix stays in the registers of one cluster or in the SMs' shared
+//      memory (tridiag.cu).  A larger one is first taken down to that size
+//      in panels (eigen_panel.cu): a cooperative kernel forms 32 reflectors (two
+//      grid barriers per column), and the trailing matrix gets the rank-64
+//      update A -= V W^T + W V^T as FP64 GEMM.
+//   3. Eigenvalues of the tridiagonal matrix by multisection on Sturm counts,
+//      one warp per eigenvalue.
 //   4. Eigenvectors of the tridiagonal matrix by inverse iteration with partial
 //      pivoting; eigenvalues closer than 1e-8 * ||T|| form clusters whose
 //      vectors are re-orthogonalised inside the iteration (one thread per
 //      cluster, members in order).
-//   5. Back-transformation C = Q Z with the compact WY form of each panel,
-//      Z -= V (T (V^T Z)), as FP64 GEMMs.
+//   5. Back-transformation C = Q Z: up to order 608 reflector by reflector with
+//      the vectors in registers, above with the compact WY form of 64
+//      reflectors, Z -= V (T (V^T Z)), as FP64 GEMMs (eigen_panel.cu).
 // Eigenvalues ascend; eigenvectors are the columns of C.
-#include <cooperative_groups.h>
-
+//
+// Whole eigensolve on the Fock matrix of a water lattice (ms, one B200),
+// against the blocked form of eigen_panel.cu: order 38 0.10 (0.57), 144 0.37
+// (2.15), 320 0.85 (4.6), 600 2.1 (9.4), 1026 6.8 (17.2), 1501 11.0 (26.6),
+// 2048 17.6 (39.0), 3072 48.7 (72.4).
+#include "eigen_ws.cuh"
 #include "mb_common.cuh"
 
-namespace cg = cooperative_groups;
-
 namespace {
-
-constexpr int NB = 32;         // panel width
-constexpr int TPB = 256;       // threads per CTA in the panel kernel
-constexpr int TCH = 16;        // row chunks per dot product in t1/t2
-
-struct PanelArgs {
-  int n, k, ib, lda;
-  double* a;
-  double* vp;      // n x NB, panel reflectors (v_j[j+1] = 1, zero above)
-  double* wp;      // n x NB
-  double* vall;    // n x n, all reflectors (column j holds v_j)
-  double* d;
-  double* e;
-  double* tau;
-  double* part;    // gridDim partial norms (column j)
-  double* partd;   // gridDim partial dots (w.v)
-  double* tvec;    // unused
-  double* tpart;   // 2*NB*TCH chunk partials of t1 = W^T v, t2 = V^T v
-  double* wvec;    // n
-};
-
-__device__ double block_sum(double v, double* sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) r += sh[i];
-  }
-  __syncthreads();
-  return r;  // valid in thread 0
-}
-
-// Sum of the gridDim.x per-CTA partials, computed by warp 0 of each CTA and
-// broadcast to the whole CTA (one load per lane per 32 partials).
-__device__ double grid_partials_sum(const double* part, double* sh_out) {
-  if (threadIdx.x < 32) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) s += part[b];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) *sh_out = s;
-  }
-  __syncthreads();
-  const double r = *sh_out;
-  __syncthreads();
-  return r;
-}
-
-__global__ void __launch_bounds__(TPB) tridiag_panel(PanelArgs p) {
-  // Two grid barriers per column.  For column j = k + i:
-  //   phase A  finish W(:, i-1) for the CTA's rows (w = tau (p - corr) + alpha v,
-  //            with w.v = tau (p.v - 2 t1.t2) so no extra reduction is needed),
-  //            update column j with the panel's earlier reflectors, partial
-  //            norm of A(j+2:n, j).                                   -> barrier
-  //   phase D  reflector, v, p = A22 v (one warp per row), partial p.v and the
-  //            chunked t1 = W^T v, t2 = V^T v.                        -> barrier
-  cg::grid_group grid = cg::this_grid();
-  __shared__ double sh[32];
-  __shared__ double s_scal[4];
-  __shared__ double s_sum;
-  __shared__ double s_vj[NB], s_wj[NB], s_t1[NB], s_t2[NB];
-  __shared__ double s_pv[TPB / 32];
-  const int n = p.n, lda = p.lda;
-  const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long gstride = (long long)gridDim.x * blockDim.x;
-  const int gwarp = (int)(gtid >> 5), nwarps = (int)(gstride >> 5), lane = threadIdx.x & 31;
-  double* A = p.a;
-#define AE(r, c) A[(long long)(c) * lda + (r)]
-#define VP(r, c) p.vp[(long long)(c) * n + (r)]
-#define WP(r, c) p.wp[(long long)(c) * n + (r)]
-  double prev_tau = 0.0;
-  for (int i = 0; i <= p.ib; ++i) {
-    const int j = p.k + i;
-    // ---------------- phase A
-    double alpha_prev = 0.0;
-    if (i > 0) {
-      const int il = i - 1;  // the column whose W is finished here
-      if (threadIdx.x < (unsigned)(2 * il)) {
-        const int dotq = threadIdx.x, l = dotq >> 1;
-        double t = 0.0;
-        for (int ch = 0; ch < TCH; ++ch) t += p.tpart[dotq * TCH + ch];
-        if ((dotq & 1) == 0) s_t1[l] = t; else s_t2[l] = t;
-      }
-      const double pv = grid_partials_sum(p.partd, &s_sum);  // also syncs s_t1/s_t2
-      double tt = 0.0;
-      for (int l = 0; l < il; ++l) tt += s_t1[l] * s_t2[l];
-      const double dot = prev_tau * (pv - 2.0 * tt);
-      alpha_prev = -0.5 * prev_tau * dot;
-      if (i == p.ib) {
-        // last column of the panel: finish W(:, il) and leave
-        for (long long r = gtid; r < n; r += gstride) {
-          if (r < j) continue;
-          double corr = 0.0;
-          for (int l = 0; l < il; ++l) corr += VP(r, l) * s_t1[l] + WP(r, l) * s_t2[l];
-          WP(r, il) = prev_tau * (p.wvec[r] - corr) + alpha_prev * VP(r, il);
-        }
-        break;
-      }
-      if (threadIdx.x == 0) {  // row j of W(:, il), needed by every CTA below
-        double corr = 0.0;
-        for (int l = 0; l < il; ++l) corr += VP(j, l) * s_t1[l] + WP(j, l) * s_t2[l];
-        s_wj[il] = prev_tau * (p.wvec[j] - corr) + alpha_prev * VP(j, il);
-      }
-    }
-    if (threadIdx.x < (unsigned)i) {
-      const int l = threadIdx.x;
-      s_vj[l] = VP(j, l);
-      if (l < i - 1) s_wj[l] = WP(j, l);
-    }
-    __syncthreads();
-    // Rows r >= j, eight lanes per row: lane q handles reflectors l = q, q+8, ...
-    // (independent loads), partial sums are combined with shuffles.  The group
-    // finishes W(r, i-1) and updates A(r, j); lane 0 accumulates the norm.
-    double sig = 0.0;
-    {
-      const int q = lane & 7;
-      const long long gstep = gstride >> 3;         // 8-lane groups in the grid
-      const long long gw0 = (gtid >> 5) << 2;       // first group of this warp
-      const int il = i - 1;
-      // the loop is warp-uniform (shuffles need every lane); each group checks
-      // its own row
-      for (long long base = j + gw0; base < n; base += gstep) {
-        const long long r = base + (lane >> 3);
-        const bool act = r < n;
-        if (i > 0) {
-          double corr = 0.0;
-          if (act)
-            for (int l = q; l < il; l += 8) corr += VP(r, l) * s_t1[l] + WP(r, l) * s_t2[l];
-          corr += __shfl_xor_sync(0xffffffffu, corr, 4);
-          corr += __shfl_xor_sync(0xffffffffu, corr, 2);
-          corr += __shfl_xor_sync(0xffffffffu, corr, 1);
-          const double wr_il = act ? prev_tau * (p.wvec[r] - corr) + alpha_prev * VP(r, il) : 0.0;
-          double upd = 0.0;
-          if (act)
-            for (int l = q; l < i; l += 8) {
-              const double wrl = (l == il) ? wr_il : WP(r, l);
-              upd += VP(r, l) * s_wj[l] + wrl * s_vj[l];
-            }
-          upd += __shfl_xor_sync(0xffffffffu, upd, 4);
-          upd += __shfl_xor_sync(0xffffffffu, upd, 2);
-          upd += __shfl_xor_sync(0xffffffffu, upd, 1);
-          if (act && q == 0) {
-            WP(r, il) = wr_il;
-            AE(r, j) = AE(r, j) - upd;
-          }
-        }
-        if (act && q == 0) {
-          if (r == j) p.d[j] = AE(j, j);
-          if (r >= j + 2) {
-            const double x = AE(r, j);
-            sig += x * x;
-          }
-        }
-      }
-    }
-    double bs = block_sum(sig, sh);
-    if (threadIdx.x == 0) p.part[blockIdx.x] = bs;
-    grid.sync();
-    // ---------------- phase D
-    const double snorm = grid_partials_sum(p.part, &s_sum);
-    if (threadIdx.x == 0) {
-      const double alpha = AE(j + 1, j);
-      double beta, tau, scal;
-      if (snorm == 0.0) {
-        beta = alpha; tau = 0.0; scal = 0.0;
-      } else {
-        beta = -copysign(sqrt(alpha * alpha + snorm), alpha);
-        tau = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
-      }
-      s_scal[0] = tau;
-      s_scal[1] = scal;
-      s_scal[2] = beta;
-    }
-    __syncthreads();
-    const double tau = s_scal[0], scal = s_scal[1];
-    if (gtid == 0) {
-      p.e[j] = s_scal[2];
-      p.tau[j] = tau;
-    }
-    for (long long r = gtid; r < n; r += gstride) {
-      const double v = (r == j + 1) ? 1.0 : (r > j + 1 ? AE(r, j) * scal : 0.0);
-      VP(r, i) = v;
-      p.vall[(long long)j * n + r] = v;
-    }
-    // p(r) = sum_{c > j} A(c, r) v(c), one warp per row r > j, eight loads in
-    // flight per lane; the warp also accumulates p(r) v(r) for p.v.
-    double pvw = 0.0;
-    {
-      const double* colj = A + (long long)j * lda;
-      for (int r = j + 1 + gwarp; r < n; r += nwarps) {
-        const double* colr = A + (long long)r * lda;
-        double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-        int c = j + 1 + lane;
-        for (; c + 224 < n; c += 256) {
-          double x[8], y[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) x[u] = __ldcs(colr + c + 32 * u);
-#pragma unroll
-          for (int u = 0; u < 8; ++u) y[u] = colj[c + 32 * u];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const double v = (c + 32 * u == j + 1) ? 1.0 : y[u] * scal;
-            if ((u & 3) == 0) acc0 += x[u] * v;
-            else if ((u & 3) == 1) acc1 += x[u] * v;
-            else if ((u & 3) == 2) acc2 += x[u] * v;
-            else acc3 += x[u] * v;
-          }
-        }
-        for (; c < n; c += 32) {
-          const double v = (c == j + 1) ? 1.0 : colj[c] * scal;
-          acc0 += colr[c] * v;
-        }
-        double acc = (acc0 + acc1) + (acc2 + acc3);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (lane == 0) {
-          p.wvec[r] = acc;
-          const double vr = (r == j + 1) ? 1.0 : colj[r] * scal;
-          pvw += acc * vr;
-        }
-      }
-      for (int r = gtid; r <= j && r < n; r += (int)gstride) p.wvec[r] = 0.0;
-    }
-    if (lane == 0) s_pv[threadIdx.x >> 5] = pvw;
-    // t1/t2 chunk partials (TCH row chunks per dot product)
-    {
-      const int rows = n - (j + 1);
-      const int chunk = (rows + TCH - 1) / TCH;
-      for (int q = nwarps - 1 - gwarp; q < 2 * i * TCH; q += nwarps) {
-        const int dotq = q / TCH, ch = q % TCH;
-        const int l = dotq >> 1;
-        const bool isw = (dotq & 1) == 0;
-        const double* col = isw ? p.wp + (long long)l * n : p.vp + (long long)l * n;
-        const int rb = j + 1 + ch * chunk, re = min(n, rb + chunk);
-        double acc = 0.0;
-        for (int r = rb + lane; r < re; r += 32) {
-          const double v = (r == j + 1) ? 1.0 : AE(r, j) * scal;
-          acc += col[r] * v;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (lane == 0) p.tpart[q] = acc;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_pv[w];
-      p.partd[blockIdx.x] = t;
-    }
-    prev_tau = tau;
-    grid.sync();
-  }
-#undef AE
-#undef VP
-#undef WP
-}
-
-// Second form of the panel kernel, used when every row of the matrix can own
-// an 8-lane group of the grid for the whole panel (n <= grid * TPB / 8).
-// Row r belongs to group r throughout, so the group keeps its own V(r, l) and
-// W(r, l) in registers (lane q holds l = q, q+8, q+16, q+24), prefetches
-// A(r, j+1) before the column's last barrier, and updates A(r, j) with no
-// global loads but p(r).  After each barrier the loads that remain (the
-// per-CTA partials, the broadcast row j, p(r)) are issued by different warps at
-// once.  The symmetric matrix-vector product gives each row 1, 2, 4 or 8
-// warps of one CTA as the trailing matrix shrinks, so late columns are not
-// bound by one warp's chain of loads.  Arithmetic per element follows the
-// first form, except that p(r) is summed in wpr column slices for wpr > 1.
-__global__ void __launch_bounds__(TPB) tridiag_panel2(PanelArgs p) {
-  cg::grid_group grid = cg::this_grid();
-  __shared__ double sh[32];
-  __shared__ double s_scal[4];
-  __shared__ double s_sum, s_alpha, s_wjr;
-  __shared__ double s_vj[NB], s_wj[NB], s_t1[NB], s_t2[NB];
-  __shared__ double s_pv[TPB / 32];
-  __shared__ double s_symv[TPB / 32];
-  __shared__ double s_gv[TPB / 8][NB], s_gw[TPB / 8][NB];  // V(r, l), W(r, l) of the CTA's rows
-  const int n = p.n, lda = p.lda;
-  const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long gstride = (long long)gridDim.x * blockDim.x;
-  const int gwarp = (int)(gtid >> 5), nwarps = (int)(gstride >> 5), lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5, q = lane & 7;
-  double* A = p.a;
-#define AE(r, c) A[(long long)(c) * lda + (r)]
-#define VP(r, c) p.vp[(long long)(c) * n + (r)]
-#define WP(r, c) p.wp[(long long)(c) * n + (r)]
-  const int r = (int)(gtid >> 3);  // the row this group owns
-  const bool own = r < n;
-  const int g = threadIdx.x >> 3;
-  double* gv = s_gv[g];
-  double* gw = s_gw[g];
-  double a_cur = (own && r >= p.k) ? AE(r, p.k) : 0.0;  // A(r, j) as the panel found it
-  double prev_tau = 0.0;
-  for (int i = 0; i <= p.ib; ++i) {
-    const int j = p.k + i;
-    const bool act = own && r >= j;
-    double anew = a_cur;
-    // ---------------- phase A
-    if (i > 0) {
-      const int il = i - 1;
-      double wv = act ? p.wvec[r] : 0.0;
-      if (wid == 0) {
-        double sacc = 0.0;
-        for (int b = lane; b < (int)gridDim.x; b += 32) sacc += p.partd[b];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sacc += __shfl_down_sync(0xffffffffu, sacc, o);
-        if (lane == 0) s_sum = sacc;
-      } else if (threadIdx.x >= 32 && threadIdx.x < (unsigned)(32 + 2 * il)) {
-        const int dotq = threadIdx.x - 32, l = dotq >> 1;
-        double t = 0.0;
-        for (int ch = 0; ch < TCH; ++ch) t += p.tpart[dotq * TCH + ch];
-        if ((dotq & 1) == 0) s_t1[l] = t; else s_t2[l] = t;
-      } else if (wid == TPB / 32 - 1) {
-        for (int l = lane; l < i; l += 32) {
-          s_vj[l] = VP(j, l);
-          if (l < il) s_wj[l] = WP(j, l);
-        }
-        if (lane == 0) s_wjr = p.wvec[j];
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double tt = 0.0;
-        for (int l = 0; l < il; ++l) tt += s_t1[l] * s_t2[l];
-        const double dot = prev_tau * (s_sum - 2.0 * tt);
-        const double ap = -0.5 * prev_tau * dot;
-        double corr = 0.0;
-        for (int l = 0; l < il; ++l) corr += s_vj[l] * s_t1[l] + s_wj[l] * s_t2[l];
-        s_wj[il] = prev_tau * (s_wjr - corr) + ap * s_vj[il];
-        s_scal[3] = ap;
-      }
-      __syncthreads();
-      const double alpha_prev = s_scal[3];
-      // W(r, il) from the group's registers
-      double corr = 0.0;
-      if (act)
-        for (int l = q; l < il; l += 8) corr += gv[l] * s_t1[l] + gw[l] * s_t2[l];
-      corr += __shfl_xor_sync(0xffffffffu, corr, 4);
-      corr += __shfl_xor_sync(0xffffffffu, corr, 2);
-      corr += __shfl_xor_sync(0xffffffffu, corr, 1);
-      const double wr_il = act ? prev_tau * (wv - corr) + alpha_prev * gv[il] : 0.0;
-      if (act && q == 0) WP(r, il) = wr_il;
-      if (i == p.ib) break;  // last column of the panel: W(:, il) was all that was left
-      double upd = 0.0;
-      if (act)
-        for (int l = q; l < i; l += 8) {
-          const double wrl = (l == il) ? wr_il : gw[l];
-          upd += gv[l] * s_wj[l] + wrl * s_vj[l];
-        }
-      __syncwarp();
-      if (q == (il & 7)) gw[il] = wr_il;
-      upd += __shfl_xor_sync(0xffffffffu, upd, 4);
-      upd += __shfl_xor_sync(0xffffffffu, upd, 2);
-      upd += __shfl_xor_sync(0xffffffffu, upd, 1);
-      anew = a_cur - upd;
-      if (act && q == 0) AE(r, j) = anew;
-    }
-    double sig = 0.0;
-    if (act && q == 0) {
-      if (r == j) p.d[j] = anew;
-      if (r >= j + 2) sig = anew * anew;
-    }
-    const double bs = block_sum(sig, sh);
-    if (threadIdx.x == 0) p.part[blockIdx.x] = bs;
-    grid.sync();
-    // ---------------- phase D
-    if (wid == 0) {
-      double sacc = 0.0;
-      for (int b = lane; b < (int)gridDim.x; b += 32) sacc += p.part[b];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sacc += __shfl_down_sync(0xffffffffu, sacc, o);
-      if (lane == 0) s_sum = sacc;
-    } else if (wid == 1 && lane == 0) {
-      s_alpha = AE(j + 1, j);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const double snorm = s_sum, alpha = s_alpha;
-      double beta, tau, scal;
-      if (snorm == 0.0) {
-        beta = alpha; tau = 0.0; scal = 0.0;
-      } else {
-        beta = -copysign(sqrt(alpha * alpha + snorm), alpha);
-        tau = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
-      }
-      s_scal[0] = tau;
-      s_scal[1] = scal;
-      s_scal[2] = beta;
-    }
-    __syncthreads();
-    const double tau = s_scal[0], scal = s_scal[1];
-    if (gtid == 0) {
-      p.e[j] = s_scal[2];
-      p.tau[j] = tau;
-    }
-    {
-      const double v = !own ? 0.0 : (r == j + 1 ? 1.0 : (r > j + 1 ? anew * scal : 0.0));
-      if (q == 0) {
-        gv[i] = v;
-        if (own) {
-          VP(r, i) = v;
-          p.vall[(long long)j * n + r] = v;
-        }
-      }
-    }
-    const double* colj = A + (long long)j * lda;
-    // p(r) = sum_{c > j} A(c, r) v(c) with wpr warps of one CTA per row
-    double pvw = 0.0;
-    {
-      const int R = n - j - 1;
-      int wpr = 1;
-      while (wpr < 8 && (long long)gridDim.x * (TPB / 32 / (wpr * 2)) >= R) wpr *= 2;
-      const int rpc = (TPB / 32) / wpr;
-      const int sub = wid % wpr;
-      const int rounds = (R + (int)gridDim.x * rpc - 1) / ((int)gridDim.x * rpc);
-      for (int t = 0; t < rounds; ++t) {
-        const int rho = (t * (int)gridDim.x + (int)blockIdx.x) * rpc + wid / wpr;
-        const int rr = j + 1 + rho;
-        double acc = 0.0;
-        if (rho < R) {
-          const double* colr = A + (long long)rr * lda;
-          double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-          const int step = 32 * wpr;
-          int c = j + 1 + lane + 32 * sub;
-          for (; c + 7 * step < n; c += 8 * step) {
-            double x[8], y[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) x[u] = __ldcs(colr + c + step * u);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) y[u] = colj[c + step * u];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const double v = (c + step * u == j + 1) ? 1.0 : y[u] * scal;
-              if ((u & 3) == 0) acc0 += x[u] * v;
-              else if ((u & 3) == 1) acc1 += x[u] * v;
-              else if ((u & 3) == 2) acc2 += x[u] * v;
-              else acc3 += x[u] * v;
-            }
-          }
-          for (; c < n; c += step) {
-            const double v = (c == j + 1) ? 1.0 : colj[c] * scal;
-            acc0 += colr[c] * v;
-          }
-          acc = (acc0 + acc1) + (acc2 + acc3);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (wpr > 1) {
-          if (lane == 0) s_symv[wid] = acc;
-          __syncthreads();
-          if (sub == 0 && lane == 0 && rho < R) {
-            double tot = 0.0;
-            for (int u = 0; u < wpr; ++u) tot += s_symv[wid + u];
-            acc = tot;
-          }
-          __syncthreads();
-        }
-        if (sub == 0 && lane == 0 && rho < R) {
-          p.wvec[rr] = acc;
-          const double vr = (rr == j + 1) ? 1.0 : colj[rr] * scal;
-          pvw += acc * vr;
-        }
-      }
-      for (int rz = (int)gtid; rz <= j && rz < n; rz += (int)gstride) p.wvec[rz] = 0.0;
-    }
-    if (lane == 0) s_pv[wid] = pvw;
-    // t1/t2 chunk partials (TCH row chunks per dot product)
-    {
-      const int rows = n - (j + 1);
-      const int chunk = (rows + TCH - 1) / TCH;
-      for (int qq = nwarps - 1 - gwarp; qq < 2 * i * TCH; qq += nwarps) {
-        const int dotq = qq / TCH, ch = qq % TCH;
-        const int l = dotq >> 1;
-        const bool isw = (dotq & 1) == 0;
-        const double* col = isw ? p.wp + (long long)l * n : p.vp + (long long)l * n;
-        const int rb = j + 1 + ch * chunk, re = min(n, rb + chunk);
-        double acc = 0.0;
-        for (int rw = rb + lane; rw < re; rw += 32) {
-          const double v = (rw == j + 1) ? 1.0 : AE(rw, j) * scal;
-          acc += col[rw] * v;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (lane == 0) p.tpart[qq] = acc;
-      }
-    }
-    // the next column of A for this row, in flight across the barrier
-    a_cur = (own && r >= j + 1 && i < p.ib) ? AE(r, j + 1) : 0.0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_pv[w];
-      p.partd[blockIdx.x] = t;
-    }
-    prev_tau = tau;
-    grid.sync();
-  }
-#undef AE
-#undef VP
-#undef WP
-}
-
-__global__ void copy_last_diag(int n, const double* a, int lda, double* d) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) d[n - 1] = a[(long long)(n - 1) * lda + (n - 1)];
-}
 
 // ---------------------------------------------------------------- bisection
 // 1/q from the hardware's approximate reciprocal refined by two Newton steps,
@@ -551,79 +45,125 @@ __device__ __forceinline__ double recip_nr2(double q) {
   return fma(r, e, r);
 }
 
-__device__ __forceinline__ int sturm_count(int n, const double* __restrict__ d, const double* __restrict__ e2,
-                                           double x, double pivmin) {
-  int cnt = 0;
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  cnt += q < 0.0;
-  // operands of eight rows are fetched ahead of the dependent recurrence
-  for (int i0 = 1; i0 < n; i0 += 8) {
-    double db[8], eb[8];
+// Sturm count (eigenvalues below x) from the leading principal minors'
+// three-term recurrence p_i = (d_i - x) p_(i-1) - e_(i-1)^2 p_(i-2): its
+// dependent chain is one multiply-add per row, against a reciprocal and four
+// for the quotients q_i = p_i / p_(i-1), and a change of sign from p_(i-1) to
+// p_i is a negative q_i.  Eight rows at a time, from a pair scaled by a power
+// of two to [1, 2); T has norm <= 1 here, so a row grows p at most threefold.
+// A block in which some |p_i| falls below kSturmTiny (a chain of tiny
+// couplings at one of its eigenvalues) is taken again by quotients, whose
+// pivots are bounded below by pivmin.  de[i] = (d_i, e_(i-1)^2), followed by
+// 2 SB records (2, 0): rows that keep the sign of p.
+constexpr int SB = 8;
+constexpr int kSturmTiny = 0x27100000;  // high word of 2^-398, about 1e-120
+constexpr double kPivmin = 1.0e-290;
+
+__device__ __forceinline__ int sturm_count(int n, const double2* __restrict__ de, double x) {
+  double p1 = de[0].x - x, p0 = 1.0;
+  if (fabs(p1) < kPivmin) p1 = -kPivmin;
+  int cnt = p1 < 0.0;
+  double2 nx[SB];  // the next block's rows
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u;
-      db[u] = i < n ? d[i] : 0.0;
-      eb[u] = i < n ? e2[i - 1] : 0.0;
-    }
+  for (int u = 0; u < SB; ++u) nx[u] = de[1 + u];
+  for (int i0 = 1; i0 < n; i0 += SB) {
+    double db[SB], eb[SB];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      if (i0 + u >= n) break;
-      q = db[u] - x - eb[u] * recip_nr2(q);
-      if (fabs(q) < pivmin) q = -pivmin;
-      cnt += q < 0.0;
+    for (int u = 0; u < SB; ++u) {
+      db[u] = nx[u].x - x;
+      eb[u] = nx[u].y;
+      nx[u] = de[i0 + SB + u];
     }
+    const int ex = max((__double2hiint(p0) >> 20) & 0x7ff, (__double2hiint(p1) >> 20) & 0x7ff);
+    const double sc = __hiloint2double((2046 - ex) << 20, 0);
+    p0 *= sc;
+    p1 *= sc;
+    const double s0 = p0, s1 = p1;
+    int c = 0, least = 0x7fffffff;  // high words of |p| order as |p| does
+#pragma unroll
+    for (int u = 0; u < SB; ++u) {
+      const double p2 = fma(db[u], p1, -(eb[u] * p0));
+      c += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+      least = min(least, __double2hiint(p2) & 0x7fffffff);
+      p0 = p1;
+      p1 = p2;
+    }
+    if (least < kSturmTiny) {
+      double q = s1 / s0;
+      if (fabs(q) < kPivmin) q = -kPivmin;
+      c = 0;
+      for (int u = 0; u < SB && i0 + u < n; ++u) {
+        q = db[u] - eb[u] * recip_nr2(q);
+        if (fabs(q) < kPivmin) q = -kPivmin;
+        c += q < 0.0;
+      }
+      p0 = 1.0;
+      p1 = q;  // the pair matters up to a factor only
+    }
+    cnt += c;
   }
   return cnt;
 }
 
-__global__ void tri_bounds(int n, const double* d, const double* e, double* e2, double* bnd) {
-  __shared__ double slo[1024], shi[1024], se[1024];
-  double lo = 1e300, hi = -1e300, em = 0.0;
+// T scaled by the power of two that brings its Gershgorin bound to (1/2, 1]
+// (exact unless an element underflows next to the norm), as the records de
+// and dv, and bnd = { lower bound, upper bound, unused, norm, 1 / scale }.
+__global__ void tri_bounds(int n, const double* __restrict__ d, const double* __restrict__ e,
+                           double2* __restrict__ de, double2* __restrict__ dv, double* __restrict__ bnd) {
+  __shared__ double slo[1024], shi[1024];
+  double lo = 1e300, hi = -1e300;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
     lo = fmin(lo, d[i] - r);
     hi = fmax(hi, d[i] + r);
-    if (i < n - 1) {
-      e2[i] = e[i] * e[i];
-      em = fmax(em, e2[i]);
-    }
   }
-  slo[threadIdx.x] = lo; shi[threadIdx.x] = hi; se[threadIdx.x] = em;
+  slo[threadIdx.x] = lo; shi[threadIdx.x] = hi;
   __syncthreads();
   for (int s = blockDim.x / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) {
       slo[threadIdx.x] = fmin(slo[threadIdx.x], slo[threadIdx.x + s]);
       shi[threadIdx.x] = fmax(shi[threadIdx.x], shi[threadIdx.x + s]);
-      se[threadIdx.x] = fmax(se[threadIdx.x], se[threadIdx.x + s]);
     }
     __syncthreads();
   }
+  const double norm = fmax(fabs(slo[0]), fabs(shi[0]));
+  // 2^-k with norm 2^-k in (1/2, 1]; k clamped so that 2^k and 2^-k are normal
+  int k = 0;
+  if (norm > 0.0 && norm < 1e300) frexp(norm, &k);
+  k = max(-1000, min(1000, k));
+  const double sc = ldexp(1.0, -k);
   if (threadIdx.x == 0) {
-    double tnorm = fmax(fabs(slo[0]), fabs(shi[0]));
-    double pad = 2.0 * 2.220446049250313e-16 * tnorm * n + 1e-300;
-    bnd[0] = slo[0] - pad;
-    bnd[1] = shi[0] + pad;
-    bnd[2] = fmax(1e-290, 2.2250738585072014e-308 * fmax(1.0, se[0]));  // pivmin
+    const double tnorm = norm * sc;
+    const double pad = 2.0 * 2.220446049250313e-16 * tnorm * n + 1e-300;
+    bnd[0] = slo[0] * sc - pad;
+    bnd[1] = shi[0] * sc + pad;
+    bnd[2] = 0.0;
     bnd[3] = tnorm;
+    bnd[4] = ldexp(1.0, k);
   }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double f = i > 0 ? e[i - 1] * sc : 0.0;
+    de[i] = make_double2(d[i] * sc, f * f);
+    dv[i] = make_double2(d[i] * sc, i < n - 1 ? e[i] * sc : 0.0);
+  }
+  if (threadIdx.x < 2 * SB) de[n + threadIdx.x] = make_double2(2.0, 0.0);
 }
 
 // One warp per eigenvalue: each pass the 32 lanes evaluate Sturm counts at 32
 // interior points of the bracket, shrinking it 33-fold (about a dozen passes
-// instead of ~60 bisection steps, with 32x the parallelism).
-__global__ void bisect_kernel(int n, const double* __restrict__ d, const double* __restrict__ e2,
-                              const double* __restrict__ bnd, double* __restrict__ w) {
+// instead of ~60 bisection steps, with 32x the parallelism).  ws receives the
+// eigenvalues of the scaled T, w those of T.
+__global__ void bisect_kernel(int n, const double2* __restrict__ de, const double* __restrict__ bnd,
+                              double* __restrict__ ws, double* __restrict__ w) {
   const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (m >= n) return;
   double lo = bnd[0], hi = bnd[1];
-  const double pivmin = bnd[2];
   const double eps = 2.220446049250313e-16;
   for (int it = 0; it < 64; ++it) {
-    if (hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + pivmin) break;
+    if (hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + kPivmin) break;
     const double x = lo + (hi - lo) * ((double)(lane + 1) / 33.0);
-    const int cnt = sturm_count(n, d, e2, x, pivmin);
+    const int cnt = sturm_count(n, de, x);
     const unsigned above = __ballot_sync(0xffffffffu, cnt > m);  // lanes whose point lies above eigenvalue m
     double nlo = lo, nhi = hi;
     if (above == 0u) {
@@ -637,100 +177,158 @@ __global__ void bisect_kernel(int n, const double* __restrict__ d, const double*
     lo = nlo;
     hi = nhi;
   }
-  if (lane == 0) w[m] = 0.5 * (lo + hi);
+  if (lane == 0) {
+    const double x = 0.5 * (lo + hi);
+    ws[m] = x;
+    w[m] = x * bnd[4];
+  }
 }
 
 // --------------------------------------------------------- inverse iteration
-// LU with partial pivoting of T - lam I and solve, in place on x (stride ld).
-// u0/u1/u2 (stride ld) receive the U factor; pivots are re-derived per solve.
-// Both sweeps fetch eight rows of operands ahead of the dependent chain, so
-// the chain waits on arithmetic, not on one L2 round trip per row.
-__device__ void tri_solve(int n, const double* __restrict__ d, const double* __restrict__ e, double lam,
-                          double tiny, double* u0, double* u1, double* u2, double* x, long long ld) {
-  constexpr int B = 8;
-  // factorisation and forward substitution in one pass
-  double dd = d[0] - lam;          // current pivot row diagonal
-  double du = n > 1 ? e[0] : 0.0;  // current pivot row super-diagonal
-  double du2 = 0.0;
-  double xr = x[0];
-  for (int i0 = 0; i0 < n - 1; i0 += B) {
-    double sb[B], dnb[B], enb[B], xnb[B];
+// LU with partial pivoting of T - lam I for one vector per thread, every array
+// with stride ld.  Row i of the factor: the reciprocal of the pivot, the two
+// elements above it, the multiplier and whether rows i and i + 1 changed
+// places; later solves of the same vector reuse it.
+struct TriLu {
+  double *rp, *u1, *u2, *l;
+  unsigned char* sw;
+  long long ld;
+};
+
+// Forward substitution of x (in place) with the stored factor, or (FACTOR)
+// while forming it; x(i) * scale is what the sweep reads.  FACTOR reads the
+// start vector from the generator state instead.  Every sweep fetches the
+// operands of the next eight rows while eight pass through the dependent
+// chain.  dv[i] = (d_i, e_i).
+constexpr int TB = 8;
+
+template <bool FACTOR>
+__device__ __forceinline__ void tri_forward(int n, const double2* __restrict__ dv, double lam, double tiny,
+                                            const TriLu& f, double* x, double scale, unsigned long long seed) {
+  const long long ld = f.ld;
+  unsigned long long s = seed;
+  auto rnd = [&]() {
+    s ^= s >> 31; s *= 0x94D049BB133111EBull; s ^= s >> 29;
+    return ((double)(s >> 11) * (1.0 / 9007199254740992.0)) - 0.5;
+  };
+  double dd = 0.0, du = 0.0, sub = 0.0, xr;
+  double2 tn[TB];
+  double xn[TB], ln[TB];
+  unsigned char wn[TB];
+  auto fetch = [&](int i0) {
 #pragma unroll
-    for (int u = 0; u < B; ++u) {
+    for (int u = 0; u < TB; ++u) {
+      const int i = min(i0 + u, n - 2);
+      if (FACTOR) {
+        tn[u] = dv[i + 1];
+      } else {
+        xn[u] = x[(long long)(i + 1) * ld];
+        ln[u] = f.l[(long long)i * ld];
+        wn[u] = f.sw[(long long)i * ld];
+      }
+    }
+  };
+  if (FACTOR) {
+    const double2 t = dv[0];
+    dd = t.x - lam;
+    du = sub = n > 1 ? t.y : 0.0;
+    xr = rnd();
+  } else {
+    xr = x[0] * scale;
+  }
+  if (n > 1) fetch(0);
+  for (int i0 = 0; i0 < n - 1; i0 += TB) {
+    double2 tb[TB];
+    double xb[TB], lb[TB];
+    unsigned char wb[TB];
+#pragma unroll
+    for (int u = 0; u < TB; ++u) {
+      tb[u] = tn[u];
+      xb[u] = xn[u] * scale;
+      lb[u] = ln[u];
+      wb[u] = wn[u];
+    }
+    if (i0 + TB < n - 1) fetch(i0 + TB);
+#pragma unroll
+    for (int u = 0; u < TB; ++u) {
       const int i = i0 + u;
       if (i < n - 1) {
-        sb[u] = e[i];
-        dnb[u] = d[i + 1];
-        enb[u] = (i + 1 < n - 1) ? e[i + 1] : 0.0;
-        xnb[u] = x[(long long)(i + 1) * ld];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < B; ++u) {
-      const int i = i0 + u;
-      if (i >= n - 1) break;
-      const double sub = sb[u];          // T(i+1, i)
-      const double dn = dnb[u] - lam;    // T(i+1, i+1)
-      const double en = enb[u];
-      const double xn = xnb[u];
-      if (fabs(dd) >= fabs(sub)) {
-        // no interchange
-        double piv_ = dd;
-        if (fabs(piv_) < tiny) piv_ = copysign(tiny, piv_ == 0.0 ? 1.0 : piv_);
-        const double l = sub / piv_;
-        u0[(long long)i * ld] = piv_;
-        u1[(long long)i * ld] = du;
-        u2[(long long)i * ld] = du2;
-        x[(long long)i * ld] = xr;
-        dd = dn - l * du;
-        du = en;
-        du2 = 0.0;
-        xr = xn - l * xr;
-      } else {
-        // interchange rows i and i+1
-        const double l = dd / sub;
-        u0[(long long)i * ld] = sub;
-        u1[(long long)i * ld] = dn;
-        u2[(long long)i * ld] = en;
-        x[(long long)i * ld] = xn;
-        const double ndd = du - l * dn;
-        const double ndu = -l * en;
-        dd = ndd;
-        du = ndu;
-        du2 = 0.0;
-        xr = xr - l * xn;
+        const long long o = (long long)i * ld;
+        if (FACTOR) {
+          const double dn = tb[u].x - lam, en = i + 1 < n - 1 ? tb[u].y : 0.0, xv = rnd();
+          const bool swap = fabs(dd) < fabs(sub);
+          const double piv = fabs(dd) < tiny ? copysign(tiny, dd) : dd;
+          const double rd = recip_nr2(piv), rs = recip_nr2(swap ? sub : 1.0);
+          const double l = swap ? dd * rs : sub * rd;
+          f.rp[o] = swap ? rs : rd;
+          f.u1[o] = swap ? dn : du;
+          f.u2[o] = swap ? en : 0.0;
+          f.l[o] = l;
+          f.sw[o] = swap;
+          x[o] = swap ? xv : xr;
+          dd = swap ? fma(-l, dn, du) : fma(-l, du, dn);
+          du = swap ? -l * en : en;
+          xr = swap ? fma(-l, xv, xr) : fma(-l, xr, xv);
+          sub = en;
+        } else {
+          x[o] = wb[u] ? xb[u] : xr;
+          xr = wb[u] ? fma(-lb[u], xb[u], xr) : fma(-lb[u], xr, xb[u]);
+        }
       }
     }
   }
-  double last = dd;
-  if (fabs(last) < tiny) last = copysign(tiny, last == 0.0 ? 1.0 : last);
-  u0[(long long)(n - 1) * ld] = last;
-  // back substitution
-  double x1 = xr / last;  // x[n-1]
-  x[(long long)(n - 1) * ld] = x1;
-  double x2 = 0.0;        // x[i+2]
-  for (int i0 = n - 2; i0 >= 0; i0 -= B) {
-    double xb[B], a0[B], a1[B], a2[B];
+  x[(long long)(n - 1) * ld] = xr;
+  if (FACTOR) {
+    const double piv = fabs(dd) < tiny ? copysign(tiny, dd) : dd;
+    f.rp[(long long)(n - 1) * ld] = recip_nr2(piv);
+    f.u1[(long long)(n - 1) * ld] = 0.0;
+    f.u2[(long long)(n - 1) * ld] = 0.0;
+  }
+}
+
+// Back substitution in place; max |x| and the sum of squares.  |x| stays below
+// n / eps for a right-hand side of magnitude 1, so the squares cannot overflow.
+__device__ __forceinline__ double tri_back(int n, const TriLu& f, double* x, double* sumsq) {
+  const long long ld = f.ld;
+  double x1 = 0.0, x2 = 0.0, mx = 0.0, s0 = 0.0, s1 = 0.0;
+  double xb[TB], rb[TB], a1[TB], a2[TB];
+  auto fetch = [&](int i0) {
 #pragma unroll
-    for (int u = 0; u < B; ++u) {
+    for (int u = 0; u < TB; ++u) {
+      const long long o = (long long)max(i0 - u, 0) * ld;
+      xb[u] = x[o];
+      rb[u] = f.rp[o];
+      a1[u] = f.u1[o];
+      a2[u] = f.u2[o];
+    }
+  };
+  fetch(n - 1);
+  for (int i0 = n - 1; i0 >= 0; i0 -= TB) {
+    double cx[TB], cr[TB], c1[TB], c2[TB];
+#pragma unroll
+    for (int u = 0; u < TB; ++u) {
+      cx[u] = xb[u];
+      cr[u] = rb[u];
+      c1[u] = a1[u];
+      c2[u] = a2[u];
+    }
+    if (i0 - TB >= 0) fetch(i0 - TB);
+#pragma unroll
+    for (int u = 0; u < TB; ++u) {
       const int i = i0 - u;
       if (i >= 0) {
-        xb[u] = x[(long long)i * ld];
-        a0[u] = u0[(long long)i * ld];
-        a1[u] = u1[(long long)i * ld];
-        a2[u] = u2[(long long)i * ld];
+        const double v = fma(-c1[u], x1, fma(-c2[u], x2, cx[u])) * cr[u];
+        x[(long long)i * ld] = v;
+        mx = fmax(mx, fabs(v));
+        if (u & 1) s1 = fma(v, v, s1);
+        else s0 = fma(v, v, s0);
+        x2 = x1;
+        x1 = v;
       }
     }
-#pragma unroll
-    for (int u = 0; u < B; ++u) {
-      const int i = i0 - u;
-      if (i < 0) break;
-      const double v = (xb[u] - a1[u] * x1 - a2[u] * x2) / a0[u];
-      x[(long long)i * ld] = v;
-      x2 = x1;
-      x1 = v;
-    }
   }
+  *sumsq = s0 + s1;
+  return mx;
 }
 
 // x (stride ld) normalised to unit 2-norm; returns the norm before scaling.
@@ -771,11 +369,11 @@ __device__ double normalise(int n, double* x, long long ld) {
 }
 
 // One thread per cluster start; X is n x n with X[i*n + m] = component i of
-// vector m (so consecutive threads touch consecutive addresses).
-__global__ void inverse_iteration(int n, const double* __restrict__ d, const double* __restrict__ e,
-                                  const double* __restrict__ w, const double* __restrict__ bnd,
-                                  double* __restrict__ X, double* __restrict__ U0, double* __restrict__ U1,
-                                  double* __restrict__ U2, int* status) {
+// vector m (so consecutive threads touch consecutive addresses), still to be
+// multiplied by inv[m].  T and w are scaled to norm <= 1.
+__global__ void inverse_iteration(int n, const double2* __restrict__ dv, const double* __restrict__ w,
+                                  const double* __restrict__ bnd, double* __restrict__ X, double* __restrict__ inv,
+                                  TriLu lu, int* status) {
   const int m0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (m0 >= n) return;
   const double tnorm = bnd[3];
@@ -784,11 +382,9 @@ __global__ void inverse_iteration(int n, const double* __restrict__ d, const dou
   int m1 = m0 + 1;
   while (m1 < n && !(w[m1] - w[m1 - 1] > ortol)) ++m1;
   const double eps = 2.220446049250313e-16;
-  const double tiny = eps * fmax(tnorm, 1e-300);
+  const double tiny = eps * fmax(tnorm, 1e-290);
   const long long ld = n;
-  double* u0 = U0 + m0;
-  double* u1 = U1 + m0;
-  double* u2 = U2 + m0;
+  const TriLu f{lu.rp + m0, lu.u1 + m0, lu.u2 + m0, lu.l + m0, lu.sw + m0, ld};
   double lam_prev = 0.0;
   for (int m = m0; m < m1; ++m) {
     double lam = w[m];
@@ -798,16 +394,21 @@ __global__ void inverse_iteration(int n, const double* __restrict__ d, const dou
     }
     lam_prev = lam;
     double* x = X + m;
-    // deterministic start vector
-    unsigned long long s = 0x9E3779B97F4A7C15ull ^ (unsigned long long)(m + 1) * 0xBF58476D1CE4E5B9ull;
-    for (int i = 0; i < n; ++i) {
-      s ^= s >> 31; s *= 0x94D049BB133111EBull; s ^= s >> 29;
-      x[(long long)i * ld] = ((double)(s >> 11) * (1.0 / 9007199254740992.0)) - 0.5;
-    }
-    normalise(n, x, ld);
+    // deterministic start vector, generated inside the first forward sweep
+    const unsigned long long seed = 0x9E3779B97F4A7C15ull ^ (unsigned long long)(m + 1) * 0xBF58476D1CE4E5B9ull;
     const int nits = (m1 - m0 > 1) ? 4 : 2;
+    double scale = 1.0;
     for (int it = 0; it < nits; ++it) {
-      tri_solve(n, d, e, lam, tiny, u0, u1, u2, x, ld);
+      if (it == 0) tri_forward<true>(n, dv, lam, tiny, f, x, 1.0, seed);
+      else tri_forward<false>(n, dv, lam, tiny, f, x, scale, 0);
+      double sq;
+      const double mx = tri_back(n, f, x, &sq);
+      if (!(mx > 0.0) || !isfinite(sq)) { atomicExch(status, MB_ERR_NUMERIC); return; }
+      if (m1 - m0 == 1) {
+        scale = 1.0 / mx;
+        inv[m] = 1.0 / sqrt(sq);
+        continue;
+      }
       // re-orthogonalise against earlier members of the cluster (MGS)
       for (int q = m0; q < m; ++q) {
         const double* y = X + q;
@@ -815,15 +416,125 @@ __global__ void inverse_iteration(int n, const double* __restrict__ d, const dou
         for (int i = 0; i < n; ++i) dt += y[(long long)i * ld] * x[(long long)i * ld];
         for (int i = 0; i < n; ++i) x[(long long)i * ld] -= dt * y[(long long)i * ld];
       }
-      double nr = normalise(n, x, ld);
+      const double nr = normalise(n, x, ld);
       if (!(nr > 0.0) || !isfinite(nr)) { atomicExch(status, MB_ERR_NUMERIC); return; }
+      inv[m] = 1.0;
     }
   }
 }
 
-// Z (column-major n x n) = X^T in the X[i*n + m] layout, i.e. plain copy with
-// swapped meaning: Z(i, m) = X[i*n + m].
-__global__ void transpose_kernel(int n, const double* __restrict__ X, double* __restrict__ Z) {
+// Back-transformation of a small matrix, one reflector at a time: a warp keeps
+// two vectors in registers (lane l rows l, l + 32, ...) and applies
+// H_j = I - tau_j v_j v_j^T for j = n - 2 .. 0.  The reflectors pass through a
+// ring of shared-memory stages of BS_REF columns, which the CTA's warps share;
+// vectors are independent, so nothing else is exchanged.  X[i*n + m] =
+// component i of vector m before its normalisation inv[m]; c column-major.
+constexpr int BS_T = 128, BS_REF = 4, BS_STAGES = 4;
+
+template <int K>
+__global__ void __launch_bounds__(BS_T) back_small(int n, const double* __restrict__ V, const double* __restrict__ tau,
+                                                   const double* __restrict__ X, const double* __restrict__ inv,
+                                                   double* __restrict__ c) {
+  extern __shared__ double ring[];  // BS_STAGES x BS_REF x (32 K)
+  __shared__ double s_tau[32 * K];
+  constexpr int LD = 32 * K;
+  const int lane = threadIdx.x & 31;
+  const int m0 = 2 * (blockIdx.x * (BS_T / 32) + (threadIdx.x >> 5));
+  const bool act = m0 < n;
+  const int m1 = m0 + 1 < n ? m0 + 1 : m0;
+  double za[K], zb[K];
+  const double ia = act ? inv[m0] : 0.0, ib = act ? inv[m1] : 0.0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int r = lane + 32 * k;
+    za[k] = act && r < n ? X[(long long)r * n + m0] * ia : 0.0;
+    zb[k] = act && r < n ? X[(long long)r * n + m1] * ib : 0.0;
+  }
+  for (int i = threadIdx.x; i < n - 1; i += BS_T) s_tau[i] = tau[i];
+  for (int i = threadIdx.x; i < BS_STAGES * BS_REF * LD; i += BS_T) ring[i] = 0.0;
+  __syncthreads();
+  const int nref = n - 1, nst = (nref + BS_REF - 1) / BS_REF;
+  auto fetch = [&](int t) {  // stage t: reflectors nref - 1 - BS_REF t, descending
+    if (t < nst)
+      for (int u = 0; u < BS_REF; ++u) {
+        const int j = nref - 1 - BS_REF * t - u;
+        if (j < 0) break;
+        double* dst = ring + ((size_t)(t % BS_STAGES) * BS_REF + u) * LD;
+        for (int r = threadIdx.x; r < n; r += BS_T) {
+          const unsigned sa = (unsigned)__cvta_generic_to_shared(dst + r);
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(V + (long long)j * n + r) : "memory");
+        }
+      }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  for (int t = 0; t < BS_STAGES - 1; ++t) fetch(t);
+  for (int t = 0; t < nst; ++t) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(BS_STAGES - 2) : "memory");
+    __syncthreads();           // stage t has landed; every warp has left stage t - 1
+    fetch(t + BS_STAGES - 1);
+#pragma unroll 1
+    for (int u = 0; u < BS_REF; ++u) {
+      const int j = nref - 1 - BS_REF * t - u;
+      if (j < 0) break;
+      const double* v = ring + ((size_t)(t % BS_STAGES) * BS_REF + u) * LD + lane;
+      const int k0 = (j + 1) >> 5;
+      double vr[K], sa = 0.0, sb = 0.0, sa1 = 0.0, sb1 = 0.0;
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (k >= k0) {
+          vr[k] = v[32 * k];
+          if (k & 1) {
+            sa1 = fma(vr[k], za[k], sa1);
+            sb1 = fma(vr[k], zb[k], sb1);
+          } else {
+            sa = fma(vr[k], za[k], sa);
+            sb = fma(vr[k], zb[k], sb);
+          }
+        }
+      sa += sa1;
+      sb += sb1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        sa += __shfl_xor_sync(0xffffffffu, sa, o);
+        sb += __shfl_xor_sync(0xffffffffu, sb, o);
+      }
+      const double t0 = -s_tau[j];
+      sa *= t0;
+      sb *= t0;
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (k >= k0) {
+          za[k] = fma(sa, vr[k], za[k]);
+          zb[k] = fma(sb, vr[k], zb[k]);
+        }
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  if (!act) return;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int r = lane + 32 * k;
+    if (r < n) {
+      c[(long long)m0 * n + r] = za[k];
+      if (m1 != m0) c[(long long)m1 * n + r] = zb[k];
+    }
+  }
+}
+
+template <int K>
+int launch_back_small(int n, const double* V, const double* tau, const double* X, const double* inv, double* c,
+                      cudaStream_t stream) {
+  const size_t smem = sizeof(double) * BS_STAGES * BS_REF * 32 * K;
+  MB_CUDA(cudaFuncSetAttribute(back_small<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int per = 2 * (BS_T / 32);
+  back_small<K><<<(n + per - 1) / per, BS_T, smem, stream>>>(n, V, tau, X, inv, c);
+  MB_LAUNCH_CHECK();
+  return MB_OK;
+}
+
+// Z (column-major n x n): Z(i, m) = X[i*n + m] * inv[m].
+__global__ void transpose_kernel(int n, const double* __restrict__ X, const double* __restrict__ inv,
+                                 double* __restrict__ Z) {
   __shared__ double t[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   // X viewed as row-major [i][m]: tile rows i = by.., cols m = bx..
@@ -835,211 +546,71 @@ __global__ void transpose_kernel(int n, const double* __restrict__ X, double* __
   // Z column-major: Z(i, m) at m*n + i; write with i fastest
   for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
     int m = bx + yy, i = by + threadIdx.x;
-    if (i < n && m < n) Z[(long long)m * n + i] = t[threadIdx.x][yy];
-  }
-}
-
-// T factor of a block of reflectors (dlarft, forward columnwise):
-// T(i,i) = tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) S(0:i, i) with S = V^T V.
-// S and T both live in (dynamic) shared memory.
-constexpr int BT = 64;  // reflectors per back-transformation block
-constexpr size_t LARFT_SMEM = sizeof(double) * 2 * BT * (BT + 1);
-
-// One CTA per block of reflectors: block b holds reflectors k = b*BT ..
-// k+ib-1 of nref, S and T at b*BT*BT.
-__global__ void larft_kernel(int nref, const double* __restrict__ Sall, const double* __restrict__ tau_all,
-                             double* __restrict__ Tall) {
-  extern __shared__ double larft_sh[];
-  const int k = blockIdx.x * BT;
-  const int ib = (BT < nref - k) ? BT : nref - k;
-  if (ib <= 0) return;
-  const double* S = Sall + (size_t)blockIdx.x * BT * BT;
-  const double* tau = tau_all + k;
-  double* T = Tall + (size_t)blockIdx.x * BT * BT;
-  double(*st)[BT + 1] = reinterpret_cast<double(*)[BT + 1]>(larft_sh);
-  double(*ss)[BT + 1] = reinterpret_cast<double(*)[BT + 1]>(larft_sh + BT * (BT + 1));
-  for (int q = threadIdx.x; q < ib * ib; q += blockDim.x) {
-    const int r = q % ib, c = q / ib;
-    ss[r][c] = S[(long long)c * ib + r];
-    st[r][c] = 0.0;
-  }
-  __syncthreads();
-  for (int i = 0; i < ib; ++i) {
-    if (threadIdx.x < (unsigned)i) {
-      const int r = threadIdx.x;
-      double acc = 0.0;
-      for (int c = r; c < i; ++c) acc += st[r][c] * ss[c][i];
-      st[r][i] = -tau[i] * acc;
-    }
-    if (threadIdx.x == 0) st[i][i] = tau[i];
-    __syncthreads();
-  }
-  for (int q = threadIdx.x; q < ib * ib; q += blockDim.x) {
-    const int r = q % ib, c = q / ib;
-    T[(long long)c * ib + r] = st[r][c];
+    if (i < n && m < n) Z[(long long)m * n + i] = t[threadIdx.x][yy] * inv[m];
   }
 }
 
 }  // namespace
 
-extern "C" int mb_unpack_dev(int n, const double* pk, double* a, int lda, int perturb, double* pk_mut,
-                             cudaStream_t stream);
-extern "C" int mb_dgemm_ws(char transa, char transb, int m, int n, int k, double alpha, const double* a, int lda,
-                           const double* b, int ldb, double beta, double* c, int ldc, double* ws, size_t ws_elems,
-                           cudaStream_t stream);
-
-// Workspace: A n*n | V n*n | Z n*n | X n*n | U0,U1,U2 3*n*n | vp,wp 2*n*NB |
-// d,e,e2,tau,wvec 5n | small scratch
-extern "C" size_t mb_eigh_ws_bytes(int n) {
-  size_t nn = (size_t)n * n;
-  return sizeof(double) * (7 * nn + 3 * (size_t)n * NB + 5 * (size_t)n + 2 * NB + 2 * NB * TCH + 4096 +
-                           (size_t)BT * BT * 2 * (size_t)((n + BT - 1) / BT) +
-                           (size_t)BT * n) + 256;
-}
+extern "C" size_t mb_eigh_ws_bytes(int n) { return sizeof(double) * eigh::ws_doubles(n) + 256; }
 
 extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
                           cudaStream_t stream) {
   const size_t nn = (size_t)n * n;
-  double* b = (double*)ws;
-  double* A = b; b += nn;
-  double* V = b; b += nn;
-  double* Z = b; b += nn;
-  double* X = b; b += nn;
-  double* U0 = b; b += nn;
-  double* U1 = b; b += nn;
-  double* U2 = b; b += nn;
-  double* vwv = b; b += (size_t)n * 3 * NB;  // [V | W | V] panel columns
-  double* vp = vwv;
-  double* wp = vwv + (size_t)n * NB;
-  double* d = b; b += n;
-  double* e = b; b += n;
-  double* e2 = b; b += n;
-  double* tau = b; b += n;
-  double* wvec = b; b += n;
-  double* tvec = b; b += 2 * NB;
-  double* tpart = b; b += 2 * NB * TCH;
-  double* part = b; b += 4096;
-  const int nblk_bt = (n + BT - 1) / BT;
-  double* S = b; b += (size_t)BT * BT * nblk_bt;   // S_b = V_b^T V_b of every back-transformation block
-  double* Tm = b; b += (size_t)BT * BT * nblk_bt;  // their T factors
-  double* Y = b; b += (size_t)BT * n;
-  double* bnd = part + 2048;
-
+  const eigh::Ws w = eigh::carve(n, ws);
   MB_CUDA(cudaMemsetAsync(status_dev, 0, sizeof(int), stream));
   if (n == 1) {
-    MB_TRY(mb_unpack_dev(1, fpacked, A, 1, perturb, fpacked, stream));
-    MB_CUDA(cudaMemcpyAsync(eigs, A, sizeof(double), cudaMemcpyDeviceToDevice, stream));
+    MB_TRY(mb_unpack_dev(1, fpacked, w.A, 1, perturb, fpacked, stream));
+    MB_CUDA(cudaMemcpyAsync(eigs, w.A, sizeof(double), cudaMemcpyDeviceToDevice, stream));
     const double one = 1.0;
     MB_CUDA(cudaMemcpyAsync(c, &one, sizeof(double), cudaMemcpyHostToDevice, stream));
     return MB_OK;
   }
-  MB_TRY(mb_unpack_dev(n, fpacked, A, n, perturb, fpacked, stream));
-  MB_CUDA(cudaMemsetAsync(V, 0, sizeof(double) * nn, stream));
-  MB_CUDA(cudaMemsetAsync(e, 0, sizeof(double) * n, stream));
-
-  // cooperative grid size: co-resident CTAs of the panel form in use
-  static int sms = 0, per1 = 0;
-  if (sms == 0) {
-    int dev = 0;
-    MB_CUDA(cudaGetDevice(&dev));
-    MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, tridiag_panel, TPB, 0));
-    if (per1 > 4) per1 = 4;
-    if (per1 < 1) return mb_set_error(MB_ERR_CUDA, "tridiag_panel: cannot be co-resident");
-  }
-  const size_t smem2 = 0;
-  bool v2 = true;
-  int per = per1;
-  if (v2) {
-    int per2 = 0;
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, tridiag_panel2, TPB, smem2));
-    if (per2 > 3) per2 = 3;  // wider grids cost more per barrier than they add in bandwidth
-    // every row needs its own 8-lane group
-    if (per2 >= 1 && (long long)sms * per2 * TPB / 8 >= n) per = per2;
-    else v2 = false;
-  }
-  int grid = sms * per;
-  if (grid > 1024) grid = 1024;
-  for (int k = 0; k < n - 1; k += NB) {
-    const int ib = (NB < n - 1 - k) ? NB : n - 1 - k;
-    MB_CUDA(cudaMemsetAsync(vwv, 0, sizeof(double) * (size_t)n * 2 * NB, stream));
-    PanelArgs pa;
-    pa.n = n; pa.k = k; pa.ib = ib; pa.lda = n;
-    pa.a = A; pa.vp = vp; pa.wp = wp; pa.vall = V; pa.d = d; pa.e = e; pa.tau = tau;
-    pa.part = part; pa.partd = part + 1024; pa.tvec = tvec; pa.tpart = tpart; pa.wvec = wvec;
-    void* args[] = {&pa};
+  // T's records of the Sturm counts and of the inverse iteration, before Y is used
+  double2* de = (double2*)(((uintptr_t)w.Y + 15) & ~(uintptr_t)15);
+  double2* dv = de + n + 2 * SB;
+  double* inv = w.wvec;  // the eigenvectors' norms, after the panels have used it
+  double* weig = w.e2;   // eigenvalues of the scaled T
+  // one launch up to the order whose columns fit in the registers of 16 CTAs
+  const bool small = n <= mb_tridiag_cluster_max();
+  if (small) {
     mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, true);
-    // rows own 8-lane groups when the grid has enough of them
-    void* kfn = v2 ? (void*)tridiag_panel2 : (void*)tridiag_panel;
-    MB_CUDA(cudaLaunchCooperativeKernel(kfn, grid, TPB, args, 0, stream));
+    MB_TRY(mb_tridiag_cluster(n, fpacked, perturb, w.V, w.d, w.e, w.tau, status_dev, stream));
     mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, false);
-    mb_count_launch();
-    const int t = k + ib;
-    if (t < n) {
-      const int m = n - t;
-      double* At = A + (size_t)t * n + t;
-      if (ib == NB) {
-        // A -= [V W] [W V]^T as one GEMM with k = 2*NB
-        MB_CUDA(cudaMemcpyAsync(vwv + (size_t)n * 2 * NB, vp, sizeof(double) * (size_t)n * NB,
-                                cudaMemcpyDeviceToDevice, stream));
-        MB_TRY(mb_dgemm_dev('N', 'T', m, m, 2 * NB, -1.0, vwv + t, n, wp + t, n, 1.0, At, n, stream));
-      } else {
-        MB_TRY(mb_dgemm_dev('N', 'T', m, m, ib, -1.0, vp + t, n, wp + t, n, 1.0, At, n, stream));
-        MB_TRY(mb_dgemm_dev('N', 'T', m, m, ib, -1.0, wp + t, n, vp + t, n, 1.0, At, n, stream));
-      }
+  } else {
+    MB_TRY(mb_unpack_dev(n, fpacked, w.A, n, perturb, fpacked, stream));
+    MB_CUDA(cudaMemsetAsync(w.V, 0, sizeof(double) * nn, stream));
+    static int sms = 0;
+    if (sms == 0) {
+      int dev = 0;
+      MB_CUDA(cudaGetDevice(&dev));
+      MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     }
+    int k = 0;
+    MB_TRY(mb_eigh_panels(n, n - mb_tridiag_grid_max(sms), &w, stream, &k));
+    const size_t o = (size_t)k * n + k;
+    mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, true);
+    MB_TRY(mb_tridiag_grid(n - k, sms, w.A + o, n, w.V + o, w.d + k, w.e + k, w.tau + k, w.U0, status_dev, stream));
+    mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, false);
   }
-  copy_last_diag<<<1, 32, 0, stream>>>(n, A, n, d);
+  tri_bounds<<<1, 1024, 0, stream>>>(n, w.d, w.e, de, dv, w.bnd);
   MB_LAUNCH_CHECK();
-  // eigenvalues
-  tri_bounds<<<1, 1024, 0, stream>>>(n, d, e, e2, bnd);
+  bisect_kernel<<<(n * 32 + 127) / 128, 128, 0, stream>>>(n, de, w.bnd, weig, eigs);
   MB_LAUNCH_CHECK();
-  bisect_kernel<<<(n * 32 + 255) / 256, 256, 0, stream>>>(n, d, e2, bnd, eigs);
+  // eigenvectors of T; the reduction has no more use for A
+  const TriLu lu{w.U0, w.U1, w.U2, w.A, (unsigned char*)w.Z, 0};
+  inverse_iteration<<<(n + 31) / 32, 32, 0, stream>>>(n, dv, weig, w.bnd, w.X, inv, lu, status_dev);
   MB_LAUNCH_CHECK();
-  // eigenvectors of T
-  MB_CUDA(cudaMemsetAsync(status_dev, 0, sizeof(int), stream));
-  inverse_iteration<<<(n + 127) / 128, 128, 0, stream>>>(n, d, e, eigs, bnd, X, U0, U1, U2, status_dev);
-  MB_LAUNCH_CHECK();
-  {
-    dim3 g((n + 31) / 32, (n + 31) / 32), blk(32, 8);
-    transpose_kernel<<<g, blk, 0, stream>>>(n, X, Z);
-    MB_LAUNCH_CHECK();
+  if (small) {
+    if (n <= 64) return launch_back_small<2>(n, w.V, w.tau, w.X, inv, c, stream);
+    if (n <= 160) return launch_back_small<5>(n, w.V, w.tau, w.X, inv, c, stream);
+    if (n <= 320) return launch_back_small<10>(n, w.V, w.tau, w.X, inv, c, stream);
+    return launch_back_small<20>(n, w.V, w.tau, w.X, inv, c, stream);
   }
-  // back-transformation, blocks of BT reflectors in reverse order:
-  // Z <- (I - V T V^T) Z
-  {
-    static bool larft_attr = false;
-    if (!larft_attr) {
-      MB_CUDA(cudaFuncSetAttribute(larft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LARFT_SMEM));
-      larft_attr = true;
-    }
-    const int nref = n - 1;  // reflectors 0 .. n-2
-    const int last_k = ((nref - 1) / BT) * BT;
-    const int nblk = last_k / BT + 1;
-    // every block's T factor first (they depend on V only), in one launch
-    for (int k = 0; k <= last_k; k += BT) {
-      const int ib = (BT < nref - k) ? BT : nref - k;
-      const int r0 = k + 1;
-      const double* Vk = V + (size_t)k * n + r0;
-      MB_TRY(mb_dgemm_ws('T', 'N', ib, ib, n - r0, 1.0, Vk, n, Vk, n, 0.0, S + (size_t)(k / BT) * BT * BT, ib, U0,
-                         3 * nn, stream));
-    }
-    larft_kernel<<<nblk, BT, LARFT_SMEM, stream>>>(nref, S, tau, Tm);
-    MB_LAUNCH_CHECK();
-    for (int k = last_k; k >= 0; k -= BT) {
-      const int ib = (BT < nref - k) ? BT : nref - k;
-      if (ib <= 0) continue;
-      const int r0 = k + 1;  // first nonzero row of the block's reflectors
-      const int m = n - r0;
-      const double* Vk = V + (size_t)k * n + r0;
-      const double* Tk = Tm + (size_t)(k / BT) * BT * BT;
-      MB_TRY(mb_dgemm_ws('T', 'N', ib, n, m, 1.0, Vk, n, Z + r0, n, 0.0, Y, ib, U0, 3 * nn, stream));
-      MB_TRY(mb_dgemm_dev('N', 'N', ib, n, ib, 1.0, Tk, ib, Y, ib, 0.0, X, ib, stream));
-      MB_TRY(mb_dgemm_dev('N', 'N', m, n, ib, -1.0, Vk, n, X, ib, 1.0, Z + r0, n, stream));
-    }
-  }
-  MB_CUDA(cudaMemcpyAsync(c, Z, sizeof(double) * nn, cudaMemcpyDeviceToDevice, stream));
-  return MB_OK;
+  dim3 g((n + 31) / 32, (n + 31) / 32), blk(32, 8);
+  transpose_kernel<<<g, blk, 0, stream>>>(n, w.X, inv, w.Z);
+  MB_LAUNCH_CHECK();
+  return mb_eigh_back(n, &w, c, stream);
 }
 
 extern "C" int mb_eigh_packed_dev(int n, double* fpacked, double* c, double* eigs, cudaStream_t stream) {

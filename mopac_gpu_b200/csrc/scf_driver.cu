@@ -28,6 +28,8 @@ extern "C" int mb_cnvg_ws(int norbs, double* pnew, double* p, double* p1, int ni
 extern "C" size_t mb_eigh_ws_bytes(int n);
 extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
                           cudaStream_t stream);
+extern "C" int mb_eigh_ordered_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws,
+                                  int* status_dev, cudaStream_t stream);
 extern "C" size_t mb_pseudo_ws_bytes(int n, int nocc);
 extern "C" int mb_dgemm_dev(char transa, char transb, int m, int n, int k, double alpha, const double* a, int lda,
                             const double* b, int ldb, double beta, double* c, int ldc, cudaStream_t stream);
@@ -609,9 +611,12 @@ struct PhaseTimer {
   }
 };
 
-static int full_diag(mb_ctx* c, double* fpacked, double* eig_homo, double* eig_lumo, int ihomo, int perturb = 1) {
+// ordered: the eigensolver with a fixed order of operations (see eigen_panel.cu).
+static int full_diag(mb_ctx* c, double* fpacked, double* eig_homo, double* eig_lumo, int ihomo, int perturb,
+                     bool ordered) {
   mb_kstat_mark(MB_KSTAT_EIGH, c->stream, true);
-  MB_TRY(mb_eigh_ws(c->norbs, fpacked, perturb, c->c, c->eigs, c->eig_ws, c->status, c->stream));
+  MB_TRY((ordered ? mb_eigh_ordered_ws : mb_eigh_ws)(c->norbs, fpacked, perturb, c->c, c->eigs, c->eig_ws, c->status,
+                                                   c->stream));
   mb_kstat_mark(MB_KSTAT_EIGH, c->stream, false);
   int st = 0;
   MB_CUDA(cudaMemcpyAsync(&st, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -983,7 +988,7 @@ extern "C" int mb_scf_run(mb_ctx* c, const mb_scf_opts* opts_in, mb_scf_result* 
       mb_kstat_mark(MB_KSTAT_PSEUDO, s, false);
       res->n_pseudo_diag++;
     } else {
-      MB_TRY(full_diag(c, c->f, &eig_homo, &eig_lumo, ihomo));
+      MB_TRY(full_diag(c, c->f, &eig_homo, &eig_lumo, ihomo, 1, opts.pseudo != 0 || use_split));
       res->n_full_diag++;
     }
     t_diag.stop();
@@ -1038,7 +1043,7 @@ extern "C" int mb_scf_run(mb_ctx* c, const mb_scf_opts* opts_in, mb_scf_result* 
     res->exit_split = 1;
   } else {
     // a declined split has perturbed fdiag already
-    MB_TRY(full_diag(c, c->fdiag, &eig_homo, &eig_lumo, ihomo, split_tried ? 0 : 1));
+    MB_TRY(full_diag(c, c->fdiag, &eig_homo, &eig_lumo, ihomo, split_tried ? 0 : 1, false));
     res->n_full_diag++;
   }
   t_diag.stop();
