@@ -33,6 +33,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "mb_common.cuh"
@@ -433,27 +434,79 @@ struct GemmArgs {
   const float* bias;   // EPI_HIDDEN, EPI_OUT
   const float* zin;    // EPI_DSILU: pre-activations (ldz)
   float* zout;         // EPI_HIDDEN: pre-activations out (may be null)
-  long long ldz;
+  long long ldz;       // rows of zin, zout; EPI_F32: from one k slice's sums to the next's
   float* outf;         // EPI_OUT, EPI_F32
+  float* bias_out;     // EPI_F32: sums of A over k
   uint16_t* outh;      // EPI_HIDDEN, EPI_DSILU
   long long ldo;
 };
 
-constexpr int BM = 64, BN = 64, BK = 32, PAD = 8;
+constexpr int BM = 64, BN = 64, BK = 32, STG = 3;
+// Halves per row of a staged tile: rows of k (BK wide) or of m / n (64 wide),
+// padded so that the eight rows of an ldmatrix fall on distinct banks.
+constexpr int LDK = BK + 8, LDM = BM + 8;
+constexpr int TILE = BM * LDK > BK * LDM ? BM * LDK : BK * LDM;
 
-__device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
+__device__ __forceinline__ void mma_bf16(float* d, const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int EPI>
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const uint16_t* p) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(p);
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(s));
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(s));
+}
+
+// 64 x BK tile of an operand X(r, k), r from r0 and k from k0, zero outside
+// R x K.  KC: k is the contiguous index, the tile is kept [r][k]; else r is,
+// and it is kept [k][r] for transposing reads.  VEC: four halves per copy
+// (asynchronous), else one.
+template <bool KC, bool VEC>
+__device__ __forceinline__ void stage_tile(uint16_t* t, const uint16_t* x, long long ld, int r0, int R, int k0, int K) {
+  constexpr int W = KC ? BK : BM, H = KC ? BM : BK, LD = KC ? LDK : LDM;  // W contiguous
+  if (VEC) {
+#pragma unroll
+    for (int c = threadIdx.x; c < H * W / 4; c += 128) {
+      const int row = c / (W / 4), w = 4 * (c % (W / 4));
+      const int r = r0 + (KC ? row : w), k = k0 + (KC ? w : row);
+      const bool in = r < R && k < K;
+      const uint16_t* src = in ? x + (KC ? (long long)r * ld + k : (long long)k * ld + r) : x;
+      const unsigned d = (unsigned)__cvta_generic_to_shared(t + row * LD + w);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(in ? 8 : 0) : "memory");
+    }
+  } else {
+    for (int c = threadIdx.x; c < H * W; c += 128) {
+      const int row = c / W, w = c % W;
+      const int r = r0 + (KC ? row : w), k = k0 + (KC ? w : row);
+      t[row * LD + w] = r < R && k < K ? x[KC ? (long long)r * ld + k : (long long)k * ld + r] : (uint16_t)0;
+    }
+  }
+}
+
+// AK, BC: A's and B's k index is the contiguous one.  Each output is summed
+// over k in ascending order, 16 at a time; EPI_F32 cuts k into gridDim.z slices
+// of whole BK blocks (slice z writes its sums at outf + z * ldz, and the sums
+// of A over k at bias_out + z * ldz), which the reader adds up.
+// Three stages of cp.async keep the loads of two k blocks in flight; the
+// fragments come by ldmatrix.  Bound by the latency of a few k blocks per CTA.
+// At 2048 rows (one B200) a 128-wide forward layer takes 9 us (34 with a 2-byte
+// load per element and one stage), a weight gradient 6 us with 16 slices (176 in
+// one slice of 4 to 12 CTAs, and 45 more for the bias gradient, now the sums of
+// the tiles already staged); a training step 0.14 ms (1.11).
+template <int EPI, bool AK, bool BC, bool VEC>
 __global__ void __launch_bounds__(128) mlp_gemm_kernel(GemmArgs g) {
-  __shared__ __align__(16) uint16_t As[BM][BK + PAD];
-  __shared__ __align__(16) uint16_t Bs[BN][BK + PAD];
+  __shared__ __align__(16) uint16_t As[STG][TILE], Bs[STG][TILE];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
@@ -465,60 +518,58 @@ __global__ void __launch_bounds__(128) mlp_gemm_kernel(GemmArgs g) {
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
-
-  for (int k0 = 0; k0 < g.K; k0 += BK) {
-    // A tile: As[m][k]
-    if (g.sak == 1) {
-      const int kk = tid & 31;
-      for (int r = tid >> 5; r < BM; r += 4) {
-        int m = m0 + r, k = k0 + kk;
-        As[r][kk] = (m < g.M && k < g.K) ? g.a[(long long)m * g.sam + k] : (uint16_t)0;
-      }
-    } else {
-      const int r = tid & 63;
-      for (int kk = tid >> 6; kk < BK; kk += 2) {
-        int m = m0 + r, k = k0 + kk;
-        As[r][kk] = (m < g.M && k < g.K) ? g.a[(long long)m * g.sam + (long long)k * g.sak] : (uint16_t)0;
-      }
+  int kb = 0, ke = g.K;
+  if (EPI == EPI_F32) {
+    const int chunk = ((g.K + (int)gridDim.z - 1) / (int)gridDim.z + BK - 1) / BK * BK;
+    kb = min(g.K, (int)blockIdx.z * chunk);
+    ke = min(g.K, kb + chunk);
+  }
+  const long long lda = AK ? g.sam : g.sak, ldb = BC ? g.sbn : g.sbk;
+  auto stage = [&](int t) {
+    const int k0 = kb + t * BK;
+    if (k0 < ke) {
+      stage_tile<AK, VEC>(As[t % STG], g.a, lda, m0, g.M, k0, ke);
+      stage_tile<BC, VEC>(Bs[t % STG], g.b, ldb, n0, g.N, k0, ke);
     }
-    // B tile: Bs[n][k]
-    if (g.sbk == 1) {
-      const int kk = tid & 31;
-      for (int r = tid >> 5; r < BN; r += 4) {
-        int n = n0 + r, k = k0 + kk;
-        Bs[r][kk] = (n < g.N && k < g.K) ? g.b[(long long)n * g.sbn + k] : (uint16_t)0;
-      }
-    } else {
-      const int r = tid & 63;
-      for (int kk = tid >> 6; kk < BK; kk += 2) {
-        int n = n0 + r, k = k0 + kk;
-        Bs[r][kk] = (n < g.N && k < g.K) ? g.b[(long long)k * g.sbk + (long long)n * g.sbn] : (uint16_t)0;
-      }
-    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int nk = (ke - kb + BK - 1) / BK;
+  float colsum = 0.f;
+  for (int t = 0; t < STG - 1; ++t) stage(t);
+  for (int t = 0; t < nk; ++t) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STG - 2) : "memory");
     __syncthreads();
+    stage(t + STG - 1);
+    const uint16_t* at = As[t % STG];
+    const uint16_t* bt = Bs[t % STG];
 #pragma unroll
     for (int ks = 0; ks < BK; ks += 16) {
-      uint32_t af[2][4], bfr[4][2];
+      uint32_t af[2][4], bf[2][4];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int r = wm + i * 16 + gq;
-        af[i][0] = *reinterpret_cast<const uint32_t*>(&As[r][ks + 2 * tq]);
-        af[i][1] = *reinterpret_cast<const uint32_t*>(&As[r + 8][ks + 2 * tq]);
-        af[i][2] = *reinterpret_cast<const uint32_t*>(&As[r][ks + 2 * tq + 8]);
-        af[i][3] = *reinterpret_cast<const uint32_t*>(&As[r + 8][ks + 2 * tq + 8]);
+        if (AK) ldmatrix4<false>(af[i], at + (wm + i * 16 + (lane & 15)) * LDK + ks + (lane >> 4) * 8);
+        else ldmatrix4<true>(af[i], at + (ks + (lane & 7) + (lane >> 4) * 8) * LDM + wm + i * 16 + ((lane >> 3) & 1) * 8);
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = wn + j * 8 + gq;
-        bfr[j][0] = *reinterpret_cast<const uint32_t*>(&Bs[c][ks + 2 * tq]);
-        bfr[j][1] = *reinterpret_cast<const uint32_t*>(&Bs[c][ks + 2 * tq + 8]);
+      for (int j = 0; j < 2; ++j) {  // two 8-column blocks at a time
+        if (BC) ldmatrix4<false>(bf[j], bt + (wn + j * 16 + (lane & 7) + (lane >> 4) * 8) * LDK + ks + ((lane >> 3) & 1) * 8);
+        else ldmatrix4<true>(bf[j], bt + (ks + (lane & 15)) * LDM + wn + j * 16 + (lane >> 4) * 8);
       }
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i][0], af[i][1], af[i][2], af[i][3], bfr[j][0], bfr[j][1]);
+        for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i], bf[j >> 1][2 * (j & 1)], bf[j >> 1][2 * (j & 1) + 1]);
     }
-    __syncthreads();
+    if (EPI == EPI_F32 && blockIdx.x == 0 && tid < BM) {
+#pragma unroll 8
+      for (int k = 0; k < BK; ++k) colsum += bf2f(AK ? at[tid * LDK + k] : at[k * LDM + tid]);
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  float* outf = g.outf;
+  if (EPI == EPI_F32) {
+    outf += (long long)blockIdx.z * g.ldz;
+    if (blockIdx.x == 0 && tid < BM && m0 + tid < g.M) g.bias_out[(long long)blockIdx.z * g.ldz + m0 + tid] = colsum;
   }
   // epilogue
 #pragma unroll
@@ -536,20 +587,29 @@ __global__ void __launch_bounds__(128) mlp_gemm_kernel(GemmArgs g) {
           if (g.zout) g.zout[(long long)m * g.ldz + n] = z;
           g.outh[(long long)m * g.ldo + n] = f2bf(silu_f(z));
         } else if (EPI == EPI_OUT) {
-          g.outf[(long long)m * g.ldo + n] = v + g.bias[n];
+          outf[(long long)m * g.ldo + n] = v + g.bias[n];
         } else if (EPI == EPI_F32) {
-          g.outf[(long long)m * g.ldo + n] = v;
+          outf[(long long)m * g.ldo + n] = v;
         } else {
           g.outh[(long long)m * g.ldo + n] = f2bf(v * dsilu_f(g.zin[(long long)m * g.ldz + n]));
         }
       }
 }
 
-template <int EPI>
-int launch_gemm(const GemmArgs& g, cudaStream_t s) {
+// AK, BC as the caller lays its operands out (checked); slices: of k, EPI_F32.
+template <int EPI, bool AK, bool BC>
+int launch_gemm(const GemmArgs& g, cudaStream_t s, int slices = 1) {
   if (g.M <= 0 || g.N <= 0) return MB_OK;
-  dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM);
-  mlp_gemm_kernel<EPI><<<grid, 128, 0, s>>>(g);
+  if ((AK ? g.sak : g.sam) != 1 || (BC ? g.sbk : g.sbn) != 1)
+    return mb_set_error(MB_ERR_ARG, "mlp_gemm: operand layout");
+  // four halves at a time need whole 8-byte groups inside the operand
+  auto vec = [](const uint16_t* x, long long ld, int width) {
+    return ((uintptr_t)x & 7) == 0 && ld % 4 == 0 && width % 4 == 0;
+  };
+  const bool v = vec(g.a, AK ? g.sam : g.sak, AK ? g.K : g.M) && vec(g.b, BC ? g.sbn : g.sbk, BC ? g.K : g.N);
+  dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, slices);
+  if (v) mlp_gemm_kernel<EPI, AK, BC, true><<<grid, 128, 0, s>>>(g);
+  else mlp_gemm_kernel<EPI, AK, BC, false><<<grid, 128, 0, s>>>(g);
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
@@ -683,21 +743,17 @@ __global__ void lossgrad_kernel(int n, int nout, const float* __restrict__ y, co
   if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(loss, l);
 }
 
-// db[j] = sum over rows of dz[row * ld + j]
-__global__ void colsum_kernel(int rows, int cols, const uint16_t* __restrict__ dz, float* __restrict__ db) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += bf2f(dz[(long long)r * cols + j]);
-  db[j] = s;
-}
-
-__global__ void adam_kernel(long long n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, uint16_t* __restrict__ pbf, float lr, float b1, float b2, float c1,
-                            float c2, float eps) {
+// Gradient of each parameter as the sum of its nz slices (part + z * n), in
+// order, then (update) Adam.
+__global__ void adam_kernel(long long n, int nz, const float* __restrict__ part, int update, float* __restrict__ p,
+                            float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
+                            uint16_t* __restrict__ pbf, float lr, float b1, float b2, float c1, float c2, float eps) {
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float gi = g[i];
+  float gi = 0.f;
+  for (int z = 0; z < nz; ++z) gi += part[(long long)z * n + i];
+  g[i] = gi;
+  if (!update) return;
   float mi = b1 * m[i] + (1.f - b1) * gi;
   float vi = b2 * v[i] + (1.f - b2) * gi * gi;
   m[i] = mi;
@@ -869,7 +925,7 @@ static int forward_impl(const float* params, const uint16_t* wbf, int type, int 
     g.zout = zs ? zs + (long long)l * n * HID : nullptr;
     g.ldz = HID;
     g.outh = out; g.ldo = HID;
-    MB_TRY(launch_gemm<EPI_HIDDEN>(g, s));
+    MB_TRY((launch_gemm<EPI_HIDDEN, true, true>(g, s)));
     in = out;
     kin = HID;
   }
@@ -879,7 +935,7 @@ static int forward_impl(const float* params, const uint16_t* wbf, int type, int 
   g.b = W[3]; g.sbk = 1; g.sbn = HID;
   g.bias = b[3];
   g.outf = y; g.ldo = DOUT;
-  return launch_gemm<EPI_OUT>(g, s);
+  return launch_gemm<EPI_OUT, true, true>(g, s);
 }
 
 extern "C" int mb_guess_forward_dev(const mb_guess_model* m, int type, int n, const uint16_t* x, float* y, void* ws,
@@ -1113,6 +1169,7 @@ struct mb_guess_trainer {
   float* params = nullptr;
   uint16_t* wbf = nullptr;
   float *grads = nullptr, *mom = nullptr, *vel = nullptr;
+  float* part = nullptr;     // grad_slices(max_rows) partial gradients of one type's parameters
   int max_rows = 0;
   float* zs = nullptr;       // 3 * max_rows * HID
   uint16_t* acts = nullptr;  // 3 * max_rows * HID
@@ -1122,8 +1179,12 @@ struct mb_guess_trainer {
   long long steps[NT] = {0, 0, 0, 0, 0};
 };
 
+// Slices of the rows in the weight gradients, whose outputs are only 2 to 12
+// tiles: 128 rows each (four k blocks), up to 32.
+static int grad_slices(int rows) { return std::min(32, (rows + 127) / 128); }
+
 static void trainer_free(mb_guess_trainer* t) {
-  void* ptrs[] = {t->params, t->wbf, t->grads, t->mom, t->vel, t->zs, t->acts, t->y, t->dz, t->loss};
+  void* ptrs[] = {t->params, t->wbf, t->grads, t->mom, t->vel, t->part, t->zs, t->acts, t->y, t->dz, t->loss};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   delete t;
@@ -1142,6 +1203,7 @@ extern "C" int mb_guess_trainer_create(const float* blob, int max_rows, mb_guess
   TALLOC(t->grads, nf * sizeof(float));
   TALLOC(t->mom, nf * sizeof(float));
   TALLOC(t->vel, nf * sizeof(float));
+  TALLOC(t->part, (size_t)grad_slices(max_rows) * (TRAIN_END - TRAIN_BEGIN) * sizeof(float));
   TALLOC(t->zs, 3 * mr * HID * sizeof(float));
   TALLOC(t->acts, 3 * mr * HID * sizeof(uint16_t));
   TALLOC(t->y, mr * DOUT * sizeof(float));
@@ -1209,10 +1271,9 @@ extern "C" int mb_guess_trainer_step(mb_guess_trainer* t, int type, int n, const
   MB_LAUNCH_CHECK();
   const uint16_t* Wbf[4] = {t->wbf + base + OFF_W1, t->wbf + base + OFF_W2, t->wbf + base + OFF_W3,
                             t->wbf + base + OFF_W4};
-  float* gW[4] = {t->grads + base + OFF_W1, t->grads + base + OFF_W2, t->grads + base + OFF_W3,
-                  t->grads + base + OFF_W4};
-  float* gb[4] = {t->grads + base + OFF_B1, t->grads + base + OFF_B2, t->grads + base + OFF_B3,
-                  t->grads + base + OFF_B4};
+  const long long oW[4] = {OFF_W1, OFF_W2, OFF_W3, OFF_W4}, ob[4] = {OFF_B1, OFF_B2, OFF_B3, OFF_B4};
+  const long long nt = TRAIN_END - TRAIN_BEGIN;
+  const int slices = grad_slices(n);
   // layer l (0-based, 3 = output): dz_l has width nw[l]; its input a_{l-1}
   const int nw[4] = {HID, HID, HID, DOUT};
   const int kin[4] = {DIN, HID, HID, HID};
@@ -1224,10 +1285,9 @@ extern "C" int mb_guess_trainer_step(mb_guess_trainer* t, int type, int n, const
     g.M = nw[l]; g.N = kin[l]; g.K = n;
     g.a = dz; g.sam = 1; g.sak = nw[l];
     g.b = ain; g.sbk = kin[l]; g.sbn = 1;
-    g.outf = gW[l]; g.ldo = kin[l];
-    MB_TRY(launch_gemm<EPI_F32>(g, s));
-    colsum_kernel<<<blocks_for(nw[l], 128), 128, 0, s>>>(n, nw[l], dz, gb[l]);
-    MB_LAUNCH_CHECK();
+    g.outf = t->part + oW[l] - TRAIN_BEGIN; g.ldo = kin[l];
+    g.bias_out = t->part + ob[l] - TRAIN_BEGIN; g.ldz = nt;
+    MB_TRY((launch_gemm<EPI_F32, false, false>(g, s, slices)));
     if (l > 0) {
       // dz_{l-1} = (dz W_l) * silu'(z_{l-1})
       uint16_t* dzn = dz == dzA ? dzB : dzA;
@@ -1237,20 +1297,18 @@ extern "C" int mb_guess_trainer_step(mb_guess_trainer* t, int type, int n, const
       h.b = Wbf[l]; h.sbk = kin[l]; h.sbn = 1;
       h.zin = zs + (long long)(l - 1) * nh; h.ldz = HID;
       h.outh = dzn; h.ldo = HID;
-      MB_TRY(launch_gemm<EPI_DSILU>(h, s));
+      MB_TRY((launch_gemm<EPI_DSILU, true, false>(h, s)));
       dz = dzn;
     }
   }
-  if (update) {
-    long long st = ++t->steps[type];
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - powf(b1, (float)st), c2 = 1.f - powf(b2, (float)st);
-    const long long nt = TRAIN_END - TRAIN_BEGIN;
-    adam_kernel<<<blocks_for(nt, 256), 256, 0, s>>>(nt, t->params + base + TRAIN_BEGIN, t->grads + base + TRAIN_BEGIN,
-                                                    t->mom + base + TRAIN_BEGIN, t->vel + base + TRAIN_BEGIN,
-                                                    t->wbf + base + TRAIN_BEGIN, lr, b1, b2, c1, c2, 1e-8f);
-    MB_LAUNCH_CHECK();
-  }
+  const long long st = update ? ++t->steps[type] : 1;
+  const float b1 = 0.9f, b2 = 0.999f;
+  const float c1 = 1.f - powf(b1, (float)st), c2 = 1.f - powf(b2, (float)st);
+  adam_kernel<<<blocks_for(nt, 256), 256, 0, s>>>(nt, slices, t->part, update != 0, t->params + base + TRAIN_BEGIN,
+                                                  t->grads + base + TRAIN_BEGIN, t->mom + base + TRAIN_BEGIN,
+                                                  t->vel + base + TRAIN_BEGIN, t->wbf + base + TRAIN_BEGIN, lr, b1, b2,
+                                                  c1, c2, 1e-8f);
+  MB_LAUNCH_CHECK();
   if (loss_out) {
     double l = 0.0;
     MB_CUDA(cudaMemcpyAsync(&l, t->loss, sizeof(double), cudaMemcpyDeviceToHost, s));
