@@ -390,46 +390,128 @@ __global__ void __launch_bounds__(MZ_T) mzd_virtual(DiagArgs A) {
   }
 }
 
-// Occupied LMO energies psi^T F psi with the reference's cutoff (one thread per LMO).
-__global__ void mzd_occ_energy(MbMzLayout L, MbMzLmos Q, const double* __restrict__ fao, const double* __restrict__ p,
-                               const double* __restrict__ aocc, double cutoff, double* __restrict__ eigs) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < Q.nlmo; i += gridDim.x * blockDim.x) {
-    const int loopi = Q.ncocc[i], nn = Q.nncf[i], nc = Q.ncf[i];
+// (F psi) of atom j1's orbital jx (1-based) from atom k1 alone, in the
+// reference's order; c: k1's coefficients in the LMO, off: the pair's block.
+__device__ __forceinline__ double mzd_block_row(const double* __restrict__ fao, long long off, int k1, int nk, int j1,
+                                                int nj, int jx, const double* __restrict__ c) {
+  double sum1 = 0.0;
+  if (k1 > j1) {
+    for (int i4 = 1; i4 <= nk; ++i4)
+      sum1 = DADD(sum1, DMUL(fao[off + (long long)(i4 - 1) * nj + jx - 1], c[i4 - 1]));
+  } else if (k1 < j1) {
+    for (int i4 = 1; i4 <= nk; ++i4)
+      sum1 = DADD(sum1, DMUL(fao[off + (long long)(jx - 1) * nk + i4 - 1], c[i4 - 1]));
+  } else {
+    for (int j4 = 1; j4 <= jx; ++j4) sum1 = DADD(sum1, DMUL(fao[off + (jx * (jx - 1)) / 2 + j4 - 1], c[j4 - 1]));
+    for (int i4 = jx + 1; i4 <= nk; ++i4) sum1 = DADD(sum1, DMUL(fao[off + (i4 * (i4 - 1)) / 2 + jx - 1], c[i4 - 1]));
+  }
+  return sum1;
+}
+
+// Occupied LMO energies psi^T F psi with the reference's cutoff, a CTA per LMO.
+// For one atom j of the LMO at a time, 128 threads evaluate the terms
+// c(jx) (F psi)(jx) of 128 atoms k each; a warp keeps those the reference
+// counts, in order, and one thread of a fifth warp folds the previous 128
+// atoms' terms in the reference's order (j, k, jx).  The terms wait on
+// dependent loads (the pair lookup), the fold on a chain of additions; the two
+// overlap.  (H2O)150, 600 LMOs: 0.32 ms against 15.6 with a thread per LMO.
+constexpr int OE_T = 128, OE_W = OE_T / 32;
+constexpr int OE_ATOMS = 2048;  // coefficient offsets kept in shared memory
+
+__global__ void __launch_bounds__(OE_T + 32) mzd_occ_energy(MbMzLayout L, MbMzLmos Q, const double* __restrict__ fao,
+                                                            const double* __restrict__ p,
+                                                            const double* __restrict__ aocc, double cutoff,
+                                                            double* __restrict__ eigs) {
+  __shared__ double s_term[2][OE_W][32][4];  // [buffer][warp][kept atom][jx]
+  __shared__ int s_cnt[2][OE_W];
+  __shared__ int s_off[OE_ATOMS];            // each atom's first coefficient, from the LMO's first
+  const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int loopi = Q.ncocc[i], nn = Q.nncf[i], nc = Q.ncf[i];
+  if (nc > OE_ATOMS) {  // an LMO over more atoms than the offsets hold: one thread
+    if (tid != 0) return;
     double sum = 0.0;
     int jl = loopi;
     for (int j = nn; j < nn + nc; ++j) {
-      const int j1 = Q.icocc[j] - 1;
-      const int nj = L.iorbs[j1];
+      const int j1 = Q.icocc[j] - 1, nj = L.iorbs[j1];
       int kl = loopi;
       for (int k = nn; k < nn + nc; ++k) {
-        const int k1 = Q.icocc[k] - 1;
-        const int nk = L.iorbs[k1];
-        const long long k1j1 = pair_offset(L, k1, j1);
+        const int k1 = Q.icocc[k] - 1, nk = L.iorbs[k1];
+        const long long off = pair_offset(L, k1, j1);
         // avir(k1) of this LMO equals aocc of k1's entry
-        if (k1j1 >= 0 && DMUL(DMUL(aocc[k], p[k1j1]), aocc[k]) >= cutoff) {
-          for (int jx = 1; jx <= nj; ++jx) {
-            double sum1 = 0.0;
-            if (k1 > j1) {
-              for (int i4 = 1; i4 <= nk; ++i4)
-                sum1 = DADD(sum1, DMUL(fao[k1j1 + (long long)(i4 - 1) * nj + jx - 1], Q.cocc[kl + i4 - 1]));
-            } else if (k1 < j1) {
-              for (int i4 = 1; i4 <= nk; ++i4)
-                sum1 = DADD(sum1, DMUL(fao[k1j1 + (long long)(jx - 1) * nk + i4 - 1], Q.cocc[kl + i4 - 1]));
-            } else {
-              for (int j4 = 1; j4 <= jx; ++j4)
-                sum1 = DADD(sum1, DMUL(fao[k1j1 + (jx * (jx - 1)) / 2 + j4 - 1], Q.cocc[kl + j4 - 1]));
-              for (int i4 = jx + 1; i4 <= nk; ++i4)
-                sum1 = DADD(sum1, DMUL(fao[k1j1 + (i4 * (i4 - 1)) / 2 + jx - 1], Q.cocc[kl + i4 - 1]));
-            }
-            sum = DADD(sum, DMUL(Q.cocc[jl + jx - 1], sum1));
-          }
-        }
+        if (off >= 0 && DMUL(DMUL(aocc[k], p[off]), aocc[k]) >= cutoff)
+          for (int jx = 1; jx <= nj; ++jx)
+            sum = DADD(sum, DMUL(Q.cocc[jl + jx - 1], mzd_block_row(fao, off, k1, nk, j1, nj, jx, Q.cocc + kl)));
         kl += nk;
       }
       jl += nj;
     }
     eigs[i] = sum;
+    return;
   }
+  if (warp == 0) {
+    int base = 0;
+    for (int k0 = 0; k0 < nc; k0 += 32) {
+      const int nk = k0 + lane < nc ? L.iorbs[Q.icocc[nn + k0 + lane] - 1] : 0;
+      int x = nk;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (k0 + lane < nc) s_off[k0 + lane] = base + x - nk;
+      base += __shfl_sync(0xffffffffu, x, 31);
+    }
+  }
+  __syncthreads();
+  double sum = 0.0;
+  int buf = 0, prev = 0;  // prev: orbitals of the atom j whose terms wait in buffer buf ^ 1
+  auto fold = [&]() {
+    if (tid != OE_T || prev == 0) return;
+    for (int w = 0; w < OE_W; ++w) {
+      const int n = s_cnt[buf ^ 1][w];
+      const double(*t)[4] = s_term[buf ^ 1][w];
+      if (prev == 1) {
+#pragma unroll 8
+        for (int k = 0; k < n; ++k) sum = DADD(sum, t[k][0]);
+      } else {
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) sum = DADD(DADD(DADD(DADD(sum, t[k][0]), t[k][1]), t[k][2]), t[k][3]);
+      }
+    }
+  };
+  for (int j = 0; j < nc; ++j) {
+    const int j1 = Q.icocc[nn + j] - 1, nj = L.iorbs[j1];
+    const double* cj = Q.cocc + loopi + s_off[j];
+    for (int k0 = 0; k0 < nc; k0 += OE_T) {
+      if (tid < OE_T) {
+        const int k = k0 + tid;
+        bool keep = false;
+        int k1 = 0;
+        long long off = -1;
+        if (k < nc) {
+          k1 = Q.icocc[nn + k] - 1;
+          off = pair_offset(L, k1, j1);
+          const double ak = aocc[nn + k];
+          keep = off >= 0 && DMUL(DMUL(ak, p[off]), ak) >= cutoff;
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) s_cnt[buf][warp] = __popc(mask);
+        if (keep) {
+          double* t = s_term[buf][warp][__popc(mask & ((1u << lane) - 1u))];
+          const int nk = L.iorbs[k1];
+          for (int jx = 1; jx <= nj; ++jx)
+            t[jx - 1] = DMUL(cj[jx - 1], mzd_block_row(fao, off, k1, nk, j1, nj, jx, Q.cocc + loopi + s_off[k]));
+        }
+      } else {
+        fold();
+      }
+      __syncthreads();
+      prev = nj;
+      buf ^= 1;
+    }
+  }
+  fold();
+  if (tid == OE_T) eigs[i] = sum;
 }
 
 inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -591,7 +673,7 @@ extern "C" int mb_mz_diagg1_dev(const MbMzLayout* L, const MbMzLmos* occ, const 
     const double t2 = tiny * tiny;
     fref = t2 * t2;
   } else {
-    mzd_occ_energy<<<(occ->nlmo + 127) / 128, 128, 0, stream>>>(*L, *occ, fao, p, aocc, cutoff, eigs);
+    mzd_occ_energy<<<occ->nlmo, OE_T + 32, 0, stream>>>(*L, *occ, fao, p, aocc, cutoff, eigs);
     MB_LAUNCH_CHECK();
     oldlim = tiny * safety * 1.0e-3;
     const double t2 = tiny * tiny;
