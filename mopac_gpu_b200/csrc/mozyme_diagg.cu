@@ -722,8 +722,8 @@ __device__ __forceinline__ int find_atom(const int* ic, int nn, int cnt, const i
 // coefficients as not modifying.  The atom numbers it appends before a
 // rejection stay in the LMOs' spare slots in the reference (it restores the
 // counts, not the slots); the dry run writes them too.
-// ---------------------------------------------------------- warp per rotation
-// diagg2's 2x2 rotation (diagg2.F90:180-345), one warp per rotation: the atom lists of
+// ---------------------------------------------------------- 2x2 rotations
+// diagg2's 2x2 rotation (diagg2.F90:180-345) by one warp: the atom lists of
 // the two LMOs are walked 32 atoms at a time, one lane per atom, and what the
 // sequential loop carries from atom to atom -- the running coefficient offset,
 // the number of atoms appended so far and their coefficient count -- is a
@@ -736,9 +736,7 @@ __device__ __forceinline__ int find_atom(const int* ic, int nn, int cnt, const i
 // overflow check fails first at the same atom as in the sequential loop:
 // the running totals only grow.
 constexpr int WMAP = 1024;            // slots per map; at most WMAP / 2 atoms mapped
-constexpr int D2W = 4;                // warps (rotations) per CTA
 constexpr unsigned FULLW = 0xffffffffu;
-constexpr size_t D2_SMEM = sizeof(int) * 4 * WMAP * D2W;  // two maps (keys, values) per warp
 
 struct WMap {
   int* key;
@@ -799,29 +797,11 @@ __device__ __forceinline__ int wmap_find(const WMap& m, int a, const int* ic, in
   return find_atom(ic, nn, cnt, iorbs, a);
 }
 
-__global__ void __launch_bounds__(32 * D2W) mzd2_level_warp(D2Args A) {
-  extern __shared__ int d2_smem[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long q = A.lo + (long long)blockIdx.x * D2W + wid;
-  if (q >= A.hi) return;  // whole warp
-  WMap mj, mi;
-  mj.key = d2_smem + wid * 4 * WMAP;
-  mj.val = mj.key + WMAP;
-  mi.key = mj.val + WMAP;
-  mi.val = mi.key + WMAP;
-  const long long e = A.order[q];
+// Entry e of the list by the calling warp (lists of any length), with two maps
+// in shared memory.
+__device__ void rotate_warp(const D2Args& A, long long e, double c, double d, WMap mj, WMap mi) {
+  const int lane = threadIdx.x & 31;
   const int i = A.ifmo[2 * e] - 1, j = A.ifmo[2 * e + 1] - 1;
-  const double fm = A.fmo[e];
-  if (!(fabs(fm) >= A.tiny)) {
-    if (lane == 0) { A.beta_sum[e] = 0.0; A.rej[e] = 0; }
-    return;
-  }
-  const double c = DMUL(fm, A.cst);
-  const double d = DSUB(DSUB(A.eigs[j], A.eigv[i]), A.shift);
-  if (!(fabs(c / d) >= A.biglim)) {
-    if (lane == 0) { A.beta_sum[e] = 0.0; A.rej[e] = 0; }
-    return;
-  }
   int* ncf = const_cast<int*>(A.occ.ncf);
   int* icocc = const_cast<int*>(A.occ.icocc);
   double* cocc = const_cast<double*>(A.occ.cocc);
@@ -1008,6 +988,238 @@ __global__ void __launch_bounds__(32 * D2W) mzd2_level_warp(D2Args A) {
     A.rej[e] = rj;
   }
 }
+
+// The same rotation by a CTA: a thread holds an atom of each list in every
+// round of D2T (up to D2R rounds; longer lists go to rotate_warp), so that the
+// loads of both lists, then of their orbital counts, then of their
+// coefficients are in flight together, and the prefix sums (a list's
+// coefficient offsets; the atoms and coefficients appended before this one, for
+// both lists in one 64-bit word) cost one scan a round and one barrier.  Every
+// atom is still computed by one thread in the sequential loop's order.  A
+// warp's walk over lists of some 150 atoms, 32 at a time, was a chain of five
+// dependent round trips per pass and six passes; a dependency level of
+// (H2O)150 took 26 us with it, 10 with a CTA (one B200).
+constexpr int D2T = 128, D2R = 4, D2W = D2T / 32;
+
+__device__ __forceinline__ void map_insert(int* key, int* val, int b, int off) {
+  unsigned h = wmap_hash(b);
+  for (;;) {
+    const int prev = atomicCAS(&key[h], -1, b);
+    if (prev == -1 || prev == b) break;
+    h = (h + 1) & (WMAP - 1);
+  }
+  atomicMin(&val[h], off);  // a repeated atom keeps its first slot
+}
+
+__device__ __forceinline__ int map_find(const int* key, const int* val, int a) {
+  unsigned h = wmap_hash(a);
+  while (key[h] >= 0) {
+    if (key[h] == a) return val[h];
+    h = (h + 1) & (WMAP - 1);
+  }
+  return -1;
+}
+
+// sum over the atom's orbitals of (beta c)^2 > thresh: it joins the other LMO
+__device__ __forceinline__ bool d2_joins(const double* c, int no, double beta, double thresh) {
+  double sum = 0.0;
+  for (int k = 0; k < no; ++k) {
+    const double tt = DMUL(beta, c[k]);
+    sum = DADD(sum, DMUL(tt, tt));
+  }
+  return sum > thresh;
+}
+
+__global__ void __launch_bounds__(D2T) mzd2_level(D2Args A) {
+  __shared__ int s_map[4 * WMAP];
+  __shared__ unsigned long long s_tot[D2R][D2W];
+  __shared__ int s_first[2][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long e = A.order[A.lo + blockIdx.x];
+  const int i = A.ifmo[2 * e] - 1, j = A.ifmo[2 * e + 1] - 1;
+  const double fm = A.fmo[e];
+  const double c = DMUL(fm, A.cst);
+  const double d = DSUB(DSUB(A.eigs[j], A.eigv[i]), A.shift);
+  if (!(fabs(fm) >= A.tiny) || !(fabs(c / d) >= A.biglim)) {
+    if (tid == 0) { A.beta_sum[e] = 0.0; A.rej[e] = 0; }
+    return;
+  }
+  int* ncf = const_cast<int*>(A.occ.ncf);
+  int* icocc = const_cast<int*>(A.occ.icocc);
+  double* cocc = const_cast<double*>(A.occ.cocc);
+  int* nce = const_cast<int*>(A.vir.ncf);
+  int* icvir = const_cast<int*>(A.vir.icocc);
+  double* cvir = const_cast<double*>(A.vir.cocc);
+  const int ncf0 = ncf[j], nce0 = nce[i];
+  int *keyj = s_map, *valj = s_map + WMAP, *keyi = s_map + 2 * WMAP, *vali = s_map + 3 * WMAP;
+  if (ncf0 > D2T * D2R || nce0 > D2T * D2R) {
+    if (warp != 0) return;
+    WMap mj{keyj, valj, false}, mi{keyi, vali, false};
+    rotate_warp(A, e, c, d, mj, mi);
+    return;
+  }
+  const int nnj = A.occ.nncf[j], nni = A.vir.nncf[i];
+  const long long loopj = A.occ.ncocc[j], loopi = A.vir.ncocc[i];
+  const long long jlr = loopj + 1, ilr = loopi + 1;
+  long long jur = (j != A.nocc - 1) ? A.occ.ncocc[j + 1] : A.occ.ncoeff;
+  const long long jncf = (j != A.nocc - 1) ? A.occ.nncf[j + 1] : A.occ.nentries;
+  long long iur = (i != A.nvir - 1) ? A.vir.ncocc[i + 1] : A.vir.ncoeff;
+  const long long incv = (i != A.nvir - 1) ? A.vir.nncf[i + 1] : A.vir.nentries;
+  jur = jlr + A.norbs - 1 < jur ? jlr + A.norbs - 1 : jur;
+  iur = ilr + A.norbs - 1 < iur ? ilr + A.norbs - 1 : iur;
+  // the lists: atoms (-1: none), orbital counts, coefficient offsets
+  int aj[D2R], ai[D2R], nj[D2R], ni[D2R], oj[D2R], oi[D2R];
+#pragma unroll
+  for (int r = 0; r < D2R; ++r) {
+    const int t = tid + D2T * r;
+    aj[r] = t < ncf0 ? icocc[nnj + t] - 1 : -1;
+    ai[r] = t < nce0 ? icvir[nni + t] - 1 : -1;
+  }
+  for (int q = tid; q < WMAP; q += D2T) {
+    keyj[q] = keyi[q] = -1;
+    valj[q] = vali[q] = 0x7fffffff;
+  }
+#pragma unroll
+  for (int r = 0; r < D2R; ++r) {
+    nj[r] = aj[r] >= 0 ? A.iorbs[aj[r]] : 0;
+    ni[r] = ai[r] >= 0 ? A.iorbs[ai[r]] : 0;
+  }
+  // exclusive prefix over t = tid + D2T r of up to four 16-bit counts, and totals
+  auto prefix = [&](unsigned long long (&x)[D2R], unsigned long long& total) {
+    unsigned long long inc[D2R];
+#pragma unroll
+    for (int r = 0; r < D2R; ++r) {
+      unsigned long long v = x[r];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(FULLW, v, o);
+        if (lane >= o) v += y;
+      }
+      inc[r] = v;
+      if (lane == 31) s_tot[r][warp] = v;
+    }
+    __syncthreads();
+    total = 0;
+#pragma unroll
+    for (int r = 0; r < D2R; ++r)
+#pragma unroll
+      for (int w = 0; w < D2W; ++w) {
+        if (w == warp) x[r] = total + inc[r] - x[r];
+        total += s_tot[r][w];
+      }
+  };
+  long long mlf0, mle0;
+  {
+    unsigned long long x[D2R], total;
+#pragma unroll
+    for (int r = 0; r < D2R; ++r) x[r] = (unsigned long long)nj[r] | (unsigned long long)ni[r] << 32;
+    prefix(x, total);
+#pragma unroll
+    for (int r = 0; r < D2R; ++r) {
+      oj[r] = (int)(x[r] & 0xffffffffu);
+      oi[r] = (int)(x[r] >> 32);
+      if (aj[r] >= 0) map_insert(keyj, valj, aj[r], oj[r]);
+      if (ai[r] >= 0) map_insert(keyi, vali, ai[r], oi[r]);
+    }
+    mlf0 = (long long)(total & 0xffffffffu);
+    mle0 = (long long)(total >> 32);
+  }
+  __syncthreads();
+  int uj[D2R];          // offset in LMO j of the thread's atoms of LMO i, or -1
+  unsigned alone = 0;   // bit r: the thread's atom of LMO j is not in LMO i
+#pragma unroll
+  for (int r = 0; r < D2R; ++r) {
+    uj[r] = ai[r] >= 0 ? map_find(keyj, valj, ai[r]) : 0;
+    if (aj[r] >= 0 && map_find(keyi, vali, aj[r]) < 0) alone |= 1u << r;
+  }
+  const double ee = copysign(sqrt(DADD(DMUL(DMUL(4.0, c), c), DMUL(d, d))), d);
+  double alpha = sqrt(DMUL(0.5, DADD(1.0, d / ee)));
+  double bs = 0.0;
+  int rj = 0;
+  for (int it = 0;; ++it) {
+    const double beta = -copysign(sqrt(DSUB(1.0, DMUL(alpha, alpha))), c);
+    bs = DADD(bs, fabs(beta));
+    // ---- dry run: atoms of LMO i that would join LMO j (low half of the
+    // word), and of LMO j that would join LMO i
+    if (tid < 2) s_first[it & 1][tid] = 0x7fffffff;
+    unsigned c1 = 0, c2 = 0;
+    unsigned long long x[D2R], total;
+#pragma unroll
+    for (int r = 0; r < D2R; ++r) {
+      x[r] = 0;
+      if (uj[r] < 0 && d2_joins(cvir + loopi + oi[r], ni[r], beta, A.thresh)) {
+        c1 |= 1u << r;
+        x[r] |= 1ull | (unsigned long long)ni[r] << 16;
+      }
+      if ((alone >> r & 1u) && d2_joins(cocc + loopj + oj[r], nj[r], beta, A.thresh)) {
+        c2 |= 1u << r;
+        x[r] |= 1ull << 32 | (unsigned long long)nj[r] << 48;
+      }
+    }
+    prefix(x, total);
+    int n1[D2R], m1[D2R], n2[D2R], m2[D2R];
+#pragma unroll
+    for (int r = 0; r < D2R; ++r) {
+      n1[r] = ncf0 + (int)(x[r] & 0xffffu);
+      m1[r] = (int)(mlf0 + (long long)(x[r] >> 16 & 0xffffu));
+      n2[r] = nce0 + (int)(x[r] >> 32 & 0xffffu);
+      m2[r] = (int)(mle0 + (long long)(x[r] >> 48));
+      if ((c1 >> r & 1u) && (nnj + n1[r] >= jncf || m1[r] + ni[r] + loopj > jur))
+        atomicMin(&s_first[it & 1][0], tid + D2T * r);
+      if ((c2 >> r & 1u) && (nni + n2[r] >= incv || m2[r] + nj[r] + loopi > iur))
+        atomicMin(&s_first[it & 1][1], tid + D2T * r);
+    }
+    __syncthreads();
+    const int f1 = s_first[it & 1][0], f2 = s_first[it & 1][1];
+    const bool no1 = f1 != 0x7fffffff, rejected = no1 || f2 != 0x7fffffff;
+    // appended atoms, up to the first that does not fit; list j's come first
+#pragma unroll
+    for (int r = 0; r < D2R; ++r) {
+      if ((c1 >> r & 1u) && tid + D2T * r < f1) icocc[nnj + n1[r]] = ai[r] + 1;
+      if (!no1 && (c2 >> r & 1u) && tid + D2T * r < f2) icvir[nni + n2[r]] = aj[r] + 1;
+    }
+    if (rejected) {
+      ++rj;
+      if (A.retry) { alpha = DMUL(0.5, DADD(alpha, 1.0)); continue; }
+      break;
+    }
+    // ---- apply
+#pragma unroll
+    for (int r = 0; r < D2R; ++r) {
+      if (ai[r] >= 0 && uj[r] >= 0) {
+        double* pj = cocc + loopj + uj[r];
+        double* pi = cvir + loopi + oi[r];
+        for (int k = 0; k < ni[r]; ++k) {
+          const double a = pj[k], b = pi[k];
+          pj[k] = DADD(DMUL(alpha, a), DMUL(beta, b));
+          pi[k] = DSUB(DMUL(alpha, b), DMUL(beta, a));
+        }
+      } else if (c1 >> r & 1u) {
+        double* pi = cvir + loopi + oi[r];
+        for (int k = 0; k < ni[r]; ++k) {
+          cocc[loopj + m1[r] + k] = DMUL(beta, pi[k]);
+          pi[k] = DMUL(alpha, pi[k]);
+        }
+      }
+      if (c2 >> r & 1u) {
+        double* pj = cocc + loopj + oj[r];
+        for (int k = 0; k < nj[r]; ++k) {
+          cvir[loopi + m2[r] + k] = DMUL(-beta, pj[k]);
+          pj[k] = DMUL(alpha, pj[k]);
+        }
+      }
+    }
+    if (tid == 0) {
+      ncf[j] = ncf0 + (int)(total & 0xffffu);
+      nce[i] = nce0 + (int)(total >> 32 & 0xffffu);
+    }
+    break;
+  }
+  if (tid == 0) {
+    A.beta_sum[e] = bs;
+    A.rej[e] = rj;
+  }
+}
 }  // namespace
 
 extern "C" int mb_mz_diagg2_dev(const MbMzLayout* L, MbMzLmos* occ, MbMzLmos* vir, const int* ifmo, const double* fmo,
@@ -1081,17 +1293,12 @@ extern "C" int mb_mz_diagg2_dev(const MbMzLayout* L, MbMzLmos* occ, MbMzLmos* vi
   A.norbs = L->norbs;
   A.beta_sum = d_bs;
   A.rej = d_rej;
-  static bool d2_attr = false;
-  if (!d2_attr) {
-    MB_CUDA(cudaFuncSetAttribute(mzd2_level_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D2_SMEM));
-    d2_attr = true;
-  }
   for (int v = 1; v <= nlev && rc == MB_OK; ++v) {
     A.lo = start[v];
     A.hi = start[v + 1];
     const long long cnt = A.hi - A.lo;
     if (cnt <= 0) continue;
-    mzd2_level_warp<<<(unsigned)((cnt + D2W - 1) / D2W), 32 * D2W, D2_SMEM, stream>>>(A);
+    mzd2_level<<<(unsigned)cnt, D2T, 0, stream>>>(A);
     mb_count_launch();
     if (cudaGetLastError() != cudaSuccess) rc = mb_set_error(MB_ERR_CUDA, "diagg2: launch");
   }
