@@ -1,14 +1,12 @@
 // FP64 GEMM / packed SYRK (column-major, LAPACK argument conventions).
 //
 // Two tile engines:
-//  * DMMA: 128 x 128 per CTA, BK = 16, 8 warps of 64 x 32, each warp issuing
-//    mma.sync m8n8k4 f64 on the FP64 tensor path (8 x 4 fragments, 64
-//    accumulators per lane).  Used for every product whose output has more
-//    than 64 rows and columns.
-//  * FFMA: 64 x 64 per CTA, 4 x 4 outputs per thread; its 8 shared loads per
-//    16 FMAs bind it at half the FP64 rate, so it only serves skinny outputs.
-// Both double-buffer shared memory through register staging.  The
-// split-precision tensor-core path lives in gemm_tc.cu.
+//  * DMMA: 128 x 128 or 64 x 64 per CTA on mma.sync m16n8k8 f64, used for every
+//    product whose output has more than 64 rows and columns.
+//  * FFMA: 64 x 64 per CTA, 4 x 4 outputs per thread, double-buffered through
+//    registers; its 8 shared loads per 16 FMAs bind it at half the FP64 rate,
+//    so it only serves skinny outputs.
+// The split-precision tensor-core path lives in gemm_tc.cu.
 #include "mb_common.cuh"
 
 namespace {
@@ -130,110 +128,148 @@ __global__ void __launch_bounds__(NT) dgemm_kernel(int m, int n, int k, double a
 }
 
 // ------------------------------------------------------------------ DMMA
-constexpr int DBM = 128, DBN = 128, DBK = 16, DPAD = 4;  // row stride 132 doubles: conflict-free fragments
-constexpr int DMMA_SMEM = (int)sizeof(double) * 2 * DBK * (DBM + DPAD + DBN + DPAD);
+// Tiles of TILE x TILE per CTA, TILE 128 (8 warps of 64 x 32) or 64 (4 warps of
+// 32 x 32), k in blocks of DBK through a ring of DSTG shared-memory stages
+// filled by cp.async; the next fragments of eight k are read while the 4 x 4 or
+// 2 x 4 m16n8k8 products of the current ones run.  An operand is staged as it lies in
+// memory, [k][m] or (transposed) [m][k]; both strides are 4 modulo 16 doubles, so
+// a fragment's lanes hit distinct banks.
+//
+// FP64 products run at the rate of the FP64 pipe either way, so the tile is
+// chosen by how evenly its tiles divide over the SMs (dmma_tile below).  Every
+// output is summed over k in ascending order whatever the tile: both give the
+// same bits.  One B200, us (before: 128-tiles of m8n8k4 in two register-staged
+// buffers): 3072^3 1863 (2058), 3072 x 1024 x 3072 730 (1035), 1024 x 2048 x 3072
+// 518 (546), 2046 x 682 x 2046 259 (354), 682 x 1364 x 2046 174 (369), 1026^3 97
+// (187), 600^3 52 (115); packed SYRK of 3072 x 2048 630 (1043), 1026 x 684 64
+// (128), 600 x 400 34 (81), 144 x 96 16 (27).
+constexpr int DBK = 16, DSTG = 3;
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
+template <int TILE>
+struct Dmma {
+  static constexpr int THREADS = TILE * 2;                  // 8 or 4 warps
+  static constexpr int MI = TILE == 128 ? 8 : 4, NJ = 4;    // fragments of a warp
+  static constexpr int WM = 8 * MI, WROWS = TILE / WM;      // rows of a warp, warps along m
+  static constexpr int LDM = TILE + 4, LDK = DBK + 4;       // strides of [k][m] and [m][k]
+  static constexpr int STAGE = TILE * LDK > DBK * LDM ? TILE * LDK : DBK * LDM;  // doubles, one operand
+  static constexpr int SMEM = (int)sizeof(double) * 2 * DSTG * STAGE;
+};
+
+// A 16 x 8 block over eight k: bit for bit eight multiply-adds in ascending k.
+__device__ __forceinline__ void dmma(double (&c0)[2], double (&c1)[2], const double (&a0)[2], const double (&a1)[2],
+                                     const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+d"(c0[0]), "+d"(c0[1]), "+d"(c1[0]), "+d"(c1[1])
+      : "d"(a0[0]), "d"(a1[0]), "d"(a0[1]), "d"(a1[1]), "d"(b[0]), "d"(b[1]));
 }
 
-// 128 x 128 tile of op(A) op(B) over k in [kbeg, kend).  Warp w covers rows
-// (w % 2) * 64 .. +64 and columns (w / 2) * 32 .. +32; fragment (i, j) of a
-// lane holds C(row0 + 8 i + lane / 4, col0 + 8 j + 2 (lane % 4) + {0, 1}).
-template <bool TA, bool TB>
-__device__ __forceinline__ void tile_dmma(const double* __restrict__ a, int lda, const double* __restrict__ b,
-                                          int ldb, int m, int n, int kbeg, int kend, int bm, int bn,
-                                          double (&acc)[8][4][2]) {
-  extern __shared__ double dmma_sh[];  // DMMA_SMEM bytes: As[2][DBK][DBM+DPAD], Bs[2][DBK][DBN+DPAD]
-  double(*As)[DBK][DBM + DPAD] = reinterpret_cast<double(*)[DBK][DBM + DPAD]>(dmma_sh);
-  double(*Bs)[DBK][DBN + DPAD] = reinterpret_cast<double(*)[DBK][DBN + DPAD]>(dmma_sh + 2 * DBK * (DBM + DPAD));
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 1) * 64, wn = (warp >> 1) * 32;
+// Rows r0 .. r0 + TILE - 1, k0 .. k0 + DBK - 1 of an operand X(r, k), zero
+// outside R x K.  KC: k is the contiguous index (stage [r][k]), else r is
+// ([k][r]).  V: doubles per copy, 2 when pairs are 16-byte aligned.
+template <int TILE, bool KC, int V>
+__device__ __forceinline__ void dmma_stage(double* t, const double* __restrict__ x, int ld, int r0, int R, int k0,
+                                           int K) {
+  using D = Dmma<TILE>;
+  constexpr int W = KC ? DBK : TILE, H = KC ? TILE : DBK, LD = KC ? D::LDK : D::LDM;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  double ra[8], rb[8];  // 128 x 16 tiles: 8 elements per thread each
-  auto gload = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + q * NT;
-      int r, kk;
-      if (TA) { kk = e % DBK; r = e / DBK; } else { r = e % DBM; kk = e / DBM; }
-      ra[q] = load_a<TA>(a, lda, m, kend, bm + r, k0 + kk);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + q * NT;
-      int cc, kk;
-      if (TB) { cc = e % DBN; kk = e / DBN; } else { kk = e % DBK; cc = e / DBK; }
-      rb[q] = load_b<TB>(b, ldb, n, kend, k0 + kk, bn + cc);
-    }
-  };
-  auto sstore = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + q * NT;
-      int r, kk;
-      if (TA) { kk = e % DBK; r = e / DBK; } else { r = e % DBM; kk = e / DBM; }
-      As[buf][kk][r] = ra[q];
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = tid + q * NT;
-      int cc, kk;
-      if (TB) { cc = e % DBN; kk = e / DBN; } else { kk = e % DBK; cc = e / DBK; }
-      Bs[buf][kk][cc] = rb[q];
-    }
-  };
-  const int nk = (kend - kbeg + DBK - 1) / DBK;
-  gload(kbeg);
-  sstore(0);
-  __syncthreads();
-  const int fr = lane >> 2, fk = lane & 3;
-  for (int t = 0; t < nk; ++t) {
-    const int cur = t & 1;
-    if (t + 1 < nk) gload(kbeg + (t + 1) * DBK);
-#pragma unroll
-    for (int kk = 0; kk < DBK; kk += 4) {
-      double av[8], bv[4];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) av[i] = As[cur][kk + fk][wm + 8 * i + fr];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[cur][kk + fk][wn + 8 * j + fr];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j], av[i], bv[j]);
-    }
-    if (t + 1 < nk) sstore(cur ^ 1);
-    __syncthreads();
+  for (int c = threadIdx.x; c < H * W / V; c += D::THREADS) {
+    const int row = c / (W / V), w = V * (c % (W / V));
+    const int r = r0 + (KC ? row : w), k = k0 + (KC ? w : row);
+    const bool row_in = KC ? r < R : k < K;
+    const int left = KC ? K - k : R - r;  // of the contiguous index
+    const int bytes = !row_in || left <= 0 ? 0 : (left >= V ? 8 * V : 8);
+    const double* src = bytes ? x + (KC ? (long long)r * ld + k : (long long)k * ld + r) : x;
+    const unsigned d = (unsigned)__cvta_generic_to_shared(t + row * LD + w);
+    if (V == 2)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+    else
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
   }
 }
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(NT) dgemm_dmma_kernel(int m, int n, int k, double alpha,
-                                                        const double* __restrict__ a, int lda,
-                                                        const double* __restrict__ b, int ldb, double beta,
-                                                        double* __restrict__ c, int ldc) {
-  const int bm = blockIdx.y * DBM, bn = blockIdx.x * DBN;
+// TILE x TILE tile of op(A) op(B) over k in [kbeg, kend).  Warp w covers rows
+// (w % WROWS) * WM .. and columns (w / WROWS) * 32 ..; fragment (i, j) of a
+// lane holds C(row0 + 8 i + lane / 4, col0 + 8 j + 2 (lane % 4) + {0, 1}).
+template <int TILE, bool TA, bool TB, int V>
+__device__ __forceinline__ void tile_dmma(const double* __restrict__ a, int lda, const double* __restrict__ b,
+                                          int ldb, int m, int n, int kbeg, int kend, int bm, int bn,
+                                          double (&acc)[Dmma<TILE>::MI][Dmma<TILE>::NJ][2]) {
+  using D = Dmma<TILE>;
+  extern __shared__ __align__(16) double dmma_sh[];  // D::SMEM bytes: DSTG stages of A, then of B
+  double* As = dmma_sh;
+  double* Bs = dmma_sh + DSTG * D::STAGE;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wm = (warp % D::WROWS) * D::WM, wn = (warp / D::WROWS) * 32;
+#pragma unroll
+  for (int i = 0; i < D::MI; ++i)
+#pragma unroll
+    for (int j = 0; j < D::NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int nk = (kend - kbeg + DBK - 1) / DBK;
+  auto stage = [&](int t) {
+    if (t < nk) {
+      dmma_stage<TILE, TA, V>(As + (t % DSTG) * D::STAGE, a, lda, bm, m, kbeg + t * DBK, kend);
+      dmma_stage<TILE, !TB, V>(Bs + (t % DSTG) * D::STAGE, b, ldb, bn, n, kbeg + t * DBK, kend);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int fr = lane >> 2, fk = lane & 3;
+  // this lane's first element of a k4 fragment, and the step to the next row block
+  const int a0 = TA ? (wm + fr) * D::LDK + fk : fk * D::LDM + wm + fr, ai = TA ? 8 * D::LDK : 8, ak = TA ? 4 : 4 * D::LDM;
+  const int b0 = TB ? fk * D::LDM + wn + fr : (wn + fr) * D::LDK + fk, bj = TB ? 8 : 8 * D::LDK, bk = TB ? 4 * D::LDM : 4;
+  for (int t = 0; t < DSTG - 1; ++t) stage(t);
+  for (int t = 0; t < nk; ++t) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(DSTG - 2) : "memory");
+    __syncthreads();  // stage t has landed; every warp has left stage t - 1
+    stage(t + DSTG - 1);
+    const double* at = As + (t % DSTG) * D::STAGE + a0;
+    const double* bt = Bs + (t % DSTG) * D::STAGE + b0;
+    double av[2][D::MI][2], bv[2][D::NJ][2];  // fragments of eight k, as two of four
+    auto load = [&](int q) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int i = 0; i < D::MI; ++i) av[q & 1][i][h] = at[(2 * q + h) * ak + i * ai];
+#pragma unroll
+        for (int j = 0; j < D::NJ; ++j) bv[q & 1][j][h] = bt[(2 * q + h) * bk + j * bj];
+      }
+    };
+    load(0);
+#pragma unroll
+    for (int q = 0; q < DBK / 8; ++q) {
+      if (q + 1 < DBK / 8) load(q + 1);
+#pragma unroll
+      for (int i = 0; i < D::MI; i += 2)
+#pragma unroll
+        for (int j = 0; j < D::NJ; ++j)
+          dmma(acc[i][j], acc[i + 1][j], av[q & 1][i], av[q & 1][i + 1], bv[q & 1][j]);
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+template <int TILE, bool TA, bool TB, int V>
+__global__ void __launch_bounds__(Dmma<TILE>::THREADS)
+    dgemm_dmma_kernel(int m, int n, int k, double alpha, const double* __restrict__ a, int lda,
+                      const double* __restrict__ b, int ldb, double beta, double* __restrict__ c, int ldc) {
+  using D = Dmma<TILE>;
+  const int bm = blockIdx.y * TILE, bn = blockIdx.x * TILE;
   const int kchunk = (k + gridDim.z - 1) / gridDim.z;
   const int kb = blockIdx.z * kchunk, ke = min(k, kb + kchunk);
-  double acc[8][4][2];
-  tile_dmma<TA, TB>(a, lda, b, ldb, m, n, kb, ke, bm, bn, acc);
+  double acc[D::MI][D::NJ][2];
+  tile_dmma<TILE, TA, TB, V>(a, lda, b, ldb, m, n, kb, ke, bm, bn, acc);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r0 = bm + (warp & 1) * 64 + (lane >> 2), c0 = bn + (warp >> 1) * 32 + 2 * (lane & 3);
+  const int r0 = bm + (warp % D::WROWS) * D::WM + (lane >> 2), c0 = bn + (warp / D::WROWS) * 32 + 2 * (lane & 3);
   const bool partial = gridDim.z > 1;
   double* cz = partial ? c + (long long)blockIdx.z * m * n : c;
   const int ldz = partial ? m : ldc;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < D::MI; ++i) {
     const int r = r0 + 8 * i;
     if (r >= m) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < D::NJ; ++j)
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int cc = c0 + 8 * j + t;
@@ -246,20 +282,27 @@ __global__ void __launch_bounds__(NT) dgemm_dmma_kernel(int m, int n, int k, dou
 }
 
 // Packed lower P = occ * A A^T (+ P when acc) on the DMMA engine (tiles meeting the lower triangle).
-__global__ void __launch_bounds__(NT) syrk_packed_dmma_kernel(int n, int k, double occ, const double* __restrict__ a,
-                                                              int lda, double* __restrict__ p, int acc_p) {
-  const int bm = blockIdx.y * DBM, bn = blockIdx.x * DBN;
-  if (bn > bm + DBM - 1) return;
-  double acc[8][4][2];
-  tile_dmma<false, true>(a, lda, a, lda, n, n, 0, k, bm, bn, acc);
+template <int TILE, int V>
+__global__ void __launch_bounds__(Dmma<TILE>::THREADS)
+    syrk_packed_dmma_kernel(int n, int k, double occ, const double* __restrict__ a, int lda, double* __restrict__ p,
+                            int acc_p) {
+  using D = Dmma<TILE>;
+  // block b of the lower triangle of tiles, row by row
+  const long long b = blockIdx.x;
+  int tr = (int)((sqrt(8.0 * (double)b + 1.0) - 1.0) * 0.5);
+  while ((long long)tr * (tr + 1) / 2 > b) --tr;
+  while ((long long)(tr + 1) * (tr + 2) / 2 <= b) ++tr;
+  const int bm = tr * TILE, bn = (int)(b - (long long)tr * (tr + 1) / 2) * TILE;
+  double acc[D::MI][D::NJ][2];
+  tile_dmma<TILE, false, true, V>(a, lda, a, lda, n, n, 0, k, bm, bn, acc);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r0 = bm + (warp & 1) * 64 + (lane >> 2), c0 = bn + (warp >> 1) * 32 + 2 * (lane & 3);
+  const int r0 = bm + (warp % D::WROWS) * D::WM + (lane >> 2), c0 = bn + (warp / D::WROWS) * 32 + 2 * (lane & 3);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < D::MI; ++i) {
     const int r = r0 + 8 * i;
     if (r >= n) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < D::NJ; ++j)
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int cc = c0 + 8 * j + t;
@@ -270,17 +313,75 @@ __global__ void __launch_bounds__(NT) syrk_packed_dmma_kernel(int n, int k, doub
   }
 }
 
-// Opt the DMMA kernels into their dynamic shared memory once per process.
-int dmma_attrs() {
-  static bool done = false;
-  if (done) return MB_OK;
-  MB_CUDA(cudaFuncSetAttribute(dgemm_dmma_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DMMA_SMEM));
-  MB_CUDA(cudaFuncSetAttribute(dgemm_dmma_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DMMA_SMEM));
-  MB_CUDA(cudaFuncSetAttribute(dgemm_dmma_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DMMA_SMEM));
-  MB_CUDA(cudaFuncSetAttribute(dgemm_dmma_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DMMA_SMEM));
-  MB_CUDA(cudaFuncSetAttribute(syrk_packed_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DMMA_SMEM));
-  done = true;
+// 128 or 64, by the time of the fullest SM in tenths of a 64-tile's time at the
+// full rate.  Three 64-tile CTAs share an SM and cover each other's barriers;
+// one or two alone run at half and at 0.8 of the rate.  A 128-tile runs alone on
+// its SM at 0.9.  (3072^3: 31.1 TFLOP/s with 64, 28.2 with 128; 1024 x 2048 x 3072,
+// four 64-tiles or one 128-tile an SM: 21.5 and 24.9; 682 x 1364 x 2046, two or
+// one: 21.9 and 10.3.)
+int dmma_tile(long long tiles128, long long tiles64) {
+  const long long c = (tiles64 + 147) / 148, r = c % 3;
+  const long long t64 = 30 * (c / 3) + (r == 0 ? 0 : r == 1 ? 20 : 24), t128 = 44 * ((tiles128 + 147) / 148);
+  return t64 <= t128 ? 64 : 128;
+}
+
+bool dmma_pairs(const double* x, int ld) { return ((uintptr_t)x & 15) == 0 && ld % 2 == 0; }
+
+// A kernel's opt-in to its shared memory, which its launcher takes once per process.
+int dmma_attr(const void* fn, int smem) {
+  MB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   return MB_OK;
+}
+
+template <int TILE, bool TA, bool TB, int V>
+int dmma_launch(int m, int n, int k, int nz, double alpha, const double* a, int lda, const double* b, int ldb,
+                double beta, double* out, int ldc, cudaStream_t stream) {
+  static int attr = dmma_attr((const void*)dgemm_dmma_kernel<TILE, TA, TB, V>, Dmma<TILE>::SMEM);
+  if (attr != MB_OK) return attr;
+  const dim3 grid((n + TILE - 1) / TILE, (m + TILE - 1) / TILE, nz);
+  dgemm_dmma_kernel<TILE, TA, TB, V><<<grid, Dmma<TILE>::THREADS, Dmma<TILE>::SMEM, stream>>>(m, n, k, alpha, a, lda, b,
+                                                                                              ldb, beta, out, ldc);
+  MB_LAUNCH_CHECK();
+  return MB_OK;
+}
+
+template <bool TA, bool TB>
+int dmma_gemm(int m, int n, int k, int nz, double alpha, const double* a, int lda, const double* b, int ldb,
+              double beta, double* out, int ldc, cudaStream_t stream) {
+  auto tiles = [&](int t) { return (long long)nz * ((m + t - 1) / t) * ((n + t - 1) / t); };
+  const bool small = dmma_tile(tiles(128), tiles(64)) == 64;
+  // a slice starts at an even k, or its pairs along k are off their boundary
+  const bool even = nz == 1 || (k + nz - 1) / nz % 2 == 0;
+  const bool pairs = even && dmma_pairs(a, lda) && dmma_pairs(b, ldb);
+  if (small) {
+    if (pairs) return dmma_launch<64, TA, TB, 2>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream);
+    return dmma_launch<64, TA, TB, 1>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream);
+  }
+  if (pairs) return dmma_launch<128, TA, TB, 2>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream);
+  return dmma_launch<128, TA, TB, 1>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream);
+}
+
+template <int TILE, int V>
+int syrk_launch(int n, int k, double alpha, const double* a, int lda, double* p, int acc, cudaStream_t stream) {
+  static int attr = dmma_attr((const void*)syrk_packed_dmma_kernel<TILE, V>, Dmma<TILE>::SMEM);
+  if (attr != MB_OK) return attr;
+  const long long t = (n + TILE - 1) / TILE;
+  syrk_packed_dmma_kernel<TILE, V>
+      <<<(unsigned)(t * (t + 1) / 2), Dmma<TILE>::THREADS, Dmma<TILE>::SMEM, stream>>>(n, k, alpha, a, lda, p, acc);
+  MB_LAUNCH_CHECK();
+  return MB_OK;
+}
+
+int dmma_syrk(int n, int k, double alpha, const double* a, int lda, double* p, int acc, cudaStream_t stream) {
+  auto tiles = [&](int t) {
+    const long long q = (n + t - 1) / t;
+    return q * (q + 1) / 2;
+  };
+  const bool small = dmma_tile(tiles(128), tiles(64)) == 64, pairs = dmma_pairs(a, lda);
+  if (small) return pairs ? syrk_launch<64, 2>(n, k, alpha, a, lda, p, acc, stream)
+                          : syrk_launch<64, 1>(n, k, alpha, a, lda, p, acc, stream);
+  return pairs ? syrk_launch<128, 2>(n, k, alpha, a, lda, p, acc, stream)
+               : syrk_launch<128, 1>(n, k, alpha, a, lda, p, acc, stream);
 }
 
 // C = alpha * sum_z part[z] + beta * C, slices summed in order (deterministic).
@@ -338,8 +439,10 @@ extern "C" int mb_dgemm_ws(char transa, char transb, int m, int n, int k, double
   bool ta = (transa == 'T' || transa == 't' || transa == 'C' || transa == 'c');
   bool tb = (transb == 'T' || transb == 't' || transb == 'C' || transb == 'c');
   const bool wide = m > BM && n > BN;  // DMMA engine for all but skinny outputs
-  const int tbm = wide ? DBM : BM, tbn = wide ? DBN : BN;
-  const int tiles = ((n + tbn - 1) / tbn) * ((m + tbm - 1) / tbm);
+  // slices of k are counted in 128- or 64-wide tiles, whatever tile then runs:
+  // the sums' order stays the same
+  const int tb_ = wide ? 128 : BM;
+  const int tiles = ((n + tb_ - 1) / tb_) * ((m + tb_ - 1) / tb_);
   const int target = wide ? 148 : 296;
   int nz = 1;
   if (ws && k >= 512 && tiles < target) {
@@ -348,21 +451,20 @@ extern "C" int mb_dgemm_ws(char transa, char transb, int m, int n, int k, double
     if (nz > 32) nz = 32;
     while (nz > 1 && (size_t)nz * m * n > ws_elems) --nz;
   }
-  dim3 grid((n + tbn - 1) / tbn, (m + tbm - 1) / tbm, nz);
   double* out = nz > 1 ? ws : c;
   if (wide) {
-    MB_TRY(dmma_attrs());
-    if (!ta && !tb) dgemm_dmma_kernel<false, false><<<grid, NT, DMMA_SMEM, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
-    else if (!ta && tb) dgemm_dmma_kernel<false, true><<<grid, NT, DMMA_SMEM, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
-    else if (ta && !tb) dgemm_dmma_kernel<true, false><<<grid, NT, DMMA_SMEM, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
-    else dgemm_dmma_kernel<true, true><<<grid, NT, DMMA_SMEM, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
+    if (!ta && !tb) MB_TRY((dmma_gemm<false, false>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream)));
+    else if (!ta && tb) MB_TRY((dmma_gemm<false, true>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream)));
+    else if (ta && !tb) MB_TRY((dmma_gemm<true, false>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream)));
+    else MB_TRY((dmma_gemm<true, true>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream)));
   } else {
+    const dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM, nz);
     if (!ta && !tb) dgemm_kernel<false, false><<<grid, NT, 0, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
     else if (!ta && tb) dgemm_kernel<false, true><<<grid, NT, 0, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
     else if (ta && !tb) dgemm_kernel<true, false><<<grid, NT, 0, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
     else dgemm_kernel<true, true><<<grid, NT, 0, stream>>>(m, n, k, alpha, a, lda, b, ldb, beta, out, ldc);
+    MB_LAUNCH_CHECK();
   }
-  MB_LAUNCH_CHECK();
   if (nz > 1) {
     long long mn = (long long)m * n;
     int blocks = (int)((mn + 255) / 256);
@@ -387,14 +489,9 @@ int syrk_range(int n, int k0, int k1, double alpha, const double* c, int ldc, do
                cudaStream_t stream) {
   const int k = k1 > k0 ? k1 - k0 : 0;
   const double* a = c + (long long)(k > 0 ? k0 : 0) * ldc;
-  if (n > BM) {
-    dim3 grid((n + DBN - 1) / DBN, (n + DBM - 1) / DBM);
-    MB_TRY(dmma_attrs());
-    syrk_packed_dmma_kernel<<<grid, NT, DMMA_SMEM, stream>>>(n, k, alpha, a, ldc, p, acc ? 1 : 0);
-  } else {
-    dim3 grid((n + BN - 1) / BN, (n + BM - 1) / BM);
-    syrk_packed_kernel<<<grid, NT, 0, stream>>>(n, k, alpha, a, ldc, p, grid.x, acc ? 1 : 0);
-  }
+  if (n > BM) return dmma_syrk(n, k, alpha, a, ldc, p, acc ? 1 : 0, stream);
+  dim3 grid((n + BN - 1) / BN, (n + BM - 1) / BM);
+  syrk_packed_kernel<<<grid, NT, 0, stream>>>(n, k, alpha, a, ldc, p, grid.x, acc ? 1 : 0);
   MB_LAUNCH_CHECK();
   return MB_OK;
 }
