@@ -244,30 +244,38 @@ __global__ void rot_coeff_kernel(int nocc, int nvirt, const double* __restrict__
 // Apply all active rotations to C in the reference order.  Tiles are 16 x 16
 // pairs (occupied block I, virtual block J); tile (I, J) touches columns I
 // (occupied) and J (virtual) only and must follow (I, J-1), which last
-// touched columns I, and (I-1, J), which last touched columns J.  Tiles on one
-// anti-diagonal I + J = t touch disjoint columns, so they run in parallel,
-// and every column still sees its rotations in the sequential sweep's order
-// (occupied i outer, virtual j inner) -- rotations on disjoint column pairs
-// commute exactly, so C is bit-identical to the sequential sweep.
+// touched columns I, and (I-1, J), which last touched columns J.  Rows are
+// independent (a rotation mixes two columns of each row separately) and
+// rotations on disjoint column pairs commute exactly, so any schedule that
+// keeps those two orders gives every column its rotations in the sequential
+// sweep's order (occupied i outer, virtual j inner), and C is bit-identical to
+// the sequential sweep.
 //
-// One cooperative launch per sweep, scheduled as a dataflow graph: rows are
-// independent (a rotation mixes two columns of each row separately), so the
-// work item is (tile (I, J), block rb of CROWS rows), and item (I, J, rb)
-// depends on (I - 1, J, rb) and (I, J - 1, rb) only.  CTAs take items from a
-// queue ordered by anti-diagonal I + J, wait for the item's two predecessors'
-// done flags, rotate, and set the item's own flag -- no grid barrier, so
-// blocks of rows run ahead on later anti-diagonals while others finish the
-// current one.  Every predecessor of an item sits earlier in the queue and
-// was taken by a resident CTA (a CTA takes its next item only while working
-// on the current one), so the smallest unfinished item always has its inputs
-// and the sweep cannot stall; each wait is still bounded (2 s of
-// %globaltimer), after which the kernel raises an abort flag that ends every
-// CTA's loop and sets bit 4 of *err.  A CTA stages the tile's 256
-// coefficients in shared memory (every thread reads them by broadcast) and
-// each thread rotates one row of the tile's 32 columns in registers; the
-// arithmetic of every element is that of the sequential sweep, so C is
-// bit-identical to it.
-constexpr int CROWS = 128;
+// One cooperative launch per sweep, a pipeline of warps.  A CTA takes the task
+// (four occupied blocks, 32 rows); its warp k keeps the 16 occupied columns of
+// block 4 g + k in shared memory, a row a lane, and the virtual blocks
+// J = 0, 1, ... pass through the four warps in registers and shared-memory
+// slots, so a virtual column is read and written in global memory once per 64
+// occupied ones, and an occupied column once per sweep.  Warp 0 waits for block
+// J of the same rows to be released by task (g - 1), warp 3 writes and
+// releases it.  Tasks are taken in ascending g, so a task's predecessor was
+// taken before it by a resident CTA and the pipeline cannot stall; each wait is
+// still bounded (2 s of %globaltimer), after which the kernel raises an abort
+// flag that ends every warp's loop and sets bit 4 of *err.
+//
+// Bound by the FP64 pipe: six operations per rotation and row, no multiply-adds
+// (the sequential order's rounding).  The rotations alone, without columns or
+// waits, run at 15.4 T operations a second (of 17.5 for bare additions), 2.5 ms
+// at 3072 orbitals with 2048 occupied.  One B200, ms (before: a CTA per 16 x 16
+// tile and 128 rows, two flags a tile): 0.40 (0.48) at 1026 orbitals, 1.16 (1.37)
+// at 2046, 3.31 (3.85) at 3072, two thirds occupied.
+// With a flag in global memory per 16 x 16 tile the waits took a third of the
+// time (a release, a poll and a load through L2 per tile and row block), whether
+// a CTA, a warp or a warp with two rows a lane took a tile.
+constexpr int SWARPS = 4;     // warps per CTA: occupied blocks of a task
+constexpr int SROWS = 32;     // rows of a task
+constexpr int SSLOT = 2;      // virtual blocks between a warp and the next
+constexpr int STASK = 16;     // tasks posted: more than the warps can be apart
 constexpr unsigned long long kFlowWaitNs = 2000000000ull;
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
@@ -284,167 +292,205 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// sync[0]: queue head; sync[1]: abort; sync[2 + (I * ntile_v + J) * nrb + rb]:
-// done flag of item (I, J, rb).  All zero at launch.
-__global__ void __launch_bounds__(CROWS, 3) rot_sweep_kernel(int n, int nocc, int nvirt, double* __restrict__ c,
-                                                            const double* __restrict__ alpha,
-                                                            const double* __restrict__ beta,
-                                                            const unsigned int* __restrict__ tile_cnt, int ntile_o,
-                                                            int ntile_v, int* __restrict__ sync,
-                                                            int* __restrict__ err) {
-  __shared__ double2 s_ab[2][RT * RT];
-  __shared__ double s_xi[RT][CROWS];   // the occupied values of each thread's row
-  __shared__ int s_next[4];            // the next item: I, J, rb, valid
-  __shared__ int s_go;                 // 0 once the sweep is aborted
-  const int nrb = (n + CROWS - 1) / CROWS;
-  const int ndiag = ntile_o + ntile_v - 1;
+struct SweepShared {
+  double2 ab[SWARPS][2][RT * RT];              // two tiles' coefficients a warp
+  double xi[SWARPS][RT][SROWS];                // the occupied columns
+  double slot[SWARPS - 1][SSLOT][RT][SROWS];   // virtual blocks on their way to the next warp
+  int task[STASK];
+  volatile int put[SWARPS - 1], got[SWARPS - 1];  // blocks written to and read from the slots, of all tasks
+  volatile int posted;                            // tasks posted
+};
+
+// Lane 0 of a warp waits until *p > v, bounded; 0 once the sweep is aborted.  The
+// fence, and the __syncwarp that every caller puts behind it, order what the
+// posting warp did first before what this warp's lanes do next.
+__device__ __forceinline__ int sweep_wait(const volatile int* p, int v, int* abort_flag, int* err) {
+  if (*p > v) {
+    __threadfence_block();
+    return 1;
+  }
+  const unsigned long long t0 = global_ns();
+  for (unsigned it = 1; *p <= v; ++it) {
+    __nanosleep(40);
+    if ((it & 1023u) == 0 && (ld_acquire_gpu(abort_flag) != 0 || global_ns() - t0 > kFlowWaitNs)) {
+      atomicExch(abort_flag, 1);
+      if (err) atomicOr(err, 4);
+      return 0;
+    }
+  }
+  __threadfence_block();
+  return 1;
+}
+
+// sync[0]: queue head; sync[1]: abort; sync[2 + g * nrb + rb]: how many virtual
+// blocks task (g, rb) has released.  All zero at launch.
+__global__ void __launch_bounds__(32 * SWARPS, 3) rot_sweep_kernel(int n, int nocc, int nvirt, double* __restrict__ c,
+                                                                  const double* __restrict__ alpha,
+                                                                  const double* __restrict__ beta,
+                                                                  const unsigned int* __restrict__ tile_cnt,
+                                                                  int ntile_o, int ntile_v, int* __restrict__ sync,
+                                                                  int* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char sweep_sh[];
+  SweepShared& S = *reinterpret_cast<SweepShared*>(sweep_sh);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nrb = (n + SROWS - 1) / SROWS, ngroup = (ntile_o + SWARPS - 1) / SWARPS;
+  const int ntask = ngroup * nrb;
   int* const head = sync;
   int* const abort_flag = sync + 1;
   int* const done = sync + 2;
-  constexpr int PER = RT * RT / CROWS;  // coefficients each thread stages
-  // thread 0's cursor over the queue: items of anti-diagonal t are
-  // [t_start, t_start + width(t) * nrb), taken in increasing order
-  int t_cur = 0;
-  long long t_start = 0;
-  auto width = [&](int t) {
-    const int jlo = t - (ntile_o - 1) > 0 ? t - (ntile_o - 1) : 0;
-    const int jhi = t < ntile_v - 1 ? t : ntile_v - 1;
-    return jhi - jlo + 1;
-  };
-  auto take = [&]() {  // thread 0: the next item into s_next
-    const long long q = atomicAdd(head, 1);
-    while (t_cur < ndiag && q >= t_start + (long long)width(t_cur) * nrb) {
-      t_start += (long long)width(t_cur) * nrb;
-      ++t_cur;
-    }
-    if (t_cur >= ndiag) {
-      s_next[3] = 0;
-      return;
-    }
-    const long long loc = q - t_start;
-    const int jlo = t_cur - (ntile_o - 1) > 0 ? t_cur - (ntile_o - 1) : 0;
-    const int J = jlo + (int)(loc / nrb);
-    s_next[0] = t_cur - J;
-    s_next[1] = J;
-    s_next[2] = (int)(loc % nrb);
-    s_next[3] = 1;
-  };
-  auto stage = [&](int I, int J, double2* pre) {
-    const long long tb = ((long long)I * ntile_v + J) * (RT * RT);
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int e = threadIdx.x + q * CROWS;
-      pre[q] = make_double2(alpha[tb + e], beta[tb + e]);
-    }
-  };
-  if (threadIdx.x == 0) {
-    take();
-    s_go = 1;
-  }
+  if (threadIdx.x < SWARPS - 1) S.put[threadIdx.x] = S.got[threadIdx.x] = 0;
+  if (threadIdx.x == 0) S.posted = 0;
   __syncthreads();
-  int I = s_next[0], J = s_next[1], rb = s_next[2], valid = s_next[3];
-  int buf = 0;
-  if (valid) {
-    double2 pre[PER];
-    stage(I, J, pre);
+  // the coefficients of tile (I, J) into buffer J & 1, asynchronously
+  auto stage = [&](int I, int J) {
+    if (I < ntile_o && J < ntile_v) {
+      const long long tb = ((long long)I * ntile_v + J) * (RT * RT);
 #pragma unroll
-    for (int q = 0; q < PER; ++q) s_ab[0][threadIdx.x + q * CROWS] = pre[q];
-  }
-  __syncthreads();
-  while (valid) {
-    // the next item, and its coefficients in flight while this one runs
-    if (threadIdx.x == 0) take();
-    __syncthreads();
-    const int nI = s_next[0], nJ = s_next[1], nrb_ = s_next[2], nvalid = s_next[3];
-    double2 pre[PER];
-    if (nvalid) stage(nI, nJ, pre);
-    // wait for the item's predecessors
-    if (threadIdx.x == 0) {
-      bool ok = true;
-      const int* deps[2] = {I > 0 ? done + ((long long)(I - 1) * ntile_v + J) * nrb + rb : nullptr,
-                            J > 0 ? done + ((long long)I * ntile_v + (J - 1)) * nrb + rb : nullptr};
-      for (int d = 0; d < 2 && ok; ++d) {
-        if (!deps[d]) continue;
-        const unsigned long long t0 = global_ns();
-        while (ld_acquire_gpu(deps[d]) == 0) {
-          if (ld_acquire_gpu(abort_flag) != 0 || global_ns() - t0 > kFlowWaitNs) {
-            ok = false;
-            break;
-          }
-          __nanosleep(32);
-        }
-      }
-      if (!ok) {
-        atomicExch(abort_flag, 1);
-        if (err) atomicOr(err, 4);
-        s_go = 0;
+      for (int q = 0; q < RT * RT / 32; ++q) {
+        const int e = lane + 32 * q;
+        const unsigned d = (unsigned)__cvta_generic_to_shared(&S.ab[warp][J & 1][e]);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(alpha + tb + e) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d + 8), "l"(beta + tb + e) : "memory");
       }
     }
-    __syncthreads();
-    if (!s_go) break;
-    const int r = rb * CROWS + threadIdx.x;
-    if (tile_cnt[I * ntile_v + J] != 0 && r < n) {
-      const int i0 = I * RT, j0 = J * RT;
-      const double2* ab = s_ab[buf];
-      // All 32 values of the thread's row are loaded at once (one memory
-      // latency per item; past L1, which may hold lines another SM has
-      // since rewritten): the 16 virtual ones stay in registers for the
-      // tile, the 16 occupied ones wait in shared memory, since occupied
-      // column u is touched by row u of the tile only.  A skipped pair
-      // carries the identity (alpha 1, beta 0): applying it leaves both
-      // values equal (1*a + 0*b == a), so the rotations run without a
-      // branch, each row's coefficients read from shared memory ahead of
-      // its dependent chain.
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  int blocks = 0;  // virtual blocks this warp has passed on, of all tasks
+  for (int seq = 0;; ++seq) {
+    // warp 0 takes a task, the others follow
+    int task = 0;
+    if (lane == 0) {
+      if (warp == 0) {
+        task = atomicAdd(head, 1);
+        S.task[seq % STASK] = task;
+        __threadfence_block();
+        S.posted = seq + 1;
+      } else if (sweep_wait(&S.posted, seq, abort_flag, err)) {
+        task = S.task[seq % STASK];
+      } else {
+        task = ntask;
+      }
+    }
+    task = __shfl_sync(0xffffffffu, task, 0);
+    if (task >= ntask) break;
+    const int g = task / nrb, rb = task % nrb, I = g * SWARPS + warp;
+    const int i0 = I * RT, r = rb * SROWS + lane;
+    const bool row = r < n;
+    const int* pred = done + (long long)(g - 1) * nrb + rb;
+    int* own = done + (long long)g * nrb + rb;
+    int known = g > 0 ? 0 : ntile_v;  // warp 0: blocks released by the predecessor, as last seen
+    __syncwarp();
+    stage(I, 0);
+#pragma unroll
+    for (int u = 0; u < RT; ++u)
+      S.xi[warp][u][lane] = (row && i0 + u < nocc) ? __ldcg(c + (long long)(i0 + u) * n + r) : 0.0;
+    bool ok = true;
+    for (int J = 0; J < ntile_v; ++J, ++blocks) {
+      stage(I, J + 1);
       double xj[RT];
-#pragma unroll
-      for (int u = 0; u < RT; ++u)
-        s_xi[u][threadIdx.x] = (i0 + u < nocc) ? __ldcg(c + (long long)(i0 + u) * n + r) : 0.0;
-#pragma unroll
-      for (int v = 0; v < RT; ++v) xj[v] = (j0 + v < nvirt) ? __ldcg(c + (long long)(nocc + j0 + v) * n + r) : 0.0;
-#pragma unroll 1
-      for (int u = 0; u < RT; ++u) {
-        double x = s_xi[u][threadIdx.x];
-        double2 w[RT];
-#pragma unroll
-        for (int v = 0; v < RT; ++v) w[v] = ab[u * RT + v];
-#pragma unroll
-        for (int v = 0; v < RT; ++v) {
-          const double b = xj[v];
-          const double na = DADD(DMUL(w[v].x, x), DMUL(w[v].y, b));
-          xj[v] = DSUB(DMUL(w[v].x, b), DMUL(w[v].y, x));
-          x = na;
+      const int slot = blocks % SSLOT;
+      if (warp == 0) {
+        if (known <= J) {
+          int rel = 0;
+          if (lane == 0) {
+            rel = ld_acquire_gpu(pred);
+            const unsigned long long t0 = rel <= J ? global_ns() : 0;
+            while (rel <= J) {
+              if (ld_acquire_gpu(abort_flag) != 0 || global_ns() - t0 > kFlowWaitNs) {
+                rel = -1;
+                atomicExch(abort_flag, 1);
+                if (err) atomicOr(err, 4);
+                break;
+              }
+              __nanosleep(32);
+              rel = ld_acquire_gpu(pred);
+            }
+          }
+          known = __shfl_sync(0xffffffffu, rel, 0);
+          __syncwarp();
+          ok = known > J;
         }
-        s_xi[u][threadIdx.x] = x;
+        // past L1, which may hold lines another SM has since rewritten
+        if (ok) {
+          const double* cj = c + (long long)(nocc + J * RT) * n + r;
+#pragma unroll
+          for (int v = 0; v < RT; ++v) xj[v] = (row && J * RT + v < nvirt) ? __ldcg(cj + (long long)v * n) : 0.0;
+        }
+      } else {
+        int w = 1;
+        if (lane == 0) w = sweep_wait(&S.put[warp - 1], blocks, abort_flag, err);
+        ok = __shfl_sync(0xffffffffu, w, 0) != 0;
+        __syncwarp();
+        if (ok) {
+#pragma unroll
+          for (int v = 0; v < RT; ++v) xj[v] = S.slot[warp - 1][slot][v][lane];
+          __syncwarp();  // the slot is read
+          if (lane == 0) {
+            __threadfence_block();
+            S.got[warp - 1] = blocks + 1;
+          }
+        }
       }
+      if (!ok) break;
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // tile J's coefficients
+      __syncwarp();
+      if (I < ntile_o && tile_cnt[I * ntile_v + J] != 0) {
+        const double2* ab = S.ab[warp][J & 1];
+        // A skipped pair carries the identity (alpha 1, beta 0): applying it
+        // leaves both values equal (1*a + 0*b == a), so the rotations run
+        // without a branch, their coefficients read ahead of the dependent
+        // chain.
+#pragma unroll 1
+        for (int u = 0; u < RT; ++u) {
+          double x = S.xi[warp][u][lane];
+          double2 w[RT];
 #pragma unroll
-      for (int u = 0; u < RT; ++u)
-        if (i0 + u < nocc) c[(long long)(i0 + u) * n + r] = s_xi[u][threadIdx.x];
+          for (int v = 0; v < RT; ++v) w[v] = ab[u * RT + v];
 #pragma unroll
-      for (int v = 0; v < RT; ++v)
-        if (j0 + v < nvirt) c[(long long)(nocc + j0 + v) * n + r] = xj[v];
-    }
-    if (nvalid) {
+          for (int v = 0; v < RT; ++v) {
+            const double b = xj[v];
+            const double na = DADD(DMUL(w[v].x, x), DMUL(w[v].y, b));
+            xj[v] = DSUB(DMUL(w[v].x, b), DMUL(w[v].y, x));
+            x = na;
+          }
+          S.xi[warp][u][lane] = x;
+        }
+      }
+      if (warp < SWARPS - 1) {
+        int w = 1;  // the slot is free once the next warp has read block `blocks - SSLOT`
+        if (lane == 0) w = sweep_wait(&S.got[warp], blocks - SSLOT, abort_flag, err);
+        ok = __shfl_sync(0xffffffffu, w, 0) != 0;
+        __syncwarp();
+        if (!ok) break;
 #pragma unroll
-      for (int q = 0; q < PER; ++q) s_ab[buf ^ 1][threadIdx.x + q * CROWS] = pre[q];
+        for (int v = 0; v < RT; ++v) S.slot[warp][slot][v][lane] = xj[v];
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence_block();
+          S.put[warp] = blocks + 1;
+        }
+      } else {
+        double* cj = c + (long long)(nocc + J * RT) * n + r;
+#pragma unroll
+        for (int v = 0; v < RT; ++v)
+          if (row && J * RT + v < nvirt) cj[(long long)v * n] = xj[v];
+        __syncwarp();  // the block's rows are written
+        if (lane == 0) st_release_gpu(own, J + 1);
+      }
     }
-    __syncthreads();  // the item's rows are written; the next buffer is filled
-    if (threadIdx.x == 0) {
-      __threadfence();
-      st_release_gpu(done + ((long long)I * ntile_v + J) * nrb + rb, 1);
-    }
-    buf ^= 1;
-    I = nI;
-    J = nJ;
-    rb = nrb_;
-    valid = nvalid;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    if (!ok) break;
+#pragma unroll
+    for (int u = 0; u < RT; ++u)
+      if (row && i0 + u < nocc) c[(long long)(i0 + u) * n + r] = S.xi[warp][u][lane];
   }
 }
 
-// sync ints a sweep needs: the queue head, the abort flag and a done flag per
-// (tile, row block) item.
+// sync ints a sweep needs: the queue head, the abort flag and a count per
+// (group of occupied blocks, row block).
 size_t flow_sync_ints(int n, int nocc) {
-  const size_t to = (size_t)(nocc + RT - 1) / RT, tv = (size_t)(n - nocc + RT - 1) / RT;
-  return 2 + to * tv * (size_t)((n + CROWS - 1) / CROWS);
+  const size_t to = (size_t)(nocc + RT - 1) / RT;
+  return 2 + (to + SWARPS - 1) / SWARPS * (size_t)((n + SROWS - 1) / SROWS);
 }
 
 int launch_wavefronts(int n, int nocc, int nvirt, double* c, const double* al, const double* be,
@@ -455,15 +501,17 @@ int launch_wavefronts(int n, int nocc, int nvirt, double* c, const double* al, c
     int dev = 0, sms = 0, per = 0;
     MB_CUDA(cudaGetDevice(&dev));
     MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rot_sweep_kernel, CROWS, 0));
+    MB_CUDA(cudaFuncSetAttribute(rot_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(SweepShared)));
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rot_sweep_kernel, 32 * SWARPS, sizeof(SweepShared)));
     if (per < 1) return mb_set_error(MB_ERR_CUDA, "rot_sweep_kernel: no CTA fits on an SM");
     grid = sms * per;
   }
   (void)act;  // skipped pairs carry the identity rotation in al / be
   MB_CUDA(cudaMemsetAsync(sync, 0, sizeof(int) * flow_sync_ints(n, nocc), stream));
   void* args[] = {&n, &nocc, &nvirt, &c, &al, &be, &tcnt, &to, &tv, &sync, &err};
-  // cooperative: every CTA resident, which the dataflow queue relies on
-  MB_CUDA(cudaLaunchCooperativeKernel((void*)rot_sweep_kernel, grid, CROWS, args, 0, stream));
+  // cooperative: every CTA resident, which the pipeline relies on
+  MB_CUDA(cudaLaunchCooperativeKernel((void*)rot_sweep_kernel, grid, 32 * SWARPS, args, sizeof(SweepShared), stream));
   mb_count_launch();
   return MB_OK;
 }
