@@ -35,105 +35,146 @@ __device__ __forceinline__ double ipow(double x, int m) {
   for (int i = 0; i < m; ++i) r *= x;
   return r;
 }
-__device__ __forceinline__ int indx_(int i, int j) { return i > j ? (i * (i - 1)) / 2 + j : (j * (j - 1)) / 2 + i; }
 
-// ------------------------------------------------------------ overlaps
-struct Ovl { double a[8], b[8], sa, sb; int isp, ips; };
-
-__device__ void aintgs(Ovl& o, double x, int k) {
-  const double c = exp(-x);
-  o.a[1] = c / x;
-  for (int i = 1; i <= k; ++i) o.a[i + 1] = (o.a[i] * i + c) / x;
+// The pair functions below are templates on the two atoms' orbital counts (1 or 4):
+// with constant loop bounds every array is in registers (before, 3 KB of local
+// memory a thread; hcore_pairs of (H2O)512 took 8.5 ms, now 1.4, one B200).
+// by_kind picks the instance of a pair.  Where a sum of two products could be
+// contracted either way, it is written out, so a value does not depend on the
+// kernel its function is inlined into.
+template <int N>
+struct Orb {
+  static constexpr int n = N;
+};
+template <class F>
+__device__ __forceinline__ void by_kind(int ni, int nj, F&& f) {
+  if (c_P.el[ni].natorb == 1) {
+    if (c_P.el[nj].natorb == 1) f(Orb<1>{}, Orb<1>{});
+    else f(Orb<1>{}, Orb<4>{});
+  } else {
+    if (c_P.el[nj].natorb == 1) f(Orb<4>{}, Orb<1>{});
+    else f(Orb<4>{}, Orb<4>{});
+  }
 }
 
-__device__ void bintgs(Ovl& o, double x, int k) {
+// ------------------------------------------------------------ overlaps
+template <int K>
+struct Ovl {
+  double a[K + 2], b[K + 2], sa, sb;  // from 1
+};
+
+template <int K>
+__device__ __forceinline__ void aintgs(Ovl<K>& o, double x) {
+  const double c = exp(-x);
+  o.a[1] = c / x;
+#pragma unroll
+  for (int i = 1; i <= K; ++i) o.a[i + 1] = (o.a[i] * i + c) / x;
+}
+
+template <int K>
+__device__ __forceinline__ void bintgs(Ovl<K>& o, double x) {
   const double ax = fabs(x);
   int last = 0, mode = 0;
   if (ax > 3.0) mode = 0;
-  else if (ax > 2.0) { if (k <= 10) mode = 0; else { last = 15; mode = 1; } }
-  else if (ax > 1.0) { if (k <= 7) mode = 0; else { last = 12; mode = 1; } }
-  else if (ax > 0.5) { if (k <= 5) mode = 0; else { last = 7; mode = 1; } }
+  else if (ax > 2.0) { if (K <= 10) mode = 0; else { last = 15; mode = 1; } }
+  else if (ax > 1.0) { if (K <= 7) mode = 0; else { last = 12; mode = 1; } }
+  else if (ax > 0.5) { if (K <= 5) mode = 0; else { last = 7; mode = 1; } }
   else if (ax <= 1.0e-6) mode = 2;
   else { last = 6; mode = 1; }
   if (mode == 0) {
     const double expx = exp(x), expmx = 1.0 / expx;
     o.b[1] = (expx - expmx) / x;
-    for (int i = 1; i <= k; ++i) o.b[i + 1] = (i * o.b[i] + ((i & 1) ? -1.0 : 1.0) * expx - expmx) / x;
+#pragma unroll
+    for (int i = 1; i <= K; ++i) o.b[i + 1] = (i * o.b[i] + ((i & 1) ? -1.0 : 1.0) * expx - expmx) / x;
   } else if (mode == 1) {
-    for (int i = 0; i <= k; ++i) {
-      double y = 0.0;
-      for (int m = 0; m <= last; ++m) {
-        const double xf = m != 0 ? c_fact[m] : 1.0;
-        y = y + ipow(-x, m) * (double)(2 * ((m + i + 1) % 2)) / (xf * (double)(m + i + 1));
-      }
-      o.b[i + 1] = y;
+    // sum over m of (-x)^m 2 / (m! (m + i + 1)), m + i even, in ascending m
+#pragma unroll
+    for (int i = 0; i <= K; ++i) o.b[i + 1] = 0.0;
+    double pw = 1.0;
+    for (int m = 0; m <= last; ++m) {
+      const double xf = m != 0 ? c_fact[m] : 1.0;
+#pragma unroll
+      for (int i = 0; i <= K; ++i)
+        if (((m + i) & 1) == 0) o.b[i + 1] = o.b[i + 1] + pw * 2.0 / (xf * (double)(m + i + 1));
+      pw *= -x;
     }
   } else {
-    for (int i = 0; i <= k; ++i) o.b[i + 1] = (double)(2 * ((i + 1) % 2)) / (i + 1.0);
+#pragma unroll
+    for (int i = 0; i <= K; ++i) o.b[i + 1] = (double)(2 * ((i + 1) % 2)) / (i + 1.0);
   }
 }
 
-__device__ void set_ovl(Ovl& o, double s1, double s2, int na, int nb, double rab, int ii) {
-  if (na <= nb) { o.isp = 1; o.ips = 2; o.sa = s1; o.sb = s2; }
-  else { o.isp = 2; o.ips = 1; o.sa = s2; o.sb = s1; }
-  int j = ii + 2;
-  if (ii > 3) j = j - 1;
-  aintgs(o, 0.5 * rab * (o.sa + o.sb), j - 1);
-  bintgs(o, 0.5 * rab * (o.sb - o.sa), j - 1);
+// swap: the first atom has the higher atomic number
+template <int K>
+__device__ __forceinline__ void set_ovl(Ovl<K>& o, double s1, double s2, bool swap, double rab) {
+  o.sa = swap ? s2 : s1;
+  o.sb = swap ? s1 : s2;
+  aintgs(o, 0.5 * rab * (o.sa + o.sb));
+  bintgs(o, 0.5 * rab * (o.sb - o.sa));
 }
 
-// s[la][lb][m] (1-based) for first-row sp atoms (diat2 cases 1, 2, 4)
-__device__ void diat2(int na, double esa, double epa, double r12, int nb, double esb, double epb,
-                      double s[3][3][3]) {
-  for (int x = 0; x < 27; ++x) (&s[0][0][0])[x] = 0.0;
-  const int ina = na == 1 ? 1 : (na == 6 ? 4 : 6), inb = nb == 1 ? 1 : (nb == 6 ? 4 : 6);
-  const int jmax = ina > inb ? ina : inb, jmin = ina < inb ? ina : inb;
-  const int ii = jmax == 1 ? 1 : (jmin == 1 ? 2 : 4);
+// Local overlaps of first-row sp atoms (diat2 cases 1, 2, 4).
+struct Overlap {
+  double ss, sp, ps, pps, ppp;  // first atom's orbital first; pps sigma, ppp pi
+};
+template <int NI, int NJ>
+__device__ __forceinline__ Overlap diat2(int na, double esa, double epa, double r12, int nb, double esb, double epb) {
+  Overlap s{0.0, 0.0, 0.0, 0.0, 0.0};
   const double rab = r12 / PM7_A0;
-  Ovl o;
-  const double* a = o.a;
-  const double* b = o.b;
-  if (ii == 2) {
-    set_ovl(o, esa, esb, na, nb, rab, ii);
+  if constexpr (NI == 1 && NJ == 1) {
+    Ovl<2> o;
+    const double *a = o.a, *b = o.b;
+    set_ovl(o, esa, esb, na > nb, rab);
+    s.ss = 0.25 * sqrt(ipow(o.sa * o.sb * rab * rab, 3)) * (a[3] * b[1] - b[3] * a[1]);
+  } else if constexpr (NI == 1 || NJ == 1) {
+    Ovl<3> o;
+    const double *a = o.a, *b = o.b;
+    set_ovl(o, esa, esb, NI > 1, rab);
     const double rab4 = ipow(rab, 4) * 0.125;
     double w = sqrt(ipow(o.sa, 3) * ipow(o.sb, 5)) * rab4;
-    s[1][1][1] = w * sqrt(1.0 / 3.0) * (a[4] * b[1] - b[4] * a[1] + a[3] * b[2] - b[3] * a[2]);
-    if (na > 1) set_ovl(o, epa, esb, na, nb, rab, ii);
-    if (nb > 1) set_ovl(o, esa, epb, na, nb, rab, ii);
+    s.ss = w * sqrt(1.0 / 3.0) * (a[4] * b[1] - b[4] * a[1] + a[3] * b[2] - b[3] * a[2]);
+    set_ovl(o, NI > 1 ? epa : esa, NI > 1 ? esb : epb, NI > 1, rab);
     w = sqrt(ipow(o.sa, 3) * ipow(o.sb, 5)) * rab4;
-    s[o.isp][o.ips][1] = w * (a[3] * b[1] - b[3] * a[1] + a[4] * b[2] - b[4] * a[2]);
-  } else if (ii == 4) {
-    set_ovl(o, esa, esb, na, nb, rab, ii);
+    const double v = w * (a[3] * b[1] - b[3] * a[1] + a[4] * b[2] - b[4] * a[2]);
+    if (NI > 1) s.ps = v;
+    else s.sp = v;
+  } else {
+    Ovl<4> o;
+    const double *a = o.a, *b = o.b;
+    const bool swap = na > nb;
+    set_ovl(o, esa, esb, swap, rab);
     const double rab4 = ipow(rab, 5) * 0.0625;
     double w = sqrt(ipow(o.sa * o.sb, 5)) * rab4;
-    s[1][1][1] = w * (a[5] * b[1] + b[5] * a[1] - 2.0 * a[3] * b[3]) / 3.0;
-    set_ovl(o, esa, epb, na, nb, rab, ii);
-    if (na > nb) set_ovl(o, epa, esb, na, nb, rab, ii);
+    s.ss = w * (a[5] * b[1] + b[5] * a[1] - 2.0 * a[3] * b[3]) / 3.0;
+    set_ovl(o, swap ? epa : esa, swap ? esb : epb, swap, rab);
     w = sqrt(ipow(o.sa * o.sb, 5)) * rab4;
     const double rt3 = 1.0 / sqrt(3.0);
     double d = a[4] * (b[1] - b[3]) - a[2] * (b[3] - b[5]);
     double e = b[4] * (a[1] - a[3]) - b[2] * (a[3] - a[5]);
-    s[o.isp][o.ips][1] = w * rt3 * (d + e);
-    set_ovl(o, epa, esb, na, nb, rab, ii);
-    if (na > nb) set_ovl(o, esa, epb, na, nb, rab, ii);
+    const double u = w * rt3 * (d + e);
+    set_ovl(o, swap ? esa : epa, swap ? epb : esb, swap, rab);
     w = sqrt(ipow(o.sa * o.sb, 5)) * rab4;
     d = a[4] * (b[1] - b[3]) - a[2] * (b[3] - b[5]);
     e = b[4] * (a[1] - a[3]) - b[2] * (a[3] - a[5]);
-    s[o.ips][o.isp][1] = w * rt3 * (d - e);
-    set_ovl(o, epa, epb, na, nb, rab, ii);
+    const double v = w * rt3 * (d - e);
+    s.sp = swap ? v : u;
+    s.ps = swap ? u : v;
+    set_ovl(o, epa, epb, swap, rab);
     w = sqrt(ipow(o.sa * o.sb, 5)) * rab4;
-    s[2][2][1] = -w * (b[3] * (a[5] + a[1]) - a[3] * (b[5] + b[1]));
-    s[2][2][2] = 0.5 * w * (a[5] * (b[1] - b[3]) - b[5] * (a[1] - a[3]) - a[3] * b[1] + b[3] * a[1]);
-  } else {
-    set_ovl(o, esa, esb, na, nb, rab, ii);
-    s[1][1][1] = 0.25 * sqrt(ipow(o.sa * o.sb * rab * rab, 3)) * (a[3] * b[1] - b[3] * a[1]);
+    s.pps = -w * (b[3] * (a[5] + a[1]) - a[3] * (b[5] + b[1]));
+    s.ppp = 0.5 * w * (a[5] * (b[1] - b[3]) - b[5] * (a[1] - a[3]) - a[3] * b[1] + b[3] * a[1]);
   }
+  return s;
 }
 
-// Resonance block di[i][j] (1-based orbitals: s, px, py, pz) of atom i with
-// atom j at xj - xi.
-__device__ void h1elec(int ni, int nj, const double* xi, const double* xj, double di[5][5]) {
-  for (int x = 0; x < 25; ++x) (&di[0][0])[x] = 0.0;
+// Resonance block di[a][b] (orbitals s, px, py, pz) of atom i (a) with atom j (b)
+// at xj - xi.
+template <int NI, int NJ>
+__device__ __forceinline__ void h1elec(int ni, int nj, const double* xi, const double* xj, double (&di)[NI][NJ]) {
+#pragma unroll
+  for (int a = 0; a < NI; ++a)
+#pragma unroll
+    for (int b = 0; b < NJ; ++b) di[a][b] = 0.0;
   const double x2 = xj[0] - xi[0], y2 = xj[1] - xi[1], z2 = xj[2] - xi[2];
   const double rr = x2 * x2 + y2 * y2 + z2 * z2;
   if (rr > 1.0e4 || rr >= 225.0) return;  // cutofs (h1elec) and cutof1 (diat)
@@ -146,39 +187,22 @@ __device__ void h1elec(int ni, int nj, const double* xi, const double* xj, doubl
   else if (z2 == 0.0) { ca = 0.0; cb = 0.0; sa = 0.0; sb = 0.0; }
   else { ca = 1.0; cb = 1.0; sa = 0.0; sb = 0.0; }
   if (r < 0.001) return;
-  // c[L][slot][m] for L = s (1), p (2); slot -> orbital: s 3->1; p 2->py, 3->pz, 4->px
-  double c[3][5][5];
-  for (int x = 0; x < 75; ++x) (&c[0][0][0])[x] = 0.0;
-  c[1][3][3] = 1.0;
-  const int nij = c_P.el[ni].natorb > c_P.el[nj].natorb ? c_P.el[ni].natorb : c_P.el[nj].natorb;
-  if (nij >= 2) {
-    c[2][4][4] = ca * cb; c[2][4][3] = ca * sb; c[2][4][2] = -sa;
-    c[2][3][4] = -sb;     c[2][3][3] = cb;      c[2][3][2] = 0.0;
-    c[2][2][4] = sa * cb; c[2][2][3] = sa * sb; c[2][2][2] = ca;
-  }
-  double s[3][3][3];
-  diat2(ni, c_P.el[ni].zs, c_P.el[ni].zp, r, nj, c_P.el[nj].zs, c_P.el[nj].zp, s);
-  const int orb[3][5] = {{0, 0, 0, 0, 0}, {0, 0, 0, 1, 0}, {0, 0, 3, 4, 2}};
-  for (int i = 1; i <= 2; ++i) {
-    const int kmin = 4 - i, kmax = 2 + i;
-    for (int j = 1; j <= 2; ++j) {
-      const double aa = j == 2 ? -1.0 : 1.0, bb = 1.0;
-      const int lmin = 4 - j, lmax = 2 + j;
-      for (int k = kmin; k <= kmax; ++k)
-        for (int l = lmin; l <= lmax; ++l) {
-          const int ii = orb[i][k], jj = orb[j][l];
-          if (ii == 0 || jj == 0) continue;
-          di[ii][jj] = s[i][j][1] * (c[i][k][3] * c[j][l][3]) * aa +
-                       s[i][j][2] * (c[i][k][4] * c[j][l][4] + c[i][k][2] * c[j][l][2]) * bb +
-                       s[i][j][3] * (0.0 + 0.0);
-        }
+  // px, py, pz along sigma, pi, pi'
+  const double cs[4] = {0.0, ca * sb, sa * sb, cb}, cp[4] = {0.0, ca * cb, sa * cb, -sb}, cq[4] = {0.0, -sa, ca, 0.0};
+  const Pm7Elem& A = c_P.el[ni];
+  const Pm7Elem& B = c_P.el[nj];
+  const Overlap s = diat2<NI, NJ>(ni, A.zs, A.zp, r, nj, B.zs, B.zp);
+#pragma unroll
+  for (int a = 0; a < NI; ++a)
+#pragma unroll
+    for (int b = 0; b < NJ; ++b) {
+      double v;
+      if (a == 0 && b == 0) v = s.ss;
+      else if (a == 0) v = -(s.sp * cs[b]);
+      else if (b == 0) v = s.ps * cs[a];
+      else v = __fma_rn(s.ppp, __fma_rn(cp[a], cp[b], __dmul_rn(cq[a], cq[b])), -__dmul_rn(s.pps, __dmul_rn(cs[a], cs[b])));
+      di[a][b] = v * ((a == 0 ? A.betas : A.betap) * 0.5 + (b == 0 ? B.betas : B.betap) * 0.5);
     }
-  }
-  double bi[5], bj[5];
-  bi[1] = c_P.el[ni].betas * 0.5; bi[2] = bi[3] = bi[4] = c_P.el[ni].betap * 0.5;
-  bj[1] = c_P.el[nj].betas * 0.5; bj[2] = bj[3] = bj[4] = c_P.el[nj].betap * 0.5;
-  for (int j = 1; j <= c_P.el[nj].natorb; ++j)
-    for (int i = 1; i <= c_P.el[ni].natorb; ++i) di[i][j] = di[i][j] * (bi[i] + bj[j]);
 }
 
 // ------------------------------------------------------- local integrals
@@ -188,25 +212,26 @@ __device__ __forceinline__ void to_point(double r, double* point, double* cst) {
 }
 
 // 22 local-frame repulsion integrals (reppd, l_feather) and G_AB.
-__device__ void reppd(int ni, int nj, double rij, double ri[23], double* gab) {
+template <int NI, int NJ>
+__device__ __forceinline__ void reppd(int ni, int nj, double rij, double ri[23], double* gab) {
   const double ev1 = PM7_EV / 2, ev2 = ev1 / 2, ev3 = ev2 / 2, ev4 = ev3 / 2, td = 2.0, pp = 0.5;
+#pragma unroll
   for (int i = 0; i < 23; ++i) ri[i] = 0.0;
   const Pm7Elem& A = c_P.el[ni];
   const Pm7Elem& B = c_P.el[nj];
   const double r = rij / PM7_A0;
-  const bool si = A.natorb >= 3, sj = B.natorb >= 3;
+  constexpr bool si = NI == 4, sj = NJ == 4;
+  const double rsq = __dmul_rn(r, r);
   double aee = A.po9 + B.po9;
-  aee = aee * aee;
-  *gab = PM7_EV / sqrt(r * r + aee);
+  *gab = PM7_EV / sqrt(__fma_rn(aee, aee, rsq));
   aee = pp / A.am + pp / B.am;
-  aee = aee * aee;
-  if (!si && !sj) {
-    ri[1] = PM7_EV / sqrt(r * r + aee);
-  } else if (si && !sj) {
+  aee = __dmul_rn(aee, aee);
+  if constexpr (!si && !sj) {
+    ri[1] = PM7_EV / sqrt(rsq + aee);
+  } else if constexpr (si && !sj) {
     const double da = A.dd, qa = A.qq * td;
     double ade = pp / A.ad + pp / B.am; ade *= ade;
     double aqe = pp / A.aq + pp / B.am; aqe *= aqe;
-    const double rsq = r * r;
     const double s1 = sqrt(rsq + aee), s2 = sqrt((r + da) * (r + da) + ade), s3 = sqrt((r - da) * (r - da) + ade),
                  s4 = sqrt((r + qa) * (r + qa) + aqe), s5 = sqrt((r - qa) * (r - qa) + aqe), a6 = rsq + aqe,
                  s6 = sqrt(a6), s7 = sqrt(a6 + qa * qa);
@@ -215,11 +240,10 @@ __device__ void reppd(int ni, int nj, double rij, double ri[23], double* gab) {
     ri[2] = ev1 / s2 - ev1 / s3;
     ri[3] = ee + ev2 / s4 + ev2 / s5 - ev1 / s6;
     ri[4] = ee + ev1 / s7 - ev1 / s6;
-  } else if (!si && sj) {
+  } else if constexpr (!si && sj) {
     const double db = B.dd, qb = B.qq * td;
     double aed = pp / A.am + pp / B.ad; aed *= aed;
     double aeq = pp / A.am + pp / B.aq; aeq *= aeq;
-    const double rsq = r * r;
     const double s1 = sqrt(rsq + aee), s2 = sqrt((r - db) * (r - db) + aed), s3 = sqrt((r + db) * (r + db) + aed),
                  s4 = sqrt((r - qb) * (r - qb) + aeq), s5 = sqrt((r + qb) * (r + qb) + aeq), a6 = rsq + aeq,
                  s6 = sqrt(a6), s7 = sqrt(a6 + qb * qb);
@@ -239,7 +263,6 @@ __device__ void reppd(int ni, int nj, double rij, double ri[23], double* gab) {
     double adq = pp / A.ad + pp / B.aq; adq *= adq;
     double aqd = pp / A.aq + pp / B.ad; aqd *= aqd;
     double aqq = pp / A.aq + pp / B.aq; aqq *= aqq;
-    const double rsq = r * r;
     double sq[73];
     double xxx, yyy, zzz, www;
 #define SQ(i, v) sq[i] = sqrt(v)
@@ -360,45 +383,51 @@ __device__ void reppd(int ni, int nj, double rij, double ri[23], double* gab) {
   }
   double point, cst;
   to_point(rij, &point, &cst);
+  const double far = __dmul_rn(1.0 - cst, point);
   const unsigned coul = (1u << 1) | (1u << 3) | (1u << 4) | (1u << 11) | (1u << 12) | (1u << 16) | (1u << 17) |
                         (1u << 18) | (1u << 19) | (1u << 21);
   const unsigned neg = (1u << 2) | (1u << 5) | (1u << 8) | (1u << 9) | (1u << 10) | (1u << 13) | (1u << 14) |
                        (1u << 15);
+#pragma unroll
   for (int i = 1; i <= 22; ++i) {
-    ri[i] = ((coul >> i) & 1u) ? ri[i] * cst + (1.0 - cst) * point : ri[i] * cst;
+    ri[i] = ((coul >> i) & 1u) ? __fma_rn(ri[i], cst, far) : __dmul_rn(ri[i], cst);
     if ((neg >> i) & 1u) ri[i] = -ri[i];
   }
-  *gab = *gab * cst + (1.0 - cst) * point;
+  *gab = __fma_rn(*gab, cst, far);
 }
 
 // core[k][n]: electron-core attraction, local frame (spcore) with feathering.
-__device__ void core_terms(int ni, int nj, double rij, double core[5][3]) {
+template <int NI, int NJ>
+__device__ __forceinline__ void core_terms(int ni, int nj, double rij, double core[5][3]) {
   const Pm7Elem& A = c_P.el[ni];
   const Pm7Elem& B = c_P.el[nj];
   const double pxy[8] = {0, 1.0, -0.5, -0.5, 0.5, 0.25, 0.25, 0.5};
-  for (int x = 0; x < 15; ++x) (&core[0][0])[x] = 0.0;
-  const double r = rij / PM7_A0, r2 = r * r;
+#pragma unroll
+  for (int x = 0; x < 5; ++x) core[x][1] = core[x][2] = 0.0;
+  const double r = rij / PM7_A0, r2 = __dmul_rn(r, r);
   const double aci = A.po9, acj = B.po9;
   const double ssi = (aci + B.po1) * (aci + B.po1), ssj = (acj + A.po1) * (acj + A.po1);
   core[1][1] = -B.tore * PM7_EV / sqrt(r2 + ssj);
   core[1][2] = -A.tore * PM7_EV / sqrt(r2 + ssi);
-  if (ni >= 3) {
+  if constexpr (NI == 4) {
     const double ppj = (acj + A.po7) * (acj + A.po7), da = A.ddp2, qa = A.ddp3 / sqrt(2.0), twoqa = qa + qa;
     const double adj = (A.po2 + acj) * (A.po2 + acj), aqj = (A.po3 + acj) * (A.po3 + acj);
     double x[8];
     x[1] = r2 + ppj; x[2] = r2 + aqj; x[3] = (r + da) * (r + da) + adj; x[4] = (r - da) * (r - da) + adj;
     x[5] = (r - twoqa) * (r - twoqa) + aqj; x[6] = (r + twoqa) * (r + twoqa) + aqj; x[7] = r2 + twoqa * twoqa + aqj;
+#pragma unroll
     for (int i = 1; i <= 7; ++i) x[i] = pxy[i] / sqrt(x[i]);
     core[2][1] = -B.tore * ((x[3] + x[4]) * PM7_EV);
     core[3][1] = -B.tore * ((x[1] + x[2] + x[5] + x[6]) * PM7_EV);
     core[4][1] = -B.tore * ((x[1] + x[2] + x[7]) * PM7_EV);
   }
-  if (nj >= 3) {
+  if constexpr (NJ == 4) {
     const double ppi = (aci + B.po7) * (aci + B.po7), db = B.ddp2, qb = B.ddp3 / sqrt(2.0), twoqb = qb + qb;
     const double adi = (B.po2 + aci) * (B.po2 + aci), aqi = (B.po3 + aci) * (B.po3 + aci);
     double x[8];
     x[1] = r2 + ppi; x[2] = r2 + aqi; x[3] = (r + db) * (r + db) + adi; x[4] = (r - db) * (r - db) + adi;
     x[5] = (r - twoqb) * (r - twoqb) + aqi; x[6] = (r + twoqb) * (r + twoqb) + aqi; x[7] = r2 + twoqb * twoqb + aqi;
+#pragma unroll
     for (int i = 1; i <= 7; ++i) x[i] = pxy[i] / sqrt(x[i]);
     core[2][2] = -A.tore * (-(x[3] + x[4]) * PM7_EV);
     core[3][2] = -A.tore * ((x[1] + x[2] + x[5] + x[6]) * PM7_EV);
@@ -443,35 +472,39 @@ __device__ double rotmat(const double* ci, const double* cj, double p[4][4]) {
 __device__ __forceinline__ double ppf(const double p[4][4], int t, int k, int l) {
   const int ta[7] = {0, 1, 2, 3, 1, 1, 2}, tb[7] = {0, 1, 2, 3, 2, 3, 3};
   const int a = ta[t], b = tb[t];
-  if (k == l) return p[k][a] * p[k][b];
-  if (t <= 3) return 2.0 * p[k][a] * p[l][a];
-  return p[k][a] * p[l][b] + p[k][b] * p[l][a];
+  if (k == l) return __dmul_rn(p[k][a], p[k][b]);
+  if (t <= 3) return __dmul_rn(2.0 * p[k][a], p[l][a]);
+  return __fma_rn(p[k][a], p[l][b], __dmul_rn(p[k][b], p[l][a]));
 }
 
 // The electron-core blocks e1b (atom i) / e2a (atom j), packed local order.
-__device__ void elenuc(const double p[4][4], const double core[5][3], int li, int lj, double* e1b, double* e2a) {
+template <int NI, int NJ>
+__device__ __forceinline__ void elenuc(const double p[4][4], const double core[5][3], double* e1b, double* e2a) {
   const int indpp[4][4] = {{0, 0, 0, 0}, {0, 1, 4, 5}, {0, 4, 2, 6}, {0, 5, 6, 3}};
+#pragma unroll
   for (int nn = 1; nn <= 2; ++nn) {
-    const int lim = nn == 1 ? li : lj;
+    const int lim = nn == 1 ? NI : NJ;
     double* out = nn == 1 ? e1b : e2a;
-    int m = 0;
-    for (int i = 1; i <= lim; ++i)
-      for (int j = 1; j <= i; ++j) {
-        const int a = i - 1, b = j - 1;
+#pragma unroll
+    for (int a = 0; a < lim; ++a)
+#pragma unroll
+      for (int b = 0; b <= a; ++b) {
         double h;
         if (a == 0) h = core[1][nn];
         else if (b == 0) h = p[1][a] * core[2][nn];
         else {
           const int t = indpp[a][b];
-          h = core[3][nn] * ppf(p, t, 1, 1) + core[4][nn] * (ppf(p, t, 2, 2) + ppf(p, t, 3, 3));
+          const int u = t == 4 || t == 5 ? 1 : t == 6 ? 2 : t, v = t == 4 ? 2 : t == 5 || t == 6 ? 3 : t;
+          const double q = __fma_rn(p[2][u], p[2][v], __dmul_rn(p[3][u], p[3][v]));
+          h = __fma_rn(core[3][nn], __dmul_rn(p[1][u], p[1][v]), __dmul_rn(core[4][nn], q));
         }
-        out[m++] = 0.0 + h;
+        out[a * (a + 1) / 2 + b] = 0.0 + h;
       }
   }
 }
 
-// ccrep (PM7): r in Bohr on entry
-__device__ double ccrep(int ni, int nj, double rb, double gab) {
+// ccrep (PM7): r in Bohr on entry; z3: the sum of the two atomic numbers' powers 0.3333
+__device__ __forceinline__ double ccrep_z(int ni, int nj, double rb, double gab, double z3) {
   const double r = rb * PM7_A0;
   const Pm7Elem& A = c_P.el[ni];
   const Pm7Elem& B = c_P.el[nj];
@@ -492,7 +525,7 @@ __device__ double ccrep(int ni, int nj, double rb, double gab) {
     } else if (j == 6 && i == 6) {
       scale = scale + c_P.par1 * exp(-c_P.par2 * r);
     }
-    enuclr = enuc * scale;
+    enuclr = __dmul_rn(enuc, scale);
   } else {
     scale = 10.0 * exp(-2.18 * r);
     enuclr = fabs(scale * enuc) + enuc;
@@ -503,7 +536,7 @@ __device__ double ccrep(int ni, int nj, double rb, double gab) {
   ax = B.g2 * (r - B.g3) * (r - B.g3);
   if (ax < 25.0) scale = scale + A.tore * B.tore / r * B.g1 * exp(-ax);
   enuclr = enuclr + scale;
-  ax = r / (pow((double)ni, 0.3333) + pow((double)nj, 0.3333));
+  ax = r / z3;
   if (ax < 3.0) {
     scale = 1.0e-8 / ipow(ax, 12);
     enuclr = enuclr + (scale < 1.0e5 ? scale : 1.0e5);
@@ -511,16 +544,18 @@ __device__ double ccrep(int ni, int nj, double rb, double gab) {
   return enuclr;
 }
 
-// W block of pair (ni first, nj second) in molecular frame, reference layout.
-// Local-frame pairs of each atom are numbered (indexd) 1:ss 2:ps 10:pp(sigma)
-// 3:pi-s 11:pi-sigma 18:pi-pi 4:pi'-s 12:pi'-sigma 19:pi'-pi 25:pi'-pi'.
-__device__ void w_block(int ni, int nj, const double p[4][4], const double ri[23], double* w) {
-  const int ii = c_P.el[ni].natorb, kk = c_P.el[nj].natorb;
-  const int limkl = indx_(kk, kk), limij = indx_(ii, ii);
-  // rep index for (local pair on A, local pair on B): compact local ids 0..9
-  // order (1,1),(2,1),(2,2),(3,1),(3,2),(3,3),(4,1),(4,2),(4,3),(4,4) -> indexd
-  // 1,2,10,3,11,18,4,12,19,25
-  const int repidx[10][10] = {
+__device__ __forceinline__ double ccrep(int ni, int nj, double rb, double gab) {
+  return ccrep_z(ni, nj, rb, gab, pow((double)ni, 0.3333) + pow((double)nj, 0.3333));
+}
+
+// W block of pair (ni first, nj second) in molecular frame, a column at a time:
+// col(kl, w) gets w[ij] of molecular pair kl of the second atom, kl ascending.
+// Pairs of each atom, local or molecular: ss, ps, pp' in packed order.
+template <int NI, int NJ, class Col>
+__device__ __forceinline__ void w_block(const double p[4][4], const double ri[23], Col&& col) {
+  constexpr int LI = NI == 1 ? 1 : 10, LJ = NJ == 1 ? 1 : 10;
+  // rep index for (local pair on A, local pair on B); 0 where it vanishes
+  const int rep[10][10] = {
       // B: ss  ps  pp  pis pisg pipi pi's pi'sg pi'pi pi'pi'
       {1, 5, 11, 0, 0, 12, 0, 0, 0, 12},       // A ss
       {2, 6, 13, 0, 0, 14, 0, 0, 0, 14},       // A sigma-s
@@ -532,59 +567,85 @@ __device__ void w_block(int ni, int nj, const double p[4][4], const double ri[23
       {0, 0, 0, 0, 0, 0, 10, 20, 0, 0},        // A pi'-sigma
       {0, 0, 0, 0, 0, 0, 0, 0, 22, 0},         // A pi'-pi
       {4, 9, 17, 0, 0, 21, 0, 0, 0, 19}};      // A pi'-pi'
-  // local pair (k1, l1) on an atom -> compact id
-  // tx: v(ijA, kl_mol) for the 10 molecular pairs kl of B
-  double v[10][10];
-  for (int x = 0; x < 100; ++x) (&v[0][0])[x] = 0.0;
-  for (int a = 0; a < (ii == 1 ? 1 : 10); ++a) {
-    for (int b = 0; b < (kk == 1 ? 1 : 10); ++b) {
-      const int nd = repidx[a][b];
-      if (nd == 0) continue;
-      const double wrepp = ri[nd];
-      // b -> (k1, l1)
-      int k1 = 1, l1 = 1, e = b;
-      while (e >= k1) { e -= k1; ++k1; }
-      l1 = e + 1;
-      const int mm = (k1 == 1) ? 1 : (l1 == 1 ? 2 : 3);
-      if (mm == 1) v[a][0] = wrepp;
-      else if (mm == 2) {
-        const int k = k1 - 1;
-        v[a][1] = v[a][1] + p[k][1] * wrepp;
-        v[a][3] = v[a][3] + p[k][2] * wrepp;
-        v[a][6] = v[a][6] + p[k][3] * wrepp;
-      } else {
-        const int k = k1 - 1, l = l1 - 1;
-        v[a][2] = v[a][2] + ppf(p, 1, k, l) * wrepp;
-        v[a][5] = v[a][5] + ppf(p, 2, k, l) * wrepp;
-        v[a][9] = v[a][9] + ppf(p, 3, k, l) * wrepp;
-        v[a][4] = v[a][4] + ppf(p, 4, k, l) * wrepp;
-        v[a][7] = v[a][7] + ppf(p, 5, k, l) * wrepp;
-        v[a][8] = v[a][8] + ppf(p, 6, k, l) * wrepp;
+  const int sp[10] = {0, 1, 0, 2, 0, 0, 3, 0, 0, 0};  // pair (p_k, s): k
+  const int pt[10] = {0, 0, 1, 0, 4, 2, 0, 5, 6, 3};  // pair (p, p): ppf's molecular product
+  const int pk[10] = {0, 0, 1, 0, 2, 2, 0, 3, 3, 3}, pl[10] = {0, 0, 1, 0, 1, 2, 0, 1, 2, 3};  // its local axes
+#pragma unroll
+  for (int kl = 0; kl < LJ; ++kl) {
+    double v[LI], w[LI];
+#pragma unroll
+    for (int a = 0; a < LI; ++a) {  // B rotated
+      v[a] = 0.0;
+      if (kl == 0 && rep[a][0]) v[a] = ri[rep[a][0]];
+#pragma unroll
+      for (int b = 1; b < LJ; ++b) {
+        if (!rep[a][b]) continue;
+        if (sp[kl] && sp[b]) v[a] = __fma_rn(p[sp[b]][sp[kl]], ri[rep[a][b]], v[a]);
+        if (pt[kl] && pt[b]) v[a] = __fma_rn(ppf(p, pt[kl], pk[b], pl[b]), ri[rep[a][b]], v[a]);
       }
     }
-  }
-  for (int x = 0; x < limij * limkl; ++x) w[x] = 0.0;
-  for (int a = 0; a < (ii == 1 ? 1 : 10); ++a) {
-    int i1 = 1, j1 = 1, e = a;
-    while (e >= i1) { e -= i1; ++i1; }
-    j1 = e + 1;
-    const int mm = (i1 == 1) ? 1 : (j1 == 1 ? 2 : 3);
-    for (int kl = 1; kl <= limkl; ++kl) {
-      const double wrepp = v[a][kl - 1];
-      if (wrepp == 0.0) continue;
-#define WI(x, y) w[(indx_((x), (y)) - 1) * limkl + kl - 1]
-      if (mm == 1) WI(1, 1) = wrepp;
-      else if (mm == 2) {
-        for (int i = 1; i <= 3; ++i) WI(i + 1, 1) += p[i1 - 1][i] * wrepp;
-      } else {
-        for (int i = 1; i <= 3; ++i) {
-          WI(i + 1, i + 1) += ppf(p, i, i1 - 1, j1 - 1) * wrepp;
-          for (int j = 1; j < i; ++j) WI(i + 1, j + 1) += ppf(p, 1 + i + j, i1 - 1, j1 - 1) * wrepp;
-        }
+    w[0] = v[0];
+#pragma unroll
+    for (int ij = 1; ij < LI; ++ij) {  // A rotated
+      w[ij] = 0.0;
+#pragma unroll
+      for (int a = 1; a < LI; ++a) {
+        if (sp[ij] && sp[a]) w[ij] = __fma_rn(p[sp[a]][sp[ij]], v[a], w[ij]);
+        if (pt[ij] && pt[a]) w[ij] = __fma_rn(ppf(p, pt[ij], pk[a], pl[a]), v[a], w[ij]);
       }
-#undef WI
     }
+    col(kl, w);
   }
+}
+
+// The pair's resonance block through hput(a, b, value), its W block in the
+// reference layout (i's pair index outer, j's inner) to wb, and its core-core
+// energy.
+template <class HPut>
+__device__ __forceinline__ double pair_integrals(int ni, int nj, const double* xi, const double* xj, double* wb,
+                                                 HPut&& hput) {
+  double enuc = 0.0;
+  by_kind(ni, nj, [&](auto oi, auto oj) {
+    constexpr int NI = decltype(oi)::n, NJ = decltype(oj)::n, LI = NI == 1 ? 1 : 10, LJ = NJ == 1 ? 1 : 10;
+    double di[NI][NJ];
+    h1elec<NI, NJ>(ni, nj, xi, xj, di);
+#pragma unroll
+    for (int a = 0; a < NI; ++a)
+#pragma unroll
+      for (int b = 0; b < NJ; ++b) hput(a, b, di[a][b]);
+    const double dx = xi[0] - xj[0], dy = xi[1] - xj[1], dz = xi[2] - xj[2];
+    if (dx * dx + dy * dy + dz * dz < 0.00002) {
+      for (int x = 0; x < LI * LJ; ++x) wb[x] = 0.0;
+      return;
+    }
+    double p[4][4];
+    const double r = rotmat(xi, xj, p);
+    double ri[23], gab;
+    reppd<NI, NJ>(ni, nj, r, ri, &gab);
+    w_block<NI, NJ>(p, ri, [&](int kl, const double* w) {
+#pragma unroll
+      for (int ij = 0; ij < LI; ++ij) wb[ij * LJ + kl] = w[ij];
+    });
+    enuc = ccrep(ni, nj, r / PM7_A0, gab);
+  });
+  return enuc;
+}
+
+// The electron-core blocks of atoms i and j, packed.
+__device__ __forceinline__ void pair_cores(int ni, int nj, const double* xi, const double* xj, double* e1b,
+                                           double* e2a) {
+  double p[4][4], core[5][3];
+  const double r = rotmat(xi, xj, p);
+  by_kind(ni, nj, [&](auto oi, auto oj) {
+    constexpr int NI = decltype(oi)::n, NJ = decltype(oj)::n;
+    core_terms<NI, NJ>(ni, nj, r, core);
+    elenuc<NI, NJ>(p, core, e1b, e2a);
+  });
+}
+
+// reppd for a pair of any kind
+__device__ __forceinline__ void reppd_any(int ni, int nj, double rij, double ri[23], double* gab) {
+  by_kind(ni, nj, [&](auto oi, auto oj) { reppd<decltype(oi)::n, decltype(oj)::n>(ni, nj, rij, ri, gab); });
 }
 
 // Off-diagonal H block, two-centre W block and core-core energy of pair q.
@@ -600,24 +661,10 @@ __device__ void hcore_pair_one(long long q, const int* __restrict__ nat, const d
     const int ni = nat[ia], nj = nat[ja];
     const double* xi = coord + 3 * ia;
     const double* xj = coord + 3 * ja;
-    double di[5][5];
-    h1elec(ni, nj, xi, xj, di);
-    const int fi = at.first[ia], fj = at.first[ja], noi = at.nor[ia], noj = at.nor[ja];
-    for (int a = 1; a <= noi; ++a)
-      for (int b = 1; b <= noj; ++b) h[mb_tri(fi + a - 1, fj + b - 1)] = di[a][b];
+    const int fi = at.first[ia], fj = at.first[ja];
     double* wb = w + at.wrow[ia] + (long long)at.lim[ia] * at.cum[ja];
-    const double dx = xi[0] - xj[0], dy = xi[1] - xj[1], dz = xi[2] - xj[2];
-    if (dx * dx + dy * dy + dz * dz < 0.00002) {
-      for (int x = 0; x < at.lim[ia] * at.lim[ja]; ++x) wb[x] = 0.0;
-      enuc_pairs[q] = 0.0;
-      return;
-    }
-    double p[4][4];
-    const double r = rotmat(xi, xj, p);
-    double ri[23], gab;
-    reppd(ni, nj, r, ri, &gab);
-    w_block(ni, nj, p, ri, wb);
-    enuc_pairs[q] = ccrep(ni, nj, r / PM7_A0, gab);
+    enuc_pairs[q] = pair_integrals(ni, nj, xi, xj, wb,
+                                   [&](int a, int b, double v) { h[mb_tri(fi + a, fj + b)] = v; });
   }
 }
 
@@ -637,16 +684,9 @@ __device__ __forceinline__ bool hcore_partner(int A, int B, const int* __restric
   const double dx = xa[0] - xb[0], dy = xa[1] - xb[1], dz = xa[2] - xb[2];
   if (dx * dx + dy * dy + dz * dz < 0.00002) return false;
   const int nA = nat[A], nB = nat[B];
-  double p[4][4], core[5][3], other[10];
-  if (B < A) {  // pair (A first, B second): A receives e1b
-    const double r = rotmat(xa, xb, p);
-    core_terms(nA, nB, r, core);
-    elenuc(p, core, at.nor[A], at.nor[B], c, other);
-  } else {      // pair (B first, A second): A receives e2a
-    const double r = rotmat(xb, xa, p);
-    core_terms(nB, nA, r, core);
-    elenuc(p, core, at.nor[B], at.nor[A], other, c);
-  }
+  double other[10];
+  if (B < A) pair_cores(nA, nB, xa, xb, c, other);  // pair (A first, B second): A receives e1b
+  else pair_cores(nB, nA, xb, xa, other, c);        // pair (B first, A second): A receives e2a
   return true;
 }
 
@@ -797,26 +837,10 @@ __global__ void mz_hcore_pairs(MbMzLayout L, const int* __restrict__ nat, const 
     const int ni = nat[ia], nj = nat[ja];
     const double* xi = coord + 3 * ia;
     const double* xj = coord + 3 * ja;
-    const int noi = L.iorbs[ia], noj = L.iorbs[ja];
-    double di[5][5];
-    h1elec(ni, nj, xi, xj, di);
+    const int noj = L.iorbs[ja];
     double* hb = h + L.pair_off[e];
-    for (int a = 1; a <= noi; ++a)
-      for (int b = 1; b <= noj; ++b) hb[(a - 1) * noj + (b - 1)] = di[a][b];
-    const int li = noi * (noi + 1) / 2, lj = noj * (noj + 1) / 2;
-    double* wb = w + L.pair_woff[e];
-    const double dx = xi[0] - xj[0], dy = xi[1] - xj[1], dz = xi[2] - xj[2];
-    if (dx * dx + dy * dy + dz * dz < 0.00002) {
-      for (int x = 0; x < li * lj; ++x) wb[x] = 0.0;
-      enuc_entry[e] = 0.0;
-      continue;
-    }
-    double p[4][4];
-    const double r = rotmat(xi, xj, p);
-    double ri[23], gab;
-    reppd(ni, nj, r, ri, &gab);
-    w_block(ni, nj, p, ri, wb);
-    enuc_entry[e] = ccrep(ni, nj, r / PM7_A0, gab);
+    enuc_entry[e] = pair_integrals(ni, nj, xi, xj, w + L.pair_woff[e],
+                                   [&](int a, int b, double v) { hb[a * noj + b] = v; });
   }
 }
 
@@ -848,7 +872,7 @@ __device__ void mz_outer_terms(int ni, int nj, const double* ci, const double* c
   double x[3] = {ci[0] - cj[0], ci[1] - cj[1], ci[2] - cj[2]};
   const double rij = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
   double ri[23], gab;
-  reppd(ni, nj, rij, ri, &gab);
+  reppd_any(ni, nj, rij, ri, &gab);
   const double a = 1.0 / rij;
   x[0] *= a; x[1] *= a; x[2] *= a;
   if (fabs(x[2]) > 0.99999999) x[2] = x[2] >= 0.0 ? 1.0 : -1.0;
@@ -917,7 +941,7 @@ __global__ void __launch_bounds__(128) mz_hcore_diag(MbMzLayout L, const int* __
           cen = enuc_entry[my_entry];
         } else if (r2 < L.cutof1) {       // outer2: monopole term
           double ri[23], gab;
-          reppd(nA, nB, sqrt(r2), ri, &gab);
+          reppd_any(nA, nB, sqrt(r2), ri, &gab);
           cen = c_P.el[nA].tore * c_P.el[nB].tore * ri[1];
         } else {                          // outer1: feathered point charge
           const double rij = sqrt(r2), rb = rij / PM7_A0;
@@ -944,16 +968,11 @@ __global__ void __launch_bounds__(128) mz_hcore_diag(MbMzLayout L, const int* __
             for (int x = 0; x < 10; ++x) if (x < lA) c[x] = e2a[x];
           }
         } else {
-          double p[4][4], core[5][3];
           if (B < A) {
-            const double r = rotmat(xa, xb, p);
-            core_terms(nA, nB, r, core);
-            elenuc(p, core, noA, L.iorbs[B], e1b, e2a);
+            pair_cores(nA, nB, xa, xb, e1b, e2a);
             for (int x = 0; x < 10; ++x) if (x < lA) c[x] = e1b[x];
           } else {
-            const double r = rotmat(xb, xa, p);
-            core_terms(nB, nA, r, core);
-            elenuc(p, core, L.iorbs[B], noA, e1b, e2a);
+            pair_cores(nB, nA, xb, xa, e1b, e2a);
             for (int x = 0; x < 10; ++x) if (x < lA) c[x] = e2a[x];
           }
         }
@@ -1012,109 +1031,215 @@ __device__ __forceinline__ int pairix(int a, int b) {  // 0-based pair index of 
 // Coulomb and exchange terms with the density fixed, helect over the pair's
 // orbitals (doubled), and ccrep's core-core term; eV.  Like dhc it leaves out
 // every term that does not depend on the pair's geometry.
-__device__ double dhc_energy(int n1, int n2, const double* x1, const double* x2, const PairDens& d) {
-  const int nor1 = c_P.el[n1].natorb, nor2 = c_P.el[n2].natorb;
-  const int lim1 = nor1 * (nor1 + 1) / 2, lim2 = nor2 * (nor2 + 1) / 2;
-  double di[5][5];
-  h1elec(n1, n2, x1, x2, di);  // di[a][b]: a on atom 1, b on atom 2
-  double h1[10], h2[10], wb[100], enuc = 0.0;
-  for (int x = 0; x < 10; ++x) { h1[x] = 0.0; h2[x] = 0.0; }
-  for (int x = 0; x < 100; ++x) wb[x] = 0.0;
+//
+// N1, N2: the atoms' orbital counts.  sw: room for the W block, element
+// (ij, kl) at sw[(ij * lim1 + kl) * SW]; z3 as in ccrep_z.
+template <int N1, int N2, int SW>
+__device__ __forceinline__ double dhc_energy(int n1, int n2, const double* x1, const double* x2, const PairDens& d,
+                                             double* sw, double z3) {
+  constexpr int L1 = N1 == 1 ? 1 : 10, L2 = N2 == 1 ? 1 : 10;
+  double enuc = 0.0, e = 0.0;
+  double h1[10], h2[10], ri[23], p[4][4];
   const double dx = x2[0] - x1[0], dy = x2[1] - x1[1], dz = x2[2] - x1[2];
-  if (dx * dx + dy * dy + dz * dz >= 0.00002) {
-    double p[4][4];
+  const bool apart = dx * dx + dy * dy + dz * dz >= 0.00002;
+#pragma unroll
+  for (int x = 0; x < 10; ++x) h1[x] = h2[x] = 0.0;
+  if (apart) {
     const double r = rotmat(x2, x1, p);  // rotate(ni = atom 2, nj = atom 1) as dhc calls it
-    double ri[23], gab;
-    reppd(n2, n1, r, ri, &gab);
-    w_block(n2, n1, p, ri, wb);  // lim2 x lim1, atom 1's pair index fastest
-    double core[5][3];
-    core_terms(n2, n1, r, core);
-    elenuc(p, core, nor2, nor1, h2, h1);  // atom 2's electrons: e1b; atom 1's: e2a
-    enuc = ccrep(n2, n1, r / PM7_A0, gab);
+    double core[5][3], gab;
+    core_terms<N2, N1>(n2, n1, r, core);
+    elenuc<N2, N1>(p, core, h2, h1);  // atom 2's electrons: e1b; atom 1's: e2a
+    reppd<N2, N1>(n2, n1, r, ri, &gab);
+    enuc = ccrep_z(n2, n1, r / PM7_A0, gab, z3);
+  } else {
+#pragma unroll
+    for (int x = 0; x < 23; ++x) ri[x] = 0.0;
+#pragma unroll
+    for (int x = 0; x < 16; ++x) (&p[0][0])[x] = 0.0;
   }
   // Coulomb terms on each atom's block from the other atom's density, and the
   // energy of the diagonal blocks: sum' P (H + F), F = H + G
-  double e = 0.0;
-  for (int a = 0; a < nor1; ++a)
+  w_block<N2, N1>(p, ri, [&](int q, const double* w) {  // atom 1's pair q
+#pragma unroll
+    for (int ij = 0; ij < L2; ++ij) sw[(ij * L1 + q) * SW] = w[ij];
+    double g = 0.0;
+#pragma unroll
+    for (int x = 0; x < N2; ++x)
+#pragma unroll
+      for (int y = 0; y < N2; ++y) g += d.p2[x][y] * w[pairix(x, y)];
+#pragma unroll
+    for (int a = 0; a < N1; ++a)
+#pragma unroll
+      for (int b = 0; b <= a; ++b)
+        if (pairix(a, b) == q) {
+          const double wgt = a == b ? 0.5 : 1.0;
+          e += wgt * d.p1[a][b] * (2.0 * h1[q] + g);
+        }
+  });
+#pragma unroll
+  for (int a = 0; a < N2; ++a)
+#pragma unroll
     for (int b = 0; b <= a; ++b) {
       const int q = pairix(a, b);
       double g = 0.0;
-      for (int x = 0; x < nor2; ++x)
-        for (int y = 0; y < nor2; ++y) g += d.p2[x][y] * wb[pairix(x, y) * lim1 + q];
-      const double wgt = a == b ? 0.5 : 1.0;
-      e += wgt * d.p1[a][b] * (2.0 * h1[q] + g);
-    }
-  for (int a = 0; a < nor2; ++a)
-    for (int b = 0; b <= a; ++b) {
-      const int q = pairix(a, b);
-      double g = 0.0;
-      for (int x = 0; x < nor1; ++x)
-        for (int y = 0; y < nor1; ++y) g += d.p1[x][y] * wb[q * lim1 + pairix(x, y)];
+#pragma unroll
+      for (int x = 0; x < N1; ++x)
+#pragma unroll
+        for (int y = 0; y < N1; ++y) g += d.p1[x][y] * sw[(q * L1 + pairix(x, y)) * SW];
       const double wgt = a == b ? 0.5 : 1.0;
       e += wgt * d.p2[a][b] * (2.0 * h2[q] + g);
     }
   // the off-diagonal block: resonance and exchange (kab), PA = P / 2
-  for (int mu = 0; mu < nor2; ++mu)
-    for (int nu = 0; nu < nor1; ++nu) {
+  double di[N1][N2];
+  h1elec<N1, N2>(n1, n2, x1, x2, di);  // di[a][b]: a on atom 1, b on atom 2
+#pragma unroll
+  for (int mu = 0; mu < N2; ++mu)
+#pragma unroll
+    for (int nu = 0; nu < N1; ++nu) {
       double k = 0.0;
-      for (int la = 0; la < nor2; ++la)
-        for (int si = 0; si < nor1; ++si) k += 0.5 * d.p21[la][si] * wb[pairix(mu, la) * lim1 + pairix(nu, si)];
-      e += d.p21[mu][nu] * (2.0 * di[nu + 1][mu + 1] - k);
+#pragma unroll
+      for (int la = 0; la < N2; ++la)
+#pragma unroll
+        for (int si = 0; si < N1; ++si)
+          k += 0.5 * d.p21[la][si] * sw[(pairix(mu, la) * L1 + pairix(nu, si)) * SW];
+      e += d.p21[mu][nu] * (2.0 * di[nu][mu] - k);
     }
-  (void)lim2;
   // 2 * helect(PA, H, F) with PA = P/2 is sum' P (H + F) = e
   return e + enuc;
+}
+
+// The k-th (from 0) atom of numat that has four orbitals (heavy) or one: with
+// one or four orbitals an atom, first[a] - a is three times the heavy atoms below a.
+__device__ __forceinline__ int kth_atom(const int* __restrict__ first, int numat, int k, bool heavy) {
+  int lo = 0, hi = numat - 1;  // the largest a with at most k of the kind below it
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1, nh = (first[mid] - mid) / 3;
+    if ((heavy ? nh : mid - nh) <= k) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// q -> (i, j), i > j, q = i (i - 1) / 2 + j
+__device__ __forceinline__ void pair_of(long long q, int* ii, int* jj) {
+  long long i = (long long)((sqrt(8.0 * (double)q + 1.0) + 1.0) * 0.5);
+  while (i * (i - 1) / 2 > q) --i;
+  while ((i + 1) * i / 2 <= q) ++i;
+  *ii = (int)i;
+  *jj = (int)(q - i * (i - 1) / 2);
 }
 
 // dcart (forces/dcart.F90:60-300) for a molecule with the default finite
 // difference (no FORCE keyword): pair q = (ii, jj), jj < ii, with atom jj
 // moved by chnge/2 along all three axes, then atom ii by chnge along each
 // axis in turn; deriv = (E0 - Ek) * fpc_9 / chnge, kcal/mol/A.
-__global__ void dcart_pairs(int numat, const int* __restrict__ nat, const double* __restrict__ coord, MbAtomsDev at,
-                            const double* __restrict__ ptot, double* __restrict__ deriv) {
-  const long long npair = (long long)numat * (numat - 1) / 2;
+//
+// A lane per (pair, geometry), four lanes a pair, and a launch per kind of pair:
+// two heavy atoms (KIND 0), mixed (1; the light partners of a heavy atom in a
+// row), two light ones (2), so that the loops have constant lengths and the lanes
+// of a warp take the same branches.  The W block of two heavy atoms (100
+// numbers) is in shared memory, everything else in registers.  Bound by the FP64
+// pipe's latency, a few hundred square roots and quotients an energy, at 8 to 12
+// warps an SM.  (H2O)200, one B200: 0.25 ms; a thread per pair, with the kinds mixed
+// in a warp and the arrays in local memory, took 3.4, that split by kind and
+// geometry alone 1.0.
+template <int KIND>
+__global__ void __launch_bounds__(KIND == 0 ? 32 : 128) dcart_pairs(int numat, const int* __restrict__ nat,
+                                                                    const double* __restrict__ coord, MbAtomsDev at,
+                                                                    const double* __restrict__ ptot,
+                                                                    double* __restrict__ deriv) {
+  __shared__ double z3[9], sw[KIND == 0 ? 100 * 32 : 1];
+  if (threadIdx.x < 9) z3[threadIdx.x] = pow((double)threadIdx.x, 0.3333);
+  __syncthreads();
   const double chnge = 1.0e-4, chnge2 = chnge * 0.5;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < npair;
-       q += (long long)gridDim.x * blockDim.x) {
-    long long i = (long long)((sqrt(8.0 * (double)q + 1.0) + 1.0) * 0.5);
-    while (i * (i - 1) / 2 > q) --i;
-    while ((i + 1) * i / 2 <= q) ++i;
-    const int ii = (int)i, jj = (int)(q - i * (i - 1) / 2);
-    const int f1 = at.first[jj], f2 = at.first[ii], no1 = at.nor[jj], no2 = at.nor[ii];
-    PairDens d;
-    for (int a = 0; a < 4; ++a)
-      for (int b = 0; b < 4; ++b) {
-        d.p1[a][b] = (a < no1 && b < no1) ? ptot[mb_tri(f1 + (a > b ? a : b), f1 + (a > b ? b : a))] : 0.0;
-        d.p2[a][b] = (a < no2 && b < no2) ? ptot[mb_tri(f2 + (a > b ? a : b), f2 + (a > b ? b : a))] : 0.0;
-        d.p21[a][b] = (a < no2 && b < no1) ? ptot[mb_tri(f2 + a, f1 + b)] : 0.0;
-      }
-    double x1[3], x2[3];
-    for (int k = 0; k < 3; ++k) {
-      x1[k] = coord[3 * jj + k] + chnge2;
-      x2[k] = coord[3 * ii + k];
+  const long long nh = (at.first[numat - 1] + at.nor[numat - 1] - numat) / 3, nl = numat - nh;
+  const long long count = KIND == 0 ? nh * (nh - 1) / 2 : KIND == 1 ? nh * nl : nl * (nl - 1) / 2;
+  const int geo = threadIdx.x & 3;
+  // whole warps iterate, for the shuffle: lanes past the end repeat the last pair
+  for (long long t0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x - (threadIdx.x & 31)) >> 2; t0 < count;
+       t0 += (long long)gridDim.x * blockDim.x >> 2) {
+    long long t = t0 + ((threadIdx.x & 31) >> 2);
+    const bool live = t < count;
+    if (!live) t = count - 1;
+    int ii, jj;
+    if (KIND == 1) {
+      const int a = kth_atom(at.first, numat, (int)(t / nl), true), b = kth_atom(at.first, numat, (int)(t % nl), false);
+      ii = a > b ? a : b;
+      jj = a > b ? b : a;
+    } else {
+      pair_of(t, &ii, &jj);
+      ii = kth_atom(at.first, numat, ii, KIND == 0);
+      jj = kth_atom(at.first, numat, jj, KIND == 0);
     }
     const int n1 = nat[jj], n2 = nat[ii];
-    const double aa = dhc_energy(n1, n2, x1, x2, d);
+    const double zz = z3[n2] + z3[n1];
+    double x1[3], x2[3];
+#pragma unroll
     for (int k = 0; k < 3; ++k) {
-      x2[k] = x2[k] + chnge;
-      const double ee = dhc_energy(n1, n2, x1, x2, d);
-      x2[k] = x2[k] - chnge2;
-      x2[k] = x2[k] - chnge2;
-      deriv[3 * q + k] = (aa - ee) * PM7_FPC9 / chnge;
+      x1[k] = coord[3 * jj + k] + chnge2;
+      // dcart moves ii forth and back on one axis after another, in place
+      const double x = coord[3 * ii + k];
+      x2[k] = k + 1 > geo ? x : k + 1 == geo ? x + chnge : x + chnge - chnge2 - chnge2;
     }
+    auto energy = [&](auto o1, auto o2) {
+      constexpr int N1 = decltype(o1)::n, N2 = decltype(o2)::n;
+      const int f1 = at.first[jj], f2 = at.first[ii];
+      PairDens d;
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          d.p1[a][b] = (a < N1 && b < N1) ? ptot[mb_tri(f1 + (a > b ? a : b), f1 + (a > b ? b : a))] : 0.0;
+          d.p2[a][b] = (a < N2 && b < N2) ? ptot[mb_tri(f2 + (a > b ? a : b), f2 + (a > b ? b : a))] : 0.0;
+          d.p21[a][b] = (a < N2 && b < N1) ? ptot[mb_tri(f2 + a, f1 + b)] : 0.0;
+        }
+      if constexpr (KIND == 0) {
+        return dhc_energy<N1, N2, 32>(n1, n2, x1, x2, d, sw + threadIdx.x, zz);
+      } else {
+        double w[10];
+        return dhc_energy<N1, N2, 1>(n1, n2, x1, x2, d, w, zz);
+      }
+    };
+    double e;
+    if constexpr (KIND == 0) e = energy(Orb<4>{}, Orb<4>{});
+    else if constexpr (KIND == 2) e = energy(Orb<1>{}, Orb<1>{});
+    else if (at.nor[ii] == 1) e = energy(Orb<4>{}, Orb<1>{});
+    else e = energy(Orb<1>{}, Orb<4>{});
+    const double aa = __shfl_sync(0xffffffffu, e, threadIdx.x & 28);
+    if (live && geo > 0) deriv[3 * ((long long)ii * (ii - 1) / 2 + jj) + geo - 1] = (aa - e) * PM7_FPC9 / chnge;
   }
 }
 
 // dxyz of atom a in dcart's accumulation order: the pairs (a, jj < a), then
-// the pairs (ii > a, a), each ascending.
-__global__ void dcart_sum(int numat, const double* __restrict__ deriv, double* __restrict__ dxyz) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * numat) return;
-  const int a = t / 3, k = t - 3 * a;
-  double g = 0.0;
-  for (int b = 0; b < a; ++b) g = g - deriv[3 * ((long long)a * (a - 1) / 2 + b) + k];
-  for (int b = a + 1; b < numat; ++b) g = g + deriv[3 * ((long long)b * (b - 1) / 2 + a) + k];
-  dxyz[t] = g;
+// the pairs (ii > a, a), each ascending.  A warp per atom loads the terms of 32
+// partners at a time and its first three lanes add them in order, a coordinate
+// each; bound by the chain of additions.  600 atoms: 16 us; a thread per
+// coordinate, straight from global memory, 98.
+__global__ void __launch_bounds__(128) dcart_sum(int numat, const double* __restrict__ deriv,
+                                                 double* __restrict__ dxyz) {
+  __shared__ double term[4][96];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, a = blockIdx.x * 4 + warp;
+  if (a >= numat) return;  // warp-uniform
+  double next[3], g = 0.0;
+  auto load = [&](int b) {
+    const long long q = b < a ? (long long)a * (a - 1) / 2 + b : (long long)b * (b - 1) / 2 + a;
+    for (int k = 0; k < 3; ++k) next[k] = (b < numat && b != a) ? deriv[3 * q + k] : 0.0;
+  };
+  load(lane);
+  for (int b0 = 0; b0 < numat; b0 += 32) {
+    for (int k = 0; k < 3; ++k) term[warp][3 * lane + k] = next[k];
+    __syncwarp();
+    load(b0 + 32 + lane);
+    if (lane < 3) {
+      const int nb = numat - b0 < 32 ? numat - b0 : 32;
+#pragma unroll 8
+      for (int x = 0; x < nb; ++x) {
+        const double v = term[warp][3 * x + lane];
+        if (b0 + x != a) g = b0 + x < a ? g - v : g + v;
+      }
+    }
+    __syncwarp();
+  }
+  if (lane < 3) dxyz[3 * a + lane] = g;
 }
 
 bool g_params_uploaded = false;
@@ -1226,11 +1351,16 @@ extern "C" int mb_dcart_dev(const int* nat_d, const double* coord_d, const MbAto
   MB_TRY(upload_params());
   const long long npair = (long long)numat * (numat - 1) / 2;
   if (npair > 0) {
-    int blocks = (int)((npair + 127) / 128);
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    dcart_pairs<<<blocks, 128, 0, stream>>>(numat, nat_d, coord_d, *at, p, (double*)ws);
+    // how many pairs are of which kind is known on the device only
+    const int b32 = (int)std::min<long long>((npair + 7) / 8, 148 * 16);
+    const int b128 = (int)std::min<long long>((npair + 31) / 32, 148 * 8);
+    dcart_pairs<0><<<b32, 32, 0, stream>>>(numat, nat_d, coord_d, *at, p, (double*)ws);
     MB_LAUNCH_CHECK();
-    dcart_sum<<<(3 * numat + 127) / 128, 128, 0, stream>>>(numat, (const double*)ws, dxyz_dev);
+    dcart_pairs<1><<<b128, 128, 0, stream>>>(numat, nat_d, coord_d, *at, p, (double*)ws);
+    MB_LAUNCH_CHECK();
+    dcart_pairs<2><<<b128, 128, 0, stream>>>(numat, nat_d, coord_d, *at, p, (double*)ws);
+    MB_LAUNCH_CHECK();
+    dcart_sum<<<(numat + 3) / 4, 128, 0, stream>>>(numat, (const double*)ws, dxyz_dev);
     MB_LAUNCH_CHECK();
   } else {
     MB_CUDA(cudaMemsetAsync(dxyz_dev, 0, sizeof(double) * 3 * (size_t)numat, stream));
