@@ -12,32 +12,35 @@
 //
 // Design: two passes over a staging array.
 //
-// Pass 1 (fock2_pairs) evaluates every ordered atom pair (A, B), B != A, one
-// pair per lane: B's Coulomb contribution to A's diagonal block goes to the
-// staging array, and for B < A the exchange block F(A, B) goes straight to F.
-// Work is a queue of warp items, taken with an atomic counter:
-//   HH  heavy A, 32 heavy partners: the 10 x 10 W blocks stream through the
-//       warp as 16 row tiles, in the order of jab's density gather (row
-//       pair(x, y) at step 4x + y).  That order is also kab's (mu, lam)
-//       order, so the exchange sums and both Coulomb sums keep the
-//       reference's term sequence with one W row live per lane.
-//   X   every pair with a light atom: 128 partners, four tiles of one block
-//       (at most ten doubles) per lane.
-// A tile (32 lanes x up to 10 doubles) is copied with cp.async by the whole
+// Pass 1 (fock2_pairs) evaluates every atom pair once, one pair per lane: its
+// exchange block goes straight to F, and the Coulomb contributions that need a
+// sum over a heavy atom's density go to the staging array.  Work is a queue of
+// warp items, taken with an atomic counter:
+//   HH  heavy A, 32 heavy partners below it: the 10 x 10 W blocks stream
+//       through the warp as ten row tiles, used in the order of jab's density gather
+//       (row pair(x, y) at step 4x + y).  That order is also kab's (mu, lam)
+//       order and that of the terms of the partner's elements, so the exchange
+//       sums and both atoms' Coulomb sums keep the reference's term sequence
+//       with one W row live per lane.
+//   HX  heavy A, 128 light partners, four tiles of one ten-double block per lane.
+//   LL  light A, the light partners below it: exchange only.
+// A tile (32 lanes x ten doubles) is copied with cp.async by the whole
 // warp over the concatenated blocks -- consecutive lanes copy consecutive
 // addresses -- into per-lane slots of 11 doubles (odd, so the lanes' reads
-// hit distinct banks); each warp keeps four tiles in flight.
+// hit distinct banks), all of an item's tiles at once.
 //
-// Pass 2 (fock2_fold) runs one CTA per atom: it streams the atom's staged
-// contributions through shared memory in partner order, and up to ten owner
-// threads fold them into iter's start value, adding fock1's one-centre term
-// at the atom's own position.  A light atom's two staged values per partner
-// are fock2's one or two additions; an absent second addition is staged as
-// -0.0, which leaves every sum unchanged bit for bit.
+// Pass 2 (fock2_fold) runs one CTA per atom: it streams the contributions of
+// the atom's partners through shared memory in partner order, and up to ten
+// owner threads fold them into iter's start value, adding fock1's one-centre
+// term at the atom's own position.  A light partner's contribution is its
+// density times its W block, which is read in place of a staged record of the
+// same size.  A light atom's two values per partner are fock2's one or two
+// additions; an absent second addition is -0.0, which leaves every sum unchanged
+// bit for bit.
 //
-// Traffic: W once per ordered pair (the second read of a block mostly from
-// L2), the staged contributions written and read once, one pass over P, PA,
-// H and F.
+// Bound by sectors through L1: blocks, density and F in runs of 8 to 80 bytes.
+// (H2O)333, one B200: 65 us for the pairs and 30 for the fold; with every ordered
+// pair evaluated and staged, 122 and 19, and 5 for the lists in one CTA.
 #include <cstdint>
 #include <mutex>
 
@@ -45,14 +48,14 @@
 
 namespace {
 
-constexpr int kWarps = 4;          // warps per CTA of the pair pass
-constexpr int kDepth = 4;          // tiles in flight per warp
-static_assert(kDepth >= 4 && kDepth <= 4, "an HX item stages its four tiles at once, and cp_async_wait takes n <= 3");
+constexpr int kWarps = 2;          // warps per CTA of the pair pass, four CTAs an SM
+constexpr int kRows = 10;          // tiles per warp: the rows of a W block
 constexpr int kSlot = 11;          // doubles per lane slot in a tile
 constexpr int kTile = 32 * kSlot;  // doubles per tile
-constexpr int kStageW = 10;        // staged doubles per (A, B) record of a heavy A (a light A uses 2)
-constexpr int kFoldThreads = 128;  // pass 2: threads per CTA and partners per chunk
-constexpr int kFoldDepth = 3;      // pass 2: chunks in flight
+constexpr int kStageW = 10;        // staged doubles per (A, heavy B) record of a heavy A (a light A uses 2)
+constexpr int kFoldThreads = 128;  // pass 2: threads per CTA; one warp folds, the others fetch
+constexpr int kChunk = kFoldThreads - 32;  // pass 2: partners per chunk, one a fetching thread
+constexpr int kFoldDepth = 3;      // pass 2: chunk buffers: one folded, two on their way
 
 __host__ __device__ constexpr int pair1(int a, int b) {  // 1-based pair index of orbitals a, b (1..4)
   return a > b ? a * (a - 1) / 2 + b : b * (b - 1) / 2 + a;
@@ -60,6 +63,12 @@ __host__ __device__ constexpr int pair1(int a, int b) {  // 1-based pair index o
 
 // jab's density gather: term m uses pair index pair1(m / 4 + 1, m % 4 + 1).
 __host__ __device__ constexpr int pidx(int m) { return pair1(m / 4 + 1, m % 4 + 1); }
+// How many rows the gather visits first before term m (m / 4 <= m % 4).
+__host__ __device__ constexpr int first_visit(int m) {
+  int n = 0;
+  for (int k = 0; k < m; ++k) n += k / 4 <= k % 4;
+  return n;
+}
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -68,13 +77,24 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
-// Wait until at most n of this thread's committed groups are pending (n <= 3).
+// Wait until at most N of this thread's committed groups are pending.
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+// The same for an n known after unrolling, n < kRows.
 __device__ __forceinline__ void cp_async_wait(int n) {
   switch (n) {
-    case 0: asm volatile("cp.async.wait_group 0;\n" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;\n" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;\n" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 3;\n" ::: "memory"); break;
+    case 0: cp_async_wait<0>(); break;
+    case 1: cp_async_wait<1>(); break;
+    case 2: cp_async_wait<2>(); break;
+    case 3: cp_async_wait<3>(); break;
+    case 4: cp_async_wait<4>(); break;
+    case 5: cp_async_wait<5>(); break;
+    case 6: cp_async_wait<6>(); break;
+    case 7: cp_async_wait<7>(); break;
+    case 8: cp_async_wait<8>(); break;
+    default: cp_async_wait<9>(); break;
   }
 }
 
@@ -113,11 +133,14 @@ FockWs carve(void* ws, int numat) {
   return r;
 }
 
-// Staged record of partner B for atom A: a heavy A's ten values at
-// (A*numat + B)*10, a light A's two at A*numat*10 + 2B.
-__device__ __forceinline__ long long rec_off(int A, int numat, int B, bool heavy) {
-  return (long long)A * numat * kStageW + (long long)B * (heavy ? kStageW : 2);
+// Staged record of the rank-th heavy atom for atom A: a heavy A's ten values or a
+// light A's two.
+__device__ __forceinline__ long long rec_off(int A, int numat, int rank, bool heavy) {
+  return (long long)A * numat * kStageW + (long long)rank * (heavy ? kStageW : 2);
 }
+
+// Heavy atoms below atom A (one or four orbitals an atom).
+__device__ __forceinline__ int heavy_below(const MbAtoms& at, int A) { return (__ldg(at.first + A) - A) / 3; }
 
 __device__ __forceinline__ double f_start(const FockArgs& a, long long idx, bool diag) {
   if (!a.use_shift) return __ldg(a.h + idx);
@@ -144,23 +167,6 @@ __device__ __forceinline__ void diag_block(const FockArgs& a, int fB, double* pj
     }
 }
 
-// A light atom's two additions from heavy B's diagonal block (fock2's
-// "ib - ia >= 3" / "jb - ja >= 3" branches with one s orbital on the light
-// atom): c[0] = 2 * off-diagonal sum, c[1] = diagonal sum.
-__device__ __forceinline__ void light_from_heavy(const FockArgs& a, int fB, const double* wk, double* c) {
-  double sumoff = 0.0, sumdia = 0.0;
-  int k = 0;
-#pragma unroll
-  for (int i = 0; i <= 3; ++i) {
-#pragma unroll
-    for (int j = 1; j <= i; ++j) sumoff = DADD(sumoff, DMUL(__ldg(a.ptot + mb_tri(fB + i, fB + j - 1)), __ldg(wk + j + k - 1)));
-    k += i + 1;
-    sumdia = DADD(sumdia, DMUL(__ldg(a.ptot + mb_tri(fB + i, fB + i)), __ldg(wk + k - 1)));
-  }
-  c[0] = DMUL(sumoff, 2.0);
-  c[1] = sumdia;
-}
-
 // Warp-cooperative tile copy: 32 windows of ten doubles, window i at
 // src[i] + add, land in slots 0..31.  Flat element q = 32r + lane of round r
 // is element q % 10 of window q / 10, so consecutive lanes copy consecutive
@@ -182,97 +188,39 @@ __device__ __forceinline__ const double* w_block(const FockArgs& a, int A, int l
                : a.w + __ldg(a.at.wrow + B) + (long long)lB * __ldg(a.at.cum + A);
 }
 
-// One pair with at least one light atom, W block read from global memory.
-__device__ __forceinline__ void pair_x(const FockArgs& a, int A, int fA, int nA, int B, const double* wk,
-                                       double* out) {
-  const int fB = __ldg(a.at.first + B), nB = __ldg(a.at.nor + B);
-  if (nA == 4) {  // heavy A, light B: ten Coulomb terms
-    const double pb = __ldg(a.ptot + (mb_tri(fB, fB)));
-#pragma unroll
-    for (int q = 0; q < 10; ++q) out[q] = DMUL(pb, __ldg(wk + q));
-    if (B < A) {  // kab on the 4 x 1 block
-      double pj[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) pj[j] = __ldg(a.pa + (mb_tri(fA + j, fB)));
-#pragma unroll
-      for (int i = 1; i <= 4; ++i) {
-        double sum = 0.0;
-#pragma unroll
-        for (int j = 1; j <= 4; ++j) sum = DADD(sum, DMUL(pj[j - 1], __ldg(wk + pair1(i, j) - 1)));
-        const long long idx = mb_tri(fA + i - 1, fB);
-        a.f[idx] = DSUB(f_start(a, idx, false), sum);
-      }
-    }
-  } else if (nB == 4) {  // light A, heavy B: two additions
-    light_from_heavy(a, fB, wk, out);
-    if (B < A) {  // kab on the 1 x 4 block
-      double pl[4];
-#pragma unroll
-      for (int l = 0; l < 4; ++l) pl[l] = __ldg(a.pa + (mb_tri(fA, fB + l)));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        double sum = 0.0;
-#pragma unroll
-        for (int l = 1; l <= 4; ++l) sum = DADD(sum, DMUL(pl[l - 1], __ldg(wk + pair1(i + 1, l) - 1)));
-        const long long idx = mb_tri(fA, fB + i);
-        a.f[idx] = DSUB(f_start(a, idx, false), sum);
-      }
-    }
-  } else {  // two light atoms: one addition
-    out[0] = DMUL(__ldg(a.ptot + (mb_tri(fB, fB))), __ldg(wk));
-    out[1] = -0.0;
-    if (B < A) {
-      const long long idx = mb_tri(fA, fB);
-      a.f[idx] = DSUB(f_start(a, idx, false), DMUL(__ldg(a.pa + idx), __ldg(wk)));
-    }
-  }
-}
+// The light atoms' densities, in their order: atom 0's staged records leave the
+// room behind the heavy atoms' ten free.
+__device__ __forceinline__ double* light_density(const FockWs& ws, int nh) { return ws.stage + (long long)nh * kStageW; }
 
-// Heavy and light atom lists (ascending), their lengths, and a zero item
-// counter for the pair pass.  One CTA.
-__global__ void fock2_lists(MbAtoms at, FockWs ws) {
-  __shared__ int s_warp[32], s_base[2];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  if (tid == 0) { s_base[0] = 0; s_base[1] = 0; }
-  __syncthreads();
-  for (int b0 = 0; b0 < at.numat; b0 += blockDim.x) {
-    const int A = b0 + tid;
-    const bool valid = A < at.numat;
-    const bool heavy = valid && at.nor[A] == 4;
-    const unsigned hb = __ballot_sync(0xffffffffu, heavy), vb = __ballot_sync(0xffffffffu, valid);
-    const unsigned below = (1u << lane) - 1u;
-    const int hpre = __popc(hb & below), vpre = __popc(vb & below);
-    if (lane == 0) s_warp[warp] = (__popc(hb) << 16) | __popc(vb);
-    __syncthreads();
-    int hoff = 0, voff = 0;
-    for (int w = 0; w < warp; ++w) { hoff += s_warp[w] >> 16; voff += s_warp[w] & 0xffff; }
-    if (heavy) ws.hlist[s_base[0] + hoff + hpre] = A;
-    else if (valid) ws.llist[s_base[1] + (voff + vpre) - (hoff + hpre)] = A;
-    __syncthreads();
-    if (tid == 0) {
-      int ht = 0, vt = 0;
-      for (int w = 0; w < nw; ++w) { ht += s_warp[w] >> 16; vt += s_warp[w] & 0xffff; }
-      s_base[0] += ht;
-      s_base[1] += vt - ht;
-    }
-    __syncthreads();
+// Heavy and light atom lists (ascending), their lengths, the light atoms'
+// densities, and a zero item counter for the pair pass.
+__global__ void fock2_lists(MbAtoms at, const double* __restrict__ ptot, FockWs ws) {
+  const int A = blockIdx.x * blockDim.x + threadIdx.x;
+  if (A >= at.numat) return;
+  const int nh = heavy_below(at, A);
+  const bool heavy = at.nor[A] == 4;
+  if (heavy) ws.hlist[nh] = A;
+  else ws.llist[A - nh] = A;
+  if (!heavy) {
+    const int last = at.numat - 1, all = heavy_below(at, last) + (at.nor[last] == 4), f = __ldg(at.first + A);
+    light_density(ws, all)[A - nh] = __ldg(ptot + mb_tri(f, f));
   }
-  if (tid == 0) {
-    ws.counts[0] = s_base[0];
-    ws.counts[1] = s_base[1];
+  if (A == at.numat - 1) {
+    ws.counts[0] = nh + heavy;
+    ws.counts[1] = at.numat - nh - heavy;
     ws.counts[2] = 0;
   }
 }
 
-__global__ void __launch_bounds__(32 * kWarps, 3) fock2_pairs(FockArgs a, FockWs ws) {
-  extern __shared__ double s_tiles[];  // kWarps x kDepth tiles
-  __shared__ unsigned long long s_src[kWarps][4][32];
+__global__ void __launch_bounds__(32 * kWarps, 4) fock2_pairs(FockArgs a, FockWs ws) {
+  extern __shared__ double s_tiles[];  // kWarps x kRows tiles
+  __shared__ unsigned long long s_src[kWarps][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double* tiles = s_tiles + (size_t)warp * kDepth * kTile;
+  double* tiles = s_tiles + (size_t)warp * kRows * kTile;
   const int numat = a.at.numat;
   const int nh = ws.counts[0], nl = ws.counts[1];
-  const int th = (nh + 31) / 32, tl = (nl + 127) / 128, ta = (numat + 127) / 128;
-  const long long r1 = (long long)nh * th, r2 = r1 + (long long)nh * tl, total = r2 + (long long)nl * ta;
+  const int th = (nh + 31) / 32, tl = (nl + 127) / 128;
+  const long long r1 = (long long)th * (th + 1) / 2 * 32, r2 = r1 + (long long)nh * tl, total = r2 + nl;
 
   for (;;) {
     long long item = 0;
@@ -280,174 +228,197 @@ __global__ void __launch_bounds__(32 * kWarps, 3) fock2_pairs(FockArgs a, FockWs
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= total) break;
 
+    // HH items and the others in turn, so that loading and computing warps share an
+    // SM: (H2O)333 78 -> 67 us
+    const long long both = 2 * min(r1, total - r1);
+    if (item < both) item = (item & 1) ? r1 + (item >> 1) : item >> 1;
+    else if (2 * r1 > both) item = item - (both >> 1);
     if (item < r1) {
-      // HH: heavy A, heavy partners hlist[32 t + lane]; W rows through the tile ring
-      const int A = __ldg(ws.hlist + (item / th));
-      const int hi = 32 * (int)(item % th) + lane;
-      const int B = hi < nh ? __ldg(ws.hlist + hi) : A;
-      const bool act = B != A, lower = B < A;
+      // HH: heavy atom i = 32 I + item % 32 and its partners 32 J + lane < i, J <= I;
+      // W rows through the tile ring
+      const int tile = (int)(item / 32);
+      int I = (int)((sqrtf(8.0f * (float)tile + 1.0f) - 1.0f) * 0.5f);
+      while (I * (I + 1) / 2 > tile) --I;
+      while ((I + 1) * (I + 2) / 2 <= tile) ++I;
+      const int J = tile - I * (I + 1) / 2;
+      const int i = 32 * I + (int)(item % 32), j = 32 * J + lane;
+      if (i >= nh || 32 * J >= i) continue;
+      const bool act = j < i;
+      const int A = __ldg(ws.hlist + i), B = act ? __ldg(ws.hlist + j) : A;
       const int fA = __ldg(a.at.first + A), fB = __ldg(a.at.first + B);
-      s_src[warp][0][lane] = (unsigned long long)(act ? w_block(a, A, 10, __ldg(a.at.wrow + A), B, 10) : a.w);
+      s_src[warp][lane] =
+          (unsigned long long)(act ? a.w + __ldg(a.at.wrow + A) + 10LL * __ldg(a.at.cum + B) : a.w);
       __syncwarp();
 #pragma unroll
-      for (int m = 0; m < kDepth; ++m) {
-        issue_win10(tiles + m * kTile, s_src[warp][0], (pidx(m) - 1) * 10, lane);
-        cp_async_commit();
-      }
-      double* rec = ws.stage + rec_off(A, numat, B, true);
-      double pj[16], pk[16], hm[4], sa[10];  // sa[0..3]: a lower lane's exchange sums of the current mu
+      for (int m = 0; m < 16; ++m)
+        if (m / 4 <= m % 4) {  // a row at its first visit
+          issue_win10(tiles + (pidx(m) - 1) * kTile, s_src[warp], (pidx(m) - 1) * 10, lane);
+          cp_async_commit();
+        }
+      double* recA = ws.stage + rec_off(A, numat, j, true);
+      double pj[16], pk[16], hm[4], sa[4], sb[10];
+      // A's density block in jab's gather order, term m on lane m
+      const int gx = (lane & 15) / 4, gy = lane & 3;
+      const double pi = __ldg(a.ptot + mb_tri(fA + max(gx, gy), fA + min(gx, gy)));
       if (act) {
         diag_block(a, fB, pj);
-        if (lower) {
 #pragma unroll
-          for (int x = 0; x < 4; ++x)
+        for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int y = 0; y < 4; ++y) pk[x * 4 + y] = __ldg(a.pa + (mb_tri(fA + x, fB + y)));
-        }
+          for (int y = 0; y < 4; ++y) pk[x * 4 + y] = __ldg(a.pa + (mb_tri(fA + x, fB + y)));
       }
 #pragma unroll
       for (int m = 0; m < 16; ++m) {
         const int x = m / 4, y = m % 4;
-        if (act && lower && y == 0) {
+        if (act && y == 0) {
 #pragma unroll
           for (int nu = 0; nu < 4; ++nu) hm[nu] = __ldg(a.h + (mb_tri(fA + x, fB + nu)));
         }
-        cp_async_wait(m + kDepth <= 16 ? kDepth - 1 : 15 - m);
-        __syncwarp();
-        const double* row = tiles + (m % kDepth) * kTile + lane * kSlot;  // row pidx(m) of the block
+        if (x <= y) {
+          cp_async_wait(kRows - 1 - first_visit(m));
+          __syncwarp();
+        }
+        const double* row = tiles + (pidx(m) - 1) * kTile + lane * kSlot;  // row pidx(m) of the block
+        const double pim = __shfl_sync(0xffffffffu, pi, m);
         if (act) {
-          if (lower) {
-            if (x <= y) {  // first visit of row pidx(m): A's Coulomb term for that pair index
-              double sb = DMUL(pj[0], row[pidx(0) - 1]);
+          double w[10];
 #pragma unroll
-              for (int mm = 1; mm < 16; ++mm) sb = DADD(sb, DMUL(pj[mm], row[pidx(mm) - 1]));
-              rec[pidx(m) - 1] = sb;
+          for (int q = 0; q < 10; ++q) w[q] = row[q];
+          if (x <= y) {  // first visit of row pidx(m): A's Coulomb term for that pair index
+            double sum = DMUL(pj[0], w[pidx(0) - 1]);
+#pragma unroll
+            for (int mm = 1; mm < 16; ++mm) sum = DADD(sum, DMUL(pj[mm], w[pidx(mm) - 1]));
+            recA[pidx(m) - 1] = sum;
+          }
+          // term m of each of B's ten elements
+#pragma unroll
+          for (int q = 0; q < 10; ++q) {
+            const double tt = DMUL(pim, w[q]);
+            sb[q] = m == 0 ? tt : DADD(sb[q], tt);
+          }
+          // kab: this row is pair(mu, lam) with mu = x + 1, lam = y + 1
+#pragma unroll
+          for (int nu = 1; nu <= 4; ++nu)
+#pragma unroll
+            for (int sig = 1; sig <= 4; ++sig) {
+              const double tt = DMUL(pk[y * 4 + sig - 1], w[pair1(nu, sig) - 1]);
+              sa[nu - 1] = (y == 0 && sig == 1) ? tt : DADD(sa[nu - 1], tt);
             }
-            // kab: this row is pair(mu, lam) with mu = x + 1, lam = y + 1
+          if (y == 3) {
 #pragma unroll
-            for (int nu = 1; nu <= 4; ++nu)
-#pragma unroll
-              for (int sig = 1; sig <= 4; ++sig) {
-                const double tt = DMUL(pk[y * 4 + sig - 1], row[pair1(nu, sig) - 1]);
-                sa[nu - 1] = (y == 0 && sig == 1) ? tt : DADD(sa[nu - 1], tt);
-              }
-            if (y == 3) {
-#pragma unroll
-              for (int nu = 0; nu < 4; ++nu) {
-                const long long idx = mb_tri(fA + x, fB + nu);
-                const double st = a.use_shift
-                                      ? DADD(DADD(hm[nu], DMUL(a.shift, pk[x * 4 + nu])), DMUL((double)(idx + 1), 1.0e-16))
-                                      : hm[nu];
-                a.f[idx] = DSUB(st, sa[nu]);
-              }
-            }
-          } else {
-            // block (B, A): term m of each of A's ten elements
-#pragma unroll
-            for (int q = 0; q < 10; ++q) {
-              const double tt = DMUL(pj[m], row[q]);
-              sa[q] = m == 0 ? tt : DADD(sa[q], tt);
-            }
-            if (m == 15) {
-#pragma unroll
-              for (int q = 0; q < 10; ++q) rec[q] = sa[q];
+            for (int nu = 0; nu < 4; ++nu) {
+              const long long idx = mb_tri(fA + x, fB + nu);
+              const double st = a.use_shift
+                                    ? DADD(DADD(hm[nu], DMUL(a.shift, pk[x * 4 + nu])), DMUL((double)(idx + 1), 1.0e-16))
+                                    : hm[nu];
+              a.f[idx] = DSUB(st, sa[nu]);
             }
           }
         }
-        __syncwarp();
-        if (m + kDepth < 16) {
-          issue_win10(tiles + (m % kDepth) * kTile, s_src[warp][0], (pidx(m + kDepth) - 1) * 10, lane);
-          cp_async_commit();
-        }
+      }
+      __syncwarp();
+      if (act) {
+        double2* recB = (double2*)(ws.stage + rec_off(B, numat, i, true));
+#pragma unroll
+        for (int q = 0; q < 5; ++q) recB[q] = make_double2(sb[2 * q], sb[2 * q + 1]);
       }
     } else if (item < r2) {
       // HX: heavy A, light partners llist[128 t + 32 g + lane]; one ten-double block each
-      const long long j = item - r1;
-      const int A = __ldg(ws.hlist + (j / tl));
-      const int base = (int)(j % tl) * 128;
+      const long long k = item - r1;
+      const int rank = (int)(k / tl), A = __ldg(ws.hlist + rank);
+      const int base = (int)(k % tl) * 128;
       const int fA = __ldg(a.at.first + A);
       const long long wrowA = __ldg(a.at.wrow + A);
+      unsigned long long* src = (unsigned long long*)(tiles + 4 * kTile);
       int Bs[4];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
         const int idx = base + 32 * g + lane;
         const int B = idx < nl ? __ldg(ws.llist + idx) : -1;
         Bs[g] = B;
-        s_src[warp][g][lane] = (unsigned long long)(B >= 0 ? w_block(a, A, 10, wrowA, B, 1) : a.w);
+        // the last tiles of an HX item are free: the windows' addresses
+        src[g * 32 + lane] = (unsigned long long)(B >= 0 ? w_block(a, A, 10, wrowA, B, 1) : a.w);
       }
       __syncwarp();
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        issue_win10(tiles + g * kTile, s_src[warp][g], 0, lane);
+        issue_win10(tiles + g * kTile, src + g * 32, 0, lane);
         cp_async_commit();
       }
+      double pi[10];  // A's diagonal density block, packed
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y <= x; ++y) pi[x * (x + 1) / 2 + y] = __ldg(a.ptot + mb_tri(fA + x, fA + y));
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
         const int B = Bs[g];
-        double pb = 0.0, pj[4];
-        int fB = 0;
+        double pj[4], hs[4];
+        long long idx[4];
         if (B >= 0) {
-          fB = __ldg(a.at.first + B);
-          pb = __ldg(a.ptot + (mb_tri(fB, fB)));
-          if (B < A) {
+          const int fB = __ldg(a.at.first + B);
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) pj[jj] = __ldg(a.pa + (mb_tri(fA + jj, fB)));
+          for (int q = 0; q < 4; ++q) {
+            idx[q] = B < A ? mb_tri(fA + q, fB) : mb_tri(fB, fA + q);
+            pj[q] = __ldg(a.pa + idx[q]);
+            hs[q] = f_start_pa(a, idx[q], pj[q]);
           }
         }
         cp_async_wait(3 - g);
         __syncwarp();
         if (B >= 0) {
           const double* wk = tiles + g * kTile + lane * kSlot;
-          double* rec = ws.stage + rec_off(A, numat, B, true);
+          // B's two additions (fock2's "ib - ia >= 3" / "jb - ja >= 3" branches)
+          double sumoff = 0.0, sumdia = 0.0;
 #pragma unroll
-          for (int q = 0; q < 10; ++q) rec[q] = DMUL(pb, wk[q]);
-          if (B < A) {  // kab on the 4 x 1 block
+          for (int x = 0; x < 4; ++x) {
 #pragma unroll
-            for (int i = 1; i <= 4; ++i) {
-              double sum = 0.0;
+            for (int y = 0; y < x; ++y) sumoff = DADD(sumoff, DMUL(pi[x * (x + 1) / 2 + y], wk[x * (x + 1) / 2 + y]));
+            sumdia = DADD(sumdia, DMUL(pi[x * (x + 1) / 2 + x], wk[x * (x + 1) / 2 + x]));
+          }
+          *(double2*)(ws.stage + rec_off(B, numat, rank, false)) = make_double2(DMUL(sumoff, 2.0), sumdia);
+          // kab on the 4 x 1 or 1 x 4 block
 #pragma unroll
-              for (int jj = 1; jj <= 4; ++jj) sum = DADD(sum, DMUL(pj[jj - 1], wk[pair1(i, jj) - 1]));
-              const long long idx = mb_tri(fA + i - 1, fB);
-              a.f[idx] = DSUB(f_start_pa(a, idx, pj[i - 1]), sum);
-            }
+          for (int x = 1; x <= 4; ++x) {
+            double sum = 0.0;
+#pragma unroll
+            for (int y = 1; y <= 4; ++y) sum = DADD(sum, DMUL(pj[y - 1], wk[pair1(x, y) - 1]));
+            a.f[idx[x - 1]] = DSUB(hs[x - 1], sum);
           }
         }
       }
       __syncwarp();
     } else {
-      // LX: light A, partners 128 t + 32 g + lane; blocks of at most ten
-      // doubles read straight from W (row A's are contiguous over B < A)
-      const long long j = item - r2;
-      const int A = __ldg(ws.llist + (j / ta));
-      const int base = (int)(j % ta) * 128;
-      const int fA = __ldg(a.at.first + A);
-      const long long wrowA = __ldg(a.at.wrow + A);
-#pragma unroll 1
-      for (int g = 0; g < 4; ++g) {
-        const int B = base + 32 * g + lane;
-        if (B < numat && B != A) {
-          const double* wk = w_block(a, A, 1, wrowA, B, __ldg(a.at.lim + B));
-          double out[10];
-          pair_x(a, A, fA, 1, B, wk, out);
-          double* rec = ws.stage + rec_off(A, numat, B, false);
-          rec[0] = out[0];
-          rec[1] = out[1];
-        }
+      // LL: light A, the light partners below it
+      const int k = (int)(item - r2), A = __ldg(ws.llist + k);
+      const double* row = a.w + __ldg(a.at.wrow + A);
+      const long long f0 = mb_tri(__ldg(a.at.first + A), 0);
+#pragma unroll 4
+      for (int l = lane; l < k; l += 32) {
+        const int B = __ldg(ws.llist + l);
+        const long long idx = f0 + __ldg(a.at.first + B);
+        const double pab = __ldg(a.pa + idx);
+        a.f[idx] = DSUB(f_start_pa(a, idx, pab), DMUL(pab, __ldg(row + __ldg(a.at.cum + B))));
       }
     }
   }
 }
 
-// Pass 2: one CTA per atom; owners e < lim[A] fold in partner order.
+// Pass 2: one CTA per atom; owners e < lim[A] fold in partner order, the chain of
+// additions being the least time this takes.  In step k, one warp folds chunk
+// k - 2 while the other warps copy chunk k, whose addresses they found in step k - 1,
+// and find those of chunk k + 1.
 __global__ void __launch_bounds__(kFoldThreads) fock2_fold(FockArgs a, FockWs ws) {
-  extern __shared__ double s_buf[];  // kFoldDepth chunks of kFoldThreads records
-  const int A = blockIdx.x, tid = threadIdx.x;
+  extern __shared__ double s_buf[];  // kFoldDepth chunks of kChunk records
+  __shared__ const double* s_src[2][kChunk];
+  __shared__ double s_fac[kFoldDepth][kChunk];  // a light partner's density, 1 for a staged record
+  const int A = blockIdx.x, tid = threadIdx.x, pt = tid - 32;
   const int numat = a.at.numat;
   const int fA = __ldg(a.at.first + A), nA = __ldg(a.at.nor + A), lA = __ldg(a.at.lim + A);
   const bool heavy = nA == 4;
-  const int wv = heavy ? kStageW : 2;
   const long long wrowA = __ldg(a.at.wrow + A);
-  const double* src = ws.stage + rec_off(A, numat, 0, heavy);
+  const int cA = __ldg(a.at.cum + A);
+  const double* pl = light_density(ws, ws.counts[0]);
 
   double run = 0.0, f1 = 0.0;
   long long own_idx = 0;
@@ -461,12 +432,15 @@ __global__ void __launch_bounds__(kFoldThreads) fock2_fold(FockArgs a, FockWs ws
     own_idx = mb_tri(fA + iw - 1, fA + jw - 1);
     run = f_start(a, own_idx, iw == jw);
     // fock1 (SCF/fock1.F90): one-centre Coulomb and exchange for element (iw, jw)
-    const double* w1 = a.w + wrowA + (long long)lA * __ldg(a.at.cum + A);
+    const double* w1 = a.w + wrowA + (long long)lA * cA;
     const int ilim = lA;
     const int ijw = iw * (iw - 1) / 2 + jw;
     double sum = 0.0;
-    for (int kw = 1; kw <= nA; ++kw)
-      for (int lw = 1; lw <= nA; ++lw) {
+#pragma unroll
+    for (int kw = 1; kw <= 4; ++kw)
+#pragma unroll
+      for (int lw = 1; lw <= 4; ++lw) {
+        if (kw > nA || lw > nA) continue;
         int ip = kw > lw ? kw : lw, jp = kw < lw ? kw : lw;
         long long ijp = mb_tri(fA + ip - 1, fA + jp - 1);
         int klw = ip * (ip - 1) / 2 + jp;
@@ -480,48 +454,83 @@ __global__ void __launch_bounds__(kFoldThreads) fock2_fold(FockArgs a, FockWs ws
     f1 = sum;
   }
 
-  const int nchunk = (numat + kFoldThreads - 1) / kFoldThreads;
-  for (int k = 0; k < kFoldDepth + nchunk; ++k) {
-    if (k >= kFoldDepth) {
-      // fold chunk c = k - kFoldDepth
-      const int c = k - kFoldDepth;
-      cp_async_wait(kFoldDepth - 1);
-      __syncthreads();
-      if (tid < lA) {
-        const double* buf = s_buf + (c % kFoldDepth) * kFoldThreads * kStageW;
-        const int b0 = c * kFoldThreads;
-        const int nb = min(kFoldThreads, numat - b0);
-        const int tA = (A >= b0 && A < b0 + nb) ? A - b0 : nb;
+  const int nchunk = (numat + kChunk - 1) / kChunk;
+  const double* src = a.w;  // this thread's partner of chunk k, and its factor
+  double fac = 1.0;
+  bool staged = false;
+  auto find = [&](int k) {
+    const int B = k * kChunk + pt;
+    src = a.w;
+    fac = 1.0;
+    staged = false;
+    if (k < nchunk && B < numat && B != A) {
+      const int hB = heavy_below(a.at, B);
+      staged = __ldg(a.at.nor + B) == 4;
+      if (staged) src = ws.stage + rec_off(A, numat, hB, heavy);
+      else src = B < A ? a.w + wrowA + (long long)lA * __ldg(a.at.cum + B) : a.w + __ldg(a.at.wrow + B) + cA;
+      if (!staged) fac = __ldg(pl + (B - hB));
+    }
+    s_src[k & 1][pt] = src;
+  };
+  if (pt >= 0) find(0);
+  __syncthreads();
+  for (int k = 0; k < nchunk + 2; ++k) {
+    if (pt >= 0) {
+      if (k < nchunk) {
+        double* dst = s_buf + (k % kFoldDepth) * kChunk * kStageW;
+        s_fac[k % kFoldDepth][pt] = fac;
         if (heavy) {
-#pragma unroll 8
-          for (int t = 0; t < tA; ++t) run = DADD(run, buf[t * kStageW + tid]);
-          if (tA < nb) {
-            run = DADD(run, f1);
-#pragma unroll 8
-            for (int t = tA + 1; t < nb; ++t) run = DADD(run, buf[t * kStageW + tid]);
-          }
+          const int n = min(kChunk, numat - k * kChunk) * kStageW;
+          for (int q = pt; q < n; q += kChunk) cp_async8(dst + q, s_src[k & 1][q / kStageW] + q % kStageW);
         } else {
-#pragma unroll 8
-          for (int t = 0; t < tA; ++t) run = DADD(DADD(run, buf[2 * t]), buf[2 * t + 1]);
-          if (tA < nb) {
-            run = DADD(run, f1);
-#pragma unroll 8
-            for (int t = tA + 1; t < nb; ++t) run = DADD(DADD(run, buf[2 * t]), buf[2 * t + 1]);
-          }
+          cp_async8(dst + 2 * pt, src);
+          if (staged) cp_async8(dst + 2 * pt + 1, src + 1);
+          else dst[2 * pt + 1] = -0.0;
         }
       }
-      __syncthreads();
+      cp_async_commit();
+      find(k + 1);
+      cp_async_wait(1);  // chunk k - 1 is here
+    } else if (k >= 2 && tid < lA) {
+      const int c = k - 2;
+      const double* buf = s_buf + (c % kFoldDepth) * kChunk * kStageW;
+      const double* fc = s_fac[c % kFoldDepth];
+      const int b0 = c * kChunk;
+      const int nb = min(kChunk, numat - b0);
+      const int tA = (A >= b0 && A < b0 + nb) ? A - b0 : nb;
+      auto fold = [&](int t0, int t1) {
+        if (heavy) {
+          int t = t0;
+          for (; t + 8 <= t1; t += 8) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = DMUL(fc[t + u], buf[(t + u) * kStageW + tid]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) run = DADD(run, v[u]);
+          }
+          for (; t < t1; ++t) run = DADD(run, DMUL(fc[t], buf[t * kStageW + tid]));
+        } else {
+          int t = t0;
+          for (; t + 8 <= t1; t += 8) {
+            double v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) v[u] = buf[2 * t + u];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[2 * u] = DMUL(fc[t + u], v[2 * u]);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) run = DADD(run, v[u]);
+          }
+          for (; t < t1; ++t) run = DADD(DADD(run, DMUL(fc[t], buf[2 * t])), buf[2 * t + 1]);
+        }
+      };
+      fold(0, tA);
+      if (tA < nb) {
+        run = DADD(run, f1);
+        fold(tA + 1, nb);
+      }
     }
-    // prefetch chunk k into slot k % kFoldDepth (the slot chunk k - kFoldDepth just left)
-    if (k < nchunk) {
-      const int b0 = k * kFoldThreads;
-      const int n = min(kFoldThreads, numat - b0) * wv;
-      double* dst = s_buf + (k % kFoldDepth) * kFoldThreads * kStageW;
-      for (int q = tid; q < n; q += kFoldThreads) cp_async8(dst + q, src + (long long)b0 * wv + q);
-    }
-    cp_async_commit();
+    __syncthreads();
   }
-  cp_async_wait(0);
   if (tid < lA) a.f[own_idx] = run;
 }
 
@@ -534,11 +543,11 @@ int fock_attrs() {
   std::lock_guard<std::mutex> lock(mu);
   if (!done[dev]) {
     MB_CUDA(cudaFuncSetAttribute(fock2_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(double) * kWarps * kDepth * kTile)));
+                                 (int)(sizeof(double) * kWarps * kRows * kTile)));
     MB_CUDA(cudaFuncSetAttribute(fock2_pairs, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared));
     MB_CUDA(cudaFuncSetAttribute(fock2_fold, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(double) * kFoldDepth * kFoldThreads * kStageW)));
+                                 (int)(sizeof(double) * kFoldDepth * kChunk * kStageW)));
     done[dev] = true;
   }
   return MB_OK;
@@ -578,12 +587,11 @@ extern "C" int mb_fock2_ws(const MbAtomsDev* atoms, double* f, const double* h, 
   MB_CUDA(cudaGetDevice(&dev));
   MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   mb_kstat_mark(MB_KSTAT_FOCK, stream, true);
-  fock2_lists<<<1, 1024, 0, stream>>>(a.at, fw);
+  fock2_lists<<<(atoms->numat + 127) / 128, 128, 0, stream>>>(a.at, ptot, fw);
   MB_LAUNCH_CHECK();
-  fock2_pairs<<<sms * 3, 32 * kWarps, sizeof(double) * kWarps * kDepth * kTile, stream>>>(a, fw);
+  fock2_pairs<<<sms * 4, 32 * kWarps, sizeof(double) * kWarps * kRows * kTile, stream>>>(a, fw);
   MB_LAUNCH_CHECK();
-  fock2_fold<<<atoms->numat, kFoldThreads, sizeof(double) * kFoldDepth * kFoldThreads * kStageW, stream>>>(a,
-                                                                                                             fw);
+  fock2_fold<<<atoms->numat, kFoldThreads, sizeof(double) * kFoldDepth * kChunk * kStageW, stream>>>(a, fw);
   MB_LAUNCH_CHECK();
   mb_kstat_mark(MB_KSTAT_FOCK, stream, false);
   return MB_OK;
