@@ -14,7 +14,7 @@
 //     per off-diagonal element forms its exchange sum -- the operation order
 //     of fock2/fock1, so F is bit-identical to the oracle;
 //   * eigensolve in shared memory: Householder reduction to tridiagonal form
-//     (warp per row, two barriers per column), eigenvalues through the LUMO
+//     (16 x 16 thread tiles, two barriers per column), eigenvalues through the LUMO
 //     by 5-section Sturm counts (four lanes per eigenvalue), the occupied
 //     eigenvectors of T by inverse iteration (thread per vector, clusters
 //     re-orthogonalised), back-transformation (a lane group per vector);
@@ -327,102 +327,92 @@ __device__ double cta_helect(int n, const double* p, double cpa, const double* h
 // and, when vectors, the eigenvectors of the lowest nz in S.Z.  scr: the
 // CTA's global scratch (LU factors, then the reflectors when Z overlays A).
 
-// Sturm count of T - x I (d, e2 = e^2).
-__device__ int sturm(int n, const double* d, const double* e2, double x, double pivmin) {
-  int cnt = 0;
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  cnt += q < 0.0;
-  for (int i = 1; i < n; ++i) {
-    q = d[i] - x - e2[i - 1] * recip_nr2(q);
-    if (fabs(q) < pivmin) q = -pivmin;
-    cnt += q < 0.0;
-  }
-  return cnt;
-}
+// (Built without contraction for the Fock build's sake: the multiply-adds of the
+// eigensolver and the density are written out.)
 
-// reltol: relative width at which an eigenvalue's bracket stops shrinking.
-template <int BT_NB>
-__device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, double* scr, long long* ph) {
+// Columns k0 .. kend-1 of the Householder reduction, whose active rows lie in the
+// last NA tiles of 16: two barriers a column, the reflector's norm from the
+// previous column's update.  Thread (tr, tc) of the 16 x 16 works on element
+// (tr, tc) of every tile, so with the tiles' count constant each address is a base
+// and an offset known to the compiler, where addresses formed per element took
+// most of the issue slots: 1500 alkanes C3..C20 27.7 -> 22.0 ms with the Sturm
+// counts below (one B200; 26.5 when inlined, for the registers it takes from the
+// other phases).
+// Rows and columns below k + 1 take part with zeros; the rows from n up to the
+// tile's edge are zero.
+template <int NA>
+__device__ __noinline__ void reduce_columns(int k0, int kend, int n, double* A, double* redA, double* Sd, double* Se,
+                                            double* Stau, double* Spv, double* Sv) {
+  constexpr int P = NA > 4 ? 8 : NA > 2 ? 4 : NA;  // rows a lane group reduces, a power of two
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, tr = tid >> 4, tc = tid & 15;
-  double* A = S.A;
-  double* redA = S.red;
-  double* redB = S.red + BT_W;
-  // ---- Householder reduction to tridiagonal form, lower, two barriers per
-  // column: the reflector's norm comes from the previous column's update.
-  // The 16 x 16 tile covers n - 1 <= 127 rows and columns in 8 steps.
-  {
-    double part = 0.0;
-    for (int i = 2 + tid; i < n; i += BT_T) part += A[tri(i, 0)] * A[tri(i, 0)];
-    part = warp_sum(part);
-    if (lane == 0) redA[wp] = part;
-    __syncthreads();
+  double* redB = redA + BT_W;
+  const int base = (((n + 15) >> 4) - NA) * 16;
+  int rb[NA], cb[NA], db[NA];  // tile (a, b): row element at rb[a] + 16 b, its mirror image at cb[b] + 16 a
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+    const int i = base + tr + 16 * a, j = base + tc + 16 * a;
+    rb[a] = i * (i + 1) / 2 + base + tc;
+    cb[a] = j * (j + 1) / 2 + base + tr;
+    db[a] = (tc <= tr ? rb[a] : cb[a]) + 16 * a;
   }
-  for (int k = 0; k < n - 2; ++k) {
+  for (int k = k0; k < kend; ++k) {
+    const int k1 = k + 1;
     double sigma = redA[0];
 #pragma unroll
     for (int q = 1; q < BT_W; ++q) sigma += redA[q];
-    const double alpha = A[tri(k + 1, k)];
+    const double alpha = A[tri(k1, k)];
     double beta, tau, scal;
     if (sigma == 0.0) { beta = alpha; tau = 0.0; scal = 0.0; }
     else {
-      beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
+      beta = -copysign(sqrt(fma(alpha, alpha, sigma)), alpha);
       tau = (beta - alpha) / beta;
       scal = 1.0 / (alpha - beta);
     }
     if (tid == 0) {
-      S.e[k] = beta;
-      S.tau[k] = tau;
-      S.d[k] = A[tri(k, k)];
+      Se[k] = beta;
+      Stau[k] = tau;
+      Sd[k] = A[tri(k, k)];
     }
-    // p = tau A22 v on a 16 x 16 thread tile: thread (tr, tc) sums rows
-    // k+1+tr+16a over columns k+1+tc+16b, v on the fly from column k; the
-    // row sums are reduced over the 16 lanes of a half-warp.
-    const int k1 = k + 1;
-    // tile rows i = k1 + tr + 16 a < n, columns j = k1 + tc + 16 b < n; nrw
-    // bounds a for both half-warps of this warp (the shuffles stay uniform)
-    const int nrw = (n - k1 - 2 * wp + 15) >> 4;
-    double vr[8];
+    // p = tau A22 v: row sums over this thread's columns, then over the 16
+    // lanes, which share the rows among them
+    double vr[NA], acc[P];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const int j = k1 + tc + 16 * b;
-      vr[b] = 0.0;
-      if (j < n) vr[b] = (j == k1) ? 1.0 : A[j * (j + 1) / 2 + k] * scal;
+    for (int b = 0; b < NA; ++b) {
+      const int j = base + tc + 16 * b;
+      vr[b] = j < k1 ? 0.0 : j == k1 ? 1.0 : A[cb[b] - base - tr + k] * scal;
     }
-    double acc[8];
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
+    for (int a = 0; a < P; ++a) {
       acc[a] = 0.0;
-      const int i = k1 + tr + 16 * a;
-      if (i >= n) break;
-      const int rbase = i * (i + 1) / 2;
-      double s = 0.0;
+      if (a < NA) {
 #pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const int j = k1 + tc + 16 * b;
-        if (j >= n) break;
-        s += (j <= i ? A[rbase + j] : A[j * (j + 1) / 2 + i]) * vr[b];
+        for (int b = 0; b < NA; ++b)
+          acc[a] = fma(A[a > b ? rb[a] + 16 * b : a < b ? cb[b] + 16 * a : db[a]], vr[b], acc[a]);
       }
-      acc[a] = s;
     }
+    int a_own = 0;
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      if (a >= nrw) break;
+    for (int h = P / 2, o = 8; o > 0; h /= 2, o /= 2) {
+      if (h > 0) {
+        const bool up = (tc & o) != 0;
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], o);
+        for (int q = 0; q < h; ++q) {
+          const double send = up ? acc[q] : acc[q + h];
+          acc[q] = (up ? acc[q + h] : acc[q]) + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+        if (up) a_own += h;
+      } else {
+        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+      }
     }
     double dot = 0.0;
-    if (tc == 0) {
-#pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const int i = k1 + tr + 16 * a;
-        if (i >= n) break;
-        const double vi = (i == k1) ? 1.0 : A[i * (i + 1) / 2 + k] * scal;
-        const double s = acc[a] * tau;
-        S.pv[i] = s;
-        S.v[i] = vi;
-        dot += s * vi;
-      }
+    if ((tc & (16 / P - 1)) == 0 && a_own < NA) {
+      const int i = base + tr + 16 * a_own;
+      const double vi = i < k1 ? 0.0 : i == k1 ? 1.0 : A[i * (i + 1) / 2 + k] * scal;
+      const double s = i < k1 ? 0.0 : acc[0] * tau;
+      Spv[i] = s;
+      Sv[i] = vi;
+      dot = s * vi;
     }
     dot = warp_sum(dot);
     if (lane == 0) redB[wp] = dot;
@@ -431,40 +421,118 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
 #pragma unroll
     for (int q = 1; q < BT_W; ++q) dt += redB[q];
     const double kk = 0.5 * tau * dt;
-    // A22 -= v w^T + w v^T, w = p - kk v, on the same tile; the reflector
-    // replaces column k; squares of the new column k + 1 below its
-    // subdiagonal give the next norm
-    double wr[8];
+    // A22 -= v w^T + w v^T, w = p - kk v; the reflector replaces column k;
+    // squares of the new column k + 1 below its subdiagonal give the next norm
+    double wr[NA];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const int j = k1 + tc + 16 * b;
-      vr[b] = 0.0;
-      wr[b] = 0.0;
-      if (j < n) {
-        vr[b] = S.v[j];
-        wr[b] = S.pv[j] - kk * vr[b];
-      }
+    for (int b = 0; b < NA; ++b) {
+      const int j = base + tc + 16 * b;
+      vr[b] = Sv[j];
+      wr[b] = fma(-kk, vr[b], Spv[j]);
     }
     double nxt = 0.0;
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int i = k1 + tr + 16 * a;
-      if (i >= n) break;
-      const int rbase = i * (i + 1) / 2;
-      const double vi = S.v[i], wi = S.pv[i] - kk * vi;
+    for (int a = 0; a < NA; ++a) {
+      const int i = base + tr + 16 * a;
+      const double vi = Sv[i], wi = fma(-kk, vi, Spv[i]);
 #pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const int j = k1 + tc + 16 * b;
-        if (j > i) break;
-        const double x = A[rbase + j] - (vi * wr[b] + wi * vr[b]);
-        A[rbase + j] = x;
-        if (b == 0 && tc == 0 && i >= k + 3) nxt += x * x;
+      for (int b = 0; b <= a; ++b) {
+        if (b == a && tc > tr) continue;
+        double* x = A + rb[a] + 16 * b;
+        const double u = fma(-vi, wr[b], fma(-wi, vr[b], *x));
+        *x = u;
+        if (b == 0 && tc == (k1 & 15) && i >= k + 3) nxt = fma(u, u, nxt);
       }
-      if (tc == 0 && i >= k + 2) A[rbase + k] = vi;
+      if (tc == (k & 15) && i >= k + 2) A[rb[a] - base - tc + k] = vi;
     }
     nxt = warp_sum(nxt);
     if (lane == 0) redA[wp] = nxt;
     __syncthreads();
+  }
+}
+
+// Sturm count from the leading principal minors' three-term recurrence,
+// p_i = (d_i - x) p_(i-1) - e_(i-1)^2 p_(i-2): a dependent chain of one multiply-add
+// a row, where the quotients p_i / p_(i-1) take a reciprocal.  Eight rows at a time
+// from a pair scaled by a power of two; T has norm <= 1, so a row grows p at most
+// threefold.  A block in which some |p_i| falls below 1e-120 (2^-398) is taken again by
+// quotients.  de[i] = (d_i, e_(i-1)^2), followed by 2 SB records (2, 0): rows that
+// keep the sign of p.
+constexpr int SB = 8;
+constexpr int kSturmTiny = 0x27100000;  // high word of 2^-398
+constexpr double kPivmin = 1.0e-290;
+
+__device__ __forceinline__ int sturm(int n, const double2* de, double x) {
+  double p1 = de[0].x - x, p0 = 1.0;
+  if (fabs(p1) < kPivmin) p1 = -kPivmin;
+  int cnt = p1 < 0.0;
+  for (int i0 = 1; i0 < n; i0 += SB) {
+    double db[SB], eb[SB];
+#pragma unroll
+    for (int u = 0; u < SB; ++u) {
+      const double2 t = de[i0 + u];
+      db[u] = t.x - x;
+      eb[u] = t.y;
+    }
+    const int ex = max((__double2hiint(p0) >> 20) & 0x7ff, (__double2hiint(p1) >> 20) & 0x7ff);
+    const double sc = __hiloint2double((2046 - ex) << 20, 0);
+    p0 *= sc;
+    p1 *= sc;
+    const double s0 = p0, s1 = p1;
+    int c = 0, least = 0x7fffffff;  // high words of |p| order as |p| does
+#pragma unroll
+    for (int u = 0; u < SB; ++u) {
+      const double p2 = fma(db[u], p1, -(eb[u] * p0));
+      c += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+      least = min(least, __double2hiint(p2) & 0x7fffffff);
+      p0 = p1;
+      p1 = p2;
+    }
+    if (least < kSturmTiny) {
+      double q = s1 / s0;
+      if (fabs(q) < kPivmin) q = -kPivmin;
+      c = 0;
+      for (int u = 0; u < SB && i0 + u < n; ++u) {
+        q = fma(-eb[u], recip_nr2(q), db[u]);
+        if (fabs(q) < kPivmin) q = -kPivmin;
+        c += q < 0.0;
+      }
+      p0 = 1.0;
+      p1 = q;  // the pair matters up to a factor only
+    }
+    cnt += c;
+  }
+  return cnt;
+}
+
+// reltol: relative width at which an eigenvalue's bracket stops shrinking.
+template <int BT_NB>
+__device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, double* scr, long long* ph) {
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  double* A = S.A;
+  // ---- Householder reduction to tridiagonal form, lower
+  const int ntile = (n + 15) >> 4;
+  {
+    double part = 0.0;
+    for (int i = 2 + tid; i < n; i += BT_T) part = fma(A[tri(i, 0)], A[tri(i, 0)], part);
+    for (int q = n * (n + 1) / 2 + tid; q < 8 * ntile * (16 * ntile + 1); q += BT_T) A[q] = 0.0;
+    part = warp_sum(part);
+    if (lane == 0) S.red[wp] = part;
+    __syncthreads();
+  }
+  for (int na = ntile; na >= 1; --na) {
+    // columns k whose row k + 1 is the first active row's tile
+    const int base = (ntile - na) * 16, k0 = base > 0 ? base - 1 : 0, kend = min(base + 15, n - 2);
+    switch (na) {
+      case 8: reduce_columns<8>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+      case 7: reduce_columns<7>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+      case 6: reduce_columns<6>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+      case 5: reduce_columns<5>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+      case 4: reduce_columns<4>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+      case 3: reduce_columns<3>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+      case 2: reduce_columns<2>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+      default: reduce_columns<1>(k0, kend, n, A, S.red, S.d, S.e, S.tau, S.pv, S.v); break;
+    }
   }
   if (tid == 0) {
     if (n >= 2) {
@@ -481,21 +549,36 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
     for (int q = tid; q < n * (n + 1) / 2; q += BT_T) refl[q] = A[q];
   __syncthreads();
   ph_mark(ph, 2);
-  // ---- bounds, e^2
-  if (tid == 0) {
-    double lo = 1e300, hi = -1e300, em = 0.0;
-    for (int i = 0; i < n; ++i) {
+  // ---- bounds; T scaled by a power of two to norm <= 1 as the records of the
+  // Sturm counts (in the room of the back-transformation's T)
+  double2* de = reinterpret_cast<double2*>(S.tw);
+  if (tid < 32) {
+    double lo = 1e300, hi = -1e300;
+    for (int i = lane; i < n; i += 32) {
       const double r = (i > 0 ? fabs(S.e[i - 1]) : 0.0) + (i < n - 1 ? fabs(S.e[i]) : 0.0);
       lo = fmin(lo, S.d[i] - r);
       hi = fmax(hi, S.d[i] + r);
-      if (i < n - 1) { S.e2[i] = S.e[i] * S.e[i]; em = fmax(em, S.e2[i]); }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
     const double tnorm = fmax(fabs(lo), fabs(hi));
     const double pad = 2.0 * 2.220446049250313e-16 * tnorm * n + 1e-300;
-    S.scal[4] = lo - pad;
-    S.scal[5] = hi + pad;
-    S.scal[6] = fmax(1e-290, 2.2250738585072014e-308 * fmax(1.0, em));
-    S.scal[7] = tnorm;
+    // 2^-e with tnorm < 2^e; 1 when the norm is zero or not finite, or tiny
+    const int ex = (__double2hiint(tnorm) >> 20) & 0x7ff;
+    const double sc = (ex > 64 && ex < 1982) ? __hiloint2double((2045 - ex) << 20, 0) : 1.0;
+    if (lane == 0) {
+      S.scal[4] = lo - pad;
+      S.scal[5] = hi + pad;
+      S.scal[6] = sc;
+      S.scal[7] = tnorm;
+    }
+    for (int i = lane; i < n + 2 * SB; i += 32) {
+      const double ep = i > 0 && i < n ? S.e[i - 1] * sc : 0.0;
+      de[i] = i < n ? make_double2(S.d[i] * sc, ep * ep) : make_double2(2.0, 0.0);
+    }
   }
   __syncthreads();
   // ---- eigenvalues 0 .. LUMO by 5-section, four lanes per eigenvalue.  Every
@@ -503,8 +586,8 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
   // the 4-lane shuffles always see a converged warp.
   {
     const int grp = tid >> 2, ln = tid & 3, base = tid & 31 & ~3;
-    const double pivmin = S.scal[6];
-    const double atol = 2.220446049250313e-16 * S.scal[7] + pivmin;
+    const double sc = S.scal[6];
+    const double atol = 2.220446049250313e-16 * S.scal[7] + 1e-290;
     const int nlo = nz > 1 ? nz : 1;
     const int nev = nlo + 1 < n ? nlo + 1 : n;
     const int rounds = (nev + BT_T / 4 - 1) / (BT_T / 4);
@@ -516,7 +599,7 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
       for (int it = 0; it < 100; ++it) {
         if (!done && hi - lo <= reltol * fmax(fabs(lo), fabs(hi)) + atol) done = true;
         const double x = lo + (hi - lo) * ((double)(ln + 1) / 5.0);
-        const int cnt = done ? 0 : sturm(n, S.d, S.e2, x, pivmin);
+        const int cnt = done ? 0 : sturm(n, de, x * sc);
         const int flag = cnt > mm ? 1 : 0;
         int above = 0;
 #pragma unroll
@@ -585,13 +668,13 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
               const double rp = recip_nr2(pv);
               const double l = sub * rp;
               u0[i] = rp; u1[i] = du; u2[i] = 0.0; ul[i] = l; us[i] = 0.0;
-              dd = dn - l * du;
+              dd = fma(-l, du, dn);
               du = en;
             } else {
               const double rs = recip_nr2(sub);
               const double l = dd * rs;
               u0[i] = rs; u1[i] = dn; u2[i] = en; ul[i] = l; us[i] = 1.0;
-              dd = du - l * dn;
+              dd = fma(-l, dn, du);
               du = -l * en;
             }
           }
@@ -613,29 +696,29 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
             const double xn = itr == 0 ? rnd() : x[(i + 1) * nz];
             if (us[i] != 0.0) {
               x[i * nz] = xn;
-              xr = xr - ul[i] * xn;
+              xr = fma(-ul[i], xn, xr);
             } else {
               x[i * nz] = xr;
-              xr = xn - ul[i] * xr;
+              xr = fma(-ul[i], xr, xn);
             }
           }
           double x1 = xr * u0[n - 1], x2 = 0.0;
           x[(n - 1) * nz] = x1;
           for (int i = n - 2; i >= 0; --i) {
-            const double vv = (x[i * nz] - u1[i] * x1 - u2[i] * x2) * u0[i];
+            const double vv = fma(-u2[i], x2, fma(-u1[i], x1, x[i * nz])) * u0[i];
             x[i * nz] = vv;
             x2 = x1;
             x1 = vv;
           }
           for (int q = m0; q < mv; ++q) {  // re-orthogonalise against earlier members
             double dq = 0.0;
-            for (int i = 0; i < n; ++i) dq += Z[i * nz + q] * x[i * nz];
-            for (int i = 0; i < n; ++i) x[i * nz] -= dq * Z[i * nz + q];
+            for (int i = 0; i < n; ++i) dq = fma(Z[i * nz + q], x[i * nz], dq);
+            for (int i = 0; i < n; ++i) x[i * nz] = fma(-dq, Z[i * nz + q], x[i * nz]);
           }
           // normalise (one solve from a unit vector grows it by at most
           // n / tiny, far inside the double range)
           double ss = 0.0;
-          for (int i = 0; i < n; ++i) ss += x[i * nz] * x[i * nz];
+          for (int i = 0; i < n; ++i) ss = fma(x[i * nz], x[i * nz], ss);
           const double sc = ss > 0.0 ? 1.0 / sqrt(ss) : 0.0;
           for (int i = 0; i < n; ++i) x[i * nz] *= sc;
         }
@@ -668,7 +751,7 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
         while (j >= c) { j -= c; ++c; }
         if (c < nbb) {
           double g = 0.0;
-          for (int i = kb + c + 1; i < n; ++i) g += vref(i, kb + j) * vref(i, kb + c);
+          for (int i = kb + c + 1; i < n; ++i) g = fma(vref(i, kb + j), vref(i, kb + c), g);
           T[j * BT_NB + c] = g;
         }
       }
@@ -681,7 +764,7 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
           for (int j = 0; j < BT_NB; ++j) {
             double s = 0.0;
             if (j < c)
-              for (int l = j; l < c; ++l) s += T[j * BT_NB + l] * T[l * BT_NB + c];
+              for (int l = j; l < c; ++l) s = fma(T[j * BT_NB + l], T[l * BT_NB + c], s);
             t[j] = s;
           }
 #pragma unroll
@@ -710,13 +793,13 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
         for (; i < n && i <= kb + BT_NB; i += g) {
           const double z = Z[i * nz + col];
 #pragma unroll
-          for (int c = 0; c < BT_NB; ++c) acc[c] += vref(i, kb + c) * z;
+          for (int c = 0; c < BT_NB; ++c) acc[c] = fma(vref(i, kb + c), z, acc[c]);
         }
         for (; i < n; i += g) {
           const double z = Z[i * nz + col];
           const double* rr = refl + i * (i + 1) / 2 + kb;
 #pragma unroll
-          for (int c = 0; c < BT_NB; ++c) acc[c] += rr[c] * z;
+          for (int c = 0; c < BT_NB; ++c) acc[c] = fma(rr[c], z, acc[c]);
         }
       }
 #pragma unroll
@@ -729,7 +812,7 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
       for (int c = 0; c < BT_NB; ++c) {
         double s = 0.0;
 #pragma unroll
-        for (int j = c; j < BT_NB; ++j) s += T[c * BT_NB + j] * acc[j];
+        for (int j = c; j < BT_NB; ++j) s = fma(T[c * BT_NB + j], acc[j], s);
         wv[c] = s;
       }
       if (act) {
@@ -737,14 +820,14 @@ __device__ void cta_eigh(int n, int nz, bool vectors, double reltol, Smem& S, do
         for (; i < n && i <= kb + BT_NB; i += g) {
           double s = 0.0;
 #pragma unroll
-          for (int c = 0; c < BT_NB; ++c) s += vref(i, kb + c) * wv[c];
+          for (int c = 0; c < BT_NB; ++c) s = fma(vref(i, kb + c), wv[c], s);
           Z[i * nz + col] -= s;
         }
         for (; i < n; i += g) {
           const double* rr = refl + i * (i + 1) / 2 + kb;
           double s = 0.0;
 #pragma unroll
-          for (int c = 0; c < BT_NB; ++c) s += rr[c] * wv[c];
+          for (int c = 0; c < BT_NB; ++c) s = fma(rr[c], wv[c], s);
           Z[i * nz + col] -= s;
         }
       }
@@ -863,7 +946,7 @@ __device__ void cta_density(int n, int nz, const Smem& S, double* p) {
     int r, c;
     tri_rc(q, r, c);
     double s = 0.0;
-    for (int m = 0; m < nz; ++m) s += S.Z[r * nz + m] * S.Z[c * nz + m];
+    for (int m = 0; m < nz; ++m) s = fma(S.Z[r * nz + m], S.Z[c * nz + m], s);
     p[q] = 2.0 * s;
   }
   __syncthreads();
