@@ -139,8 +139,9 @@ __device__ __forceinline__ long long rec_off(int A, int numat, int rank, bool he
   return (long long)A * numat * kStageW + (long long)rank * (heavy ? kStageW : 2);
 }
 
-// Heavy atoms below atom A (one or four orbitals an atom).
-__device__ __forceinline__ int heavy_below(const MbAtoms& at, int A) { return (__ldg(at.first + A) - A) / 3; }
+// Heavy atoms below atom A: cum counts ten pairs for each of them and one for a
+// light atom.  (first is no measure of it: orbitals may begin anywhere and leave gaps.)
+__device__ __forceinline__ int heavy_below(const MbAtoms& at, int A) { return (__ldg(at.cum + A) - A) / 9; }
 
 __device__ __forceinline__ double f_start(const FockArgs& a, long long idx, bool diag) {
   if (!a.use_shift) return __ldg(a.h + idx);

@@ -1108,12 +1108,12 @@ __device__ __forceinline__ double dhc_energy(int n1, int n2, const double* x1, c
   return e + enuc;
 }
 
-// The k-th (from 0) atom of numat that has four orbitals (heavy) or one: with
-// one or four orbitals an atom, first[a] - a is three times the heavy atoms below a.
-__device__ __forceinline__ int kth_atom(const int* __restrict__ first, int numat, int k, bool heavy) {
+// The k-th (from 0) atom of numat that has four orbitals (heavy) or one: cum
+// counts ten pairs or one, so cum[a] - a is nine times the heavy atoms below a.
+__device__ __forceinline__ int kth_atom(const int* __restrict__ cum, int numat, int k, bool heavy) {
   int lo = 0, hi = numat - 1;  // the largest a with at most k of the kind below it
   while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1, nh = (first[mid] - mid) / 3;
+    const int mid = (lo + hi + 1) >> 1, nh = (cum[mid] - mid) / 9;
     if ((heavy ? nh : mid - nh) <= k) lo = mid; else hi = mid - 1;
   }
   return lo;
@@ -1151,7 +1151,7 @@ __global__ void __launch_bounds__(KIND == 0 ? 32 : 128) dcart_pairs(int numat, c
   if (threadIdx.x < 9) z3[threadIdx.x] = pow((double)threadIdx.x, 0.3333);
   __syncthreads();
   const double chnge = 1.0e-4, chnge2 = chnge * 0.5;
-  const long long nh = (at.first[numat - 1] + at.nor[numat - 1] - numat) / 3, nl = numat - nh;
+  const long long nh = (at.cum[numat - 1] + at.lim[numat - 1] - numat) / 9, nl = numat - nh;
   const long long count = KIND == 0 ? nh * (nh - 1) / 2 : KIND == 1 ? nh * nl : nl * (nl - 1) / 2;
   const int geo = threadIdx.x & 3;
   // whole warps iterate, for the shuffle: lanes past the end repeat the last pair
@@ -1162,13 +1162,13 @@ __global__ void __launch_bounds__(KIND == 0 ? 32 : 128) dcart_pairs(int numat, c
     if (!live) t = count - 1;
     int ii, jj;
     if (KIND == 1) {
-      const int a = kth_atom(at.first, numat, (int)(t / nl), true), b = kth_atom(at.first, numat, (int)(t % nl), false);
+      const int a = kth_atom(at.cum, numat, (int)(t / nl), true), b = kth_atom(at.cum, numat, (int)(t % nl), false);
       ii = a > b ? a : b;
       jj = a > b ? b : a;
     } else {
       pair_of(t, &ii, &jj);
-      ii = kth_atom(at.first, numat, ii, KIND == 0);
-      jj = kth_atom(at.first, numat, jj, KIND == 0);
+      ii = kth_atom(at.cum, numat, ii, KIND == 0);
+      jj = kth_atom(at.cum, numat, jj, KIND == 0);
     }
     const int n1 = nat[jj], n2 = nat[ii];
     const double zz = z3[n2] + z3[n1];
