@@ -256,7 +256,8 @@ __device__ __forceinline__ void tri_forward(int n, const double2* __restrict__ d
         const long long o = (long long)i * ld;
         if (FACTOR) {
           const double dn = tb[u].x - lam, en = i + 1 < n - 1 ? tb[u].y : 0.0, xv = rnd();
-          const bool swap = fabs(dd) < fabs(sub);
+          // a coupling below tiny is rounding of T: a row exchange would divide by it
+          const bool swap = fabs(dd) < fabs(sub) && fabs(sub) >= tiny;
           const double piv = fabs(dd) < tiny ? copysign(tiny, dd) : dd;
           const double rd = recip_nr2(piv), rs = recip_nr2(swap ? sub : 1.0);
           const double l = swap ? dd * rs : sub * rd;

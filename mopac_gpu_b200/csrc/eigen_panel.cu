@@ -668,8 +668,9 @@ __device__ void tri_solve(int n, const double* __restrict__ d, const double* __r
       const double dn = dnb[u] - lam;    // T(i+1, i+1)
       const double en = enb[u];
       const double xn = xnb[u];
-      if (fabs(dd) >= fabs(sub)) {
-        // no interchange
+      if (fabs(dd) >= fabs(sub) || fabs(sub) < tiny) {
+        // no interchange; never for a coupling below tiny, which is rounding of T
+        // (the exchange would divide by it)
         double piv_ = dd;
         if (fabs(piv_) < tiny) piv_ = copysign(tiny, piv_ == 0.0 ? 1.0 : piv_);
         const double l = sub / piv_;
