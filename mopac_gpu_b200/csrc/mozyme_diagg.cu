@@ -473,9 +473,12 @@ __global__ void __launch_bounds__(OE_T + 32) mzd_occ_energy(MbMzLayout L, MbMzLm
       if (prev == 1) {
 #pragma unroll 8
         for (int k = 0; k < n; ++k) sum = DADD(sum, t[k][0]);
-      } else {
+      } else if (prev == 4) {
 #pragma unroll 4
         for (int k = 0; k < n; ++k) sum = DADD(DADD(DADD(DADD(sum, t[k][0]), t[k][1]), t[k][2]), t[k][3]);
+      } else {
+        for (int k = 0; k < n; ++k)
+          for (int jx = 0; jx < prev; ++jx) sum = DADD(sum, t[k][jx]);
       }
     }
   };
