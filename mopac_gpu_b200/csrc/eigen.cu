@@ -526,7 +526,7 @@ template <int K>
 int launch_back_small(int n, const double* V, const double* tau, const double* X, const double* inv, double* c,
                       cudaStream_t stream) {
   const size_t smem = sizeof(double) * BS_STAGES * BS_REF * 32 * K;
-  MB_CUDA(cudaFuncSetAttribute(back_small<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MB_TRY(mb_smem_optin((const void*)back_small<K>, smem));
   const int per = 2 * (BS_T / 32);
   back_small<K><<<(n + per - 1) / per, BS_T, smem, stream>>>(n, V, tau, X, inv, c);
   MB_LAUNCH_CHECK();

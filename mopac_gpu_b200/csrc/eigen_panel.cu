@@ -945,11 +945,7 @@ extern "C" int mb_eigh_back(int n, const eigh::Ws* w, double* c, cudaStream_t st
   const size_t nn = (size_t)n * n;
   double *V = w->V, *Z = w->Z, *X = w->X, *U0 = w->U0, *S = w->S, *Tm = w->Tm, *Y = w->Y;
   const double* tau = w->tau;
-  static bool larft_attr = false;
-  if (!larft_attr) {
-    MB_CUDA(cudaFuncSetAttribute(larft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LARFT_SMEM));
-    larft_attr = true;
-  }
+  MB_TRY(mb_smem_optin((const void*)larft_kernel, LARFT_SMEM));
   const int nref = n - 1;  // reflectors 0 .. n-2
   const int last_k = ((nref - 1) / BT) * BT;
   const int nblk = last_k / BT + 1;

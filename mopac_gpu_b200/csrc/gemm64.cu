@@ -327,17 +327,10 @@ int dmma_tile(long long tiles128, long long tiles64) {
 
 bool dmma_pairs(const double* x, int ld) { return ((uintptr_t)x & 15) == 0 && ld % 2 == 0; }
 
-// A kernel's opt-in to its shared memory, which its launcher takes once per process.
-int dmma_attr(const void* fn, int smem) {
-  MB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  return MB_OK;
-}
-
 template <int TILE, bool TA, bool TB, int V>
 int dmma_launch(int m, int n, int k, int nz, double alpha, const double* a, int lda, const double* b, int ldb,
                 double beta, double* out, int ldc, cudaStream_t stream) {
-  static int attr = dmma_attr((const void*)dgemm_dmma_kernel<TILE, TA, TB, V>, Dmma<TILE>::SMEM);
-  if (attr != MB_OK) return attr;
+  MB_TRY(mb_smem_optin((const void*)dgemm_dmma_kernel<TILE, TA, TB, V>, Dmma<TILE>::SMEM));
   const dim3 grid((n + TILE - 1) / TILE, (m + TILE - 1) / TILE, nz);
   dgemm_dmma_kernel<TILE, TA, TB, V><<<grid, Dmma<TILE>::THREADS, Dmma<TILE>::SMEM, stream>>>(m, n, k, alpha, a, lda, b,
                                                                                               ldb, beta, out, ldc);
@@ -363,8 +356,7 @@ int dmma_gemm(int m, int n, int k, int nz, double alpha, const double* a, int ld
 
 template <int TILE, int V>
 int syrk_launch(int n, int k, double alpha, const double* a, int lda, double* p, int acc, cudaStream_t stream) {
-  static int attr = dmma_attr((const void*)syrk_packed_dmma_kernel<TILE, V>, Dmma<TILE>::SMEM);
-  if (attr != MB_OK) return attr;
+  MB_TRY(mb_smem_optin((const void*)syrk_packed_dmma_kernel<TILE, V>, Dmma<TILE>::SMEM));
   const long long t = (n + TILE - 1) / TILE;
   syrk_packed_dmma_kernel<TILE, V>
       <<<(unsigned)(t * (t + 1) / 2), Dmma<TILE>::THREADS, Dmma<TILE>::SMEM, stream>>>(n, k, alpha, a, lda, p, acc);

@@ -1,7 +1,9 @@
 // Opt-in per-kernel-family timing with CUDA events recorded on the stream each
 // kernel is launched on.  Used by bench.py to time the dominant kernel inside
 // the timed region; off by default (no events recorded).
+#include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "mb_common.cuh"
@@ -81,4 +83,17 @@ cudaError_t mb_malloc_async(void** p, size_t bytes, cudaStream_t s) {
     }
   }
   return cudaMallocAsync(p, bytes, s);
+}
+
+int mb_smem_optin(const void* fn, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> limit;  // what each kernel has on each device
+  int dev = 0;
+  MB_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  size_t& have = limit[{dev, fn}];
+  if (have >= bytes) return MB_OK;
+  MB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  have = bytes;
+  return MB_OK;
 }

@@ -45,6 +45,12 @@ inline cudaError_t mb_malloc_async(T** p, size_t bytes, cudaStream_t s) {
   return mb_malloc_async((void**)p, bytes, s);
 }
 
+// Opts a kernel in to `bytes` of dynamic shared memory on the current device.
+// The limit belongs to the function, not to a launch, so it is only ever raised:
+// a caller on another thread, with a smaller order, cannot take it away between
+// this call and the launch.
+int mb_smem_optin(const void* fn, size_t bytes);
+
 #define MB_TRY(expr)            \
   do {                          \
     int _rc = (expr);           \

@@ -496,13 +496,12 @@ size_t flow_sync_ints(int n, int nocc) {
 int launch_wavefronts(int n, int nocc, int nvirt, double* c, const double* al, const double* be,
                       const unsigned char* act, const unsigned int* tcnt, int to, int tv, int* sync, int* err,
                       cudaStream_t stream) {
+  MB_TRY(mb_smem_optin((const void*)rot_sweep_kernel, sizeof(SweepShared)));
   static int grid = 0;
   if (grid == 0) {
     int dev = 0, sms = 0, per = 0;
     MB_CUDA(cudaGetDevice(&dev));
     MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MB_CUDA(cudaFuncSetAttribute(rot_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(SweepShared)));
     MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rot_sweep_kernel, 32 * SWARPS, sizeof(SweepShared)));
     if (per < 1) return mb_set_error(MB_ERR_CUDA, "rot_sweep_kernel: no CTA fits on an SM");
     grid = sms * per;
@@ -553,8 +552,8 @@ extern "C" int mb_cnvg_ws(int norbs, double* pnew, double* p, double* p1, int ni
   size_t sh = sizeof(double) * 2 * (size_t)norbs;
   if (sh > 200 * 1024) return mb_set_error(MB_ERR_ARG, "mb_cnvg: norbs too large for one CTA");
   if (sh > 48 * 1024) {
-    MB_CUDA(cudaFuncSetAttribute(cnvg_diag1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
-    MB_CUDA(cudaFuncSetAttribute(cnvg_diag2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+    MB_TRY(mb_smem_optin((const void*)cnvg_diag1, sh));
+    MB_TRY(mb_smem_optin((const void*)cnvg_diag2, sh));
   }
   cnvg_diag1<<<1, 1024, sh, stream>>>(norbs, pnew, p, p1, niter, st, sum1);
   MB_LAUNCH_CHECK();

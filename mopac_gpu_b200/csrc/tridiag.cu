@@ -624,7 +624,7 @@ extern "C" int mb_tridiag_grid(int m, int ctas, const double* a, long long lda, 
                            {(void*)tridiag_grid<1, 16>, (void*)tridiag_grid<2, 16>, (void*)tridiag_grid<3, 16>,
                             (void*)tridiag_grid<4, 16>}};
   void* fn = fns[(m + ctas - 1) / ctas > 8][gr - 1];
-  MB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  MB_TRY(mb_smem_optin(fn, smem));
   GridArgs g;
   g.m = m;
   g.a = a;
