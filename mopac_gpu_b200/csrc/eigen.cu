@@ -581,12 +581,9 @@ extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double
   } else {
     MB_TRY(mb_unpack_dev(n, fpacked, w.A, n, perturb, fpacked, stream));
     MB_CUDA(cudaMemsetAsync(w.V, 0, sizeof(double) * nn, stream));
-    static int sms = 0;
-    if (sms == 0) {
-      int dev = 0;
-      MB_CUDA(cudaGetDevice(&dev));
-      MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    }
+    int dev = 0, sms = 0;
+    MB_CUDA(cudaGetDevice(&dev));
+    MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int k = 0;
     MB_TRY(mb_eigh_panels(n, n - mb_tridiag_grid_max(sms), &w, stream, &k));
     const size_t o = (size_t)k * n + k;

@@ -13,6 +13,8 @@
 // order of operations keeps the result of such an SCF what it was.
 #include <cooperative_groups.h>
 
+#include <mutex>
+
 #include "eigen_ws.cuh"
 #include "mb_common.cuh"
 
@@ -875,6 +877,30 @@ __global__ void larft_kernel(int nref, const double* __restrict__ Sall, const do
   }
 }
 
+struct PanelGrid {
+  int sms, per1, per2;  // SMs; CTAs an SM of the two panel forms
+};
+
+int panel_grid(PanelGrid* out) {
+  static std::mutex mu;
+  static PanelGrid g = {0, 0, 0};
+  std::lock_guard<std::mutex> lock(mu);
+  if (g.per1 == 0) {
+    PanelGrid t;
+    int dev = 0;
+    MB_CUDA(cudaGetDevice(&dev));
+    MB_CUDA(cudaDeviceGetAttribute(&t.sms, cudaDevAttrMultiProcessorCount, dev));
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t.per2, tridiag_panel2, TPB, 0));
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t.per1, tridiag_panel, TPB, 0));
+    if (t.per2 > 3) t.per2 = 3;  // wider grids cost more per barrier than they add in bandwidth
+    if (t.per1 > 4) t.per1 = 4;
+    if (t.per1 < 1) return mb_set_error(MB_ERR_CUDA, "tridiag_panel: cannot be co-resident");
+    g = t;
+  }
+  *out = g;
+  return MB_OK;
+}
+
 }  // namespace
 
 extern "C" int mb_dgemm_ws(char transa, char transb, int m, int n, int k, double alpha, const double* a, int lda,
@@ -894,19 +920,10 @@ extern "C" int mb_eigh_panels(int n, int cols, const eigh::Ws* w, cudaStream_t s
   double* wp = vwv + (size_t)n * NB;
   // cooperative grid size: co-resident CTAs of the panel form in use; the
   // second needs an 8-lane group for every row
-  static int sms = 0, per1 = 0, per2 = 0;
-  if (per1 == 0) {
-    int dev = 0;
-    MB_CUDA(cudaGetDevice(&dev));
-    MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, tridiag_panel2, TPB, 0));
-    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, tridiag_panel, TPB, 0));
-    if (per2 > 3) per2 = 3;  // wider grids cost more per barrier than they add in bandwidth
-    if (per1 > 4) per1 = 4;
-    if (per1 < 1) return mb_set_error(MB_ERR_CUDA, "tridiag_panel: cannot be co-resident");
-  }
-  const bool v2 = per2 >= 1 && (long long)sms * per2 * TPB / 8 >= n;
-  int grid = sms * (v2 ? per2 : per1);
+  PanelGrid pg;
+  MB_TRY(panel_grid(&pg));
+  const bool v2 = pg.per2 >= 1 && (long long)pg.sms * pg.per2 * TPB / 8 >= n;
+  int grid = pg.sms * (v2 ? pg.per2 : pg.per1);
   if (grid > 1024) grid = 1024;
   int k = 0;
   while (k < cols) {

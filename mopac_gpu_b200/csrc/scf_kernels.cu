@@ -8,6 +8,8 @@
 //            ordered 2x2 rotation sweep over the columns of C.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "mb_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -497,14 +499,15 @@ int launch_wavefronts(int n, int nocc, int nvirt, double* c, const double* al, c
                       const unsigned char* act, const unsigned int* tcnt, int to, int tv, int* sync, int* err,
                       cudaStream_t stream) {
   MB_TRY(mb_smem_optin((const void*)rot_sweep_kernel, sizeof(SweepShared)));
-  static int grid = 0;
+  static std::atomic<int> resident{0};  // threads that come first together store the same value
+  int grid = resident.load();
   if (grid == 0) {
     int dev = 0, sms = 0, per = 0;
     MB_CUDA(cudaGetDevice(&dev));
     MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, rot_sweep_kernel, 32 * SWARPS, sizeof(SweepShared)));
     if (per < 1) return mb_set_error(MB_ERR_CUDA, "rot_sweep_kernel: no CTA fits on an SM");
-    grid = sms * per;
+    resident.store(grid = sms * per);
   }
   (void)act;  // skipped pairs carry the identity rotation in al / be
   MB_CUDA(cudaMemsetAsync(sync, 0, sizeof(int) * flow_sync_ints(n, nocc), stream));

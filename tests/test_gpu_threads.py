@@ -61,3 +61,44 @@ def test_two_threads_with_orders_of_different_shared_memory():
     for r, (d, e) in zip(both, alone):
         assert int(r.status.item()) == 0
         assert torch.equal(r.d, d) and torch.equal(r.e[:-1], e[:-1])
+
+
+FIRST = """
+import sys, threading, numpy as np, torch
+from mopac_gpu_b200 import workloads
+from mopac_gpu_b200.scf import ScfContext
+done, bad = [], []
+start = threading.Barrier(4)
+def work(k):
+    try:
+        ctx = ScfContext(*workloads.water_lattice(24))
+        ctx.hcore()
+        start.wait()
+        r = ctx.run(pseudo=True, pulay=bool(k & 1))
+        done.append((k & 1, r.escf, ctx.density().tobytes()))
+        ctx.close()
+    except Exception as e:
+        bad.append(repr(e))
+threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+assert not bad, bad
+for kind in (0, 1):
+    a, b = [d[1:] for d in done if d[0] == kind]
+    assert a == b
+print("same", len(done))
+"""
+
+
+def test_contexts_that_come_first_together():
+    """Four threads whose contexts run the process's first SCFs: what a kernel's
+    launcher finds out once (grid sizes, limits) is whole for every one of them."""
+    import os
+    import subprocess
+    import sys
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", FIRST], capture_output=True, text=True, timeout=300, cwd=root)
+    assert out.returncode == 0, out.stderr[-2000:]
+    assert "same 4" in out.stdout
