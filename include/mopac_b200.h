@@ -580,12 +580,13 @@ int mb_density_occ_dev(int n, int ndubl, int nsingl, double occ, double fract, i
 /* Full eigensolve of a packed symmetric matrix after adding i*1e-10 to
  * diagonal element i (eigenvectors_LAPACK.F90:53-55; the packed input is
  * modified like the reference's xmat).  Ascending eigenvalues, vectors in
- * columns.  Returns MB_ERR_NUMERIC if the solver fails. */
+ * columns.  Returns MB_ERR_NUMERIC if the inverse iteration fails,
+ * MB_ERR_TIMEOUT if a bounded wait of the reduction gave up. */
 int mb_eigh_packed_dev(int n, double* fpacked, double* c, double* eigs, cudaStream_t stream);
 /* The same with a caller-owned workspace (mb_eigh_ws_bytes(n) bytes, 256-byte
  * aligned) and no host synchronisation: perturb = 1 adds the i*1e-10
- * diagonal; *status_dev (device int) is set nonzero if inverse iteration
- * fails. */
+ * diagonal; *status_dev (device int) is set to MB_OK or to the first failure's
+ * code, as above. */
 size_t mb_eigh_ws_bytes(int n);
 int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
                cudaStream_t stream);

@@ -27,6 +27,7 @@ extern "C" int mb_unpack_dev(int n, const double* pk, double* a, int lda, int pe
 extern "C" int mb_dgemm_ws(char transa, char transb, int m, int n, int k, double alpha, const double* a, int lda,
                            const double* b, int ldb, double beta, double* c, int ldc, double* ws, size_t ws_elems,
                            cudaStream_t stream);
+extern "C" int mb_eigh_status(int status);
 extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
                           cudaStream_t stream);
 
@@ -451,7 +452,7 @@ extern "C" int mb_campking_interp(mb_campking* ck, int np_, int mode, double e, 
       int st = 0;
       MB_CUDA(cudaMemcpyAsync(&st, status, sizeof(int), cudaMemcpyDeviceToHost, s));
       MB_CUDA(cudaStreamSynchronize(s));
-      if (st != 0) return mb_set_error(MB_ERR_NUMERIC, "Camp-King: eigensolver failed (inverse iteration)");
+      MB_TRY(mb_eigh_status(st));
     }
     // :156-174  descending order, rotation angles
     reverse_eigen<<<grid, 256, 0, s>>>(np_, m, ck->w, ck->vecl, ck->theta, VEC, n);

@@ -15,6 +15,7 @@
 
 #include "mb_common.cuh"
 
+extern "C" int mb_eigh_status(int status);
 extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
                           cudaStream_t stream);
 extern "C" size_t mb_eigh_ws_bytes(int n);
@@ -167,7 +168,7 @@ int eigh_host(int n, const double* A_upper, int lda, double* vecs, int ldv, doub
   if (fpacked_host && perturb)
     MB_CUDA(cudaMemcpyAsync(fpacked_host, pk, sizeof(double) * mp, cudaMemcpyDeviceToHost, g_stream));
   MB_CUDA(cudaStreamSynchronize(g_stream));
-  if (hst != 0) return mb_set_error(MB_ERR_NUMERIC, "eigensolver: inverse iteration failed");
+  MB_TRY(mb_eigh_status(hst));
   return MB_OK;
 }
 

@@ -377,6 +377,7 @@ __global__ void inverse_iteration(int n, const double2* __restrict__ dv, const d
                                   TriLu lu, int* status) {
   const int m0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (m0 >= n) return;
+  if (*status == MB_ERR_TIMEOUT) return;  // the reduction gave up: T is not whole
   const double tnorm = bnd[3];
   const double ortol = 1.0e-8 * tnorm;
   if (m0 > 0 && !(w[m0] - w[m0 - 1] > ortol)) return;  // not a cluster start
@@ -404,7 +405,7 @@ __global__ void inverse_iteration(int n, const double2* __restrict__ dv, const d
       else tri_forward<false>(n, dv, lam, tiny, f, x, scale, 0);
       double sq;
       const double mx = tri_back(n, f, x, &sq);
-      if (!(mx > 0.0) || !isfinite(sq)) { atomicExch(status, MB_ERR_NUMERIC); return; }
+      if (!(mx > 0.0) || !isfinite(sq)) { atomicCAS(status, MB_OK, MB_ERR_NUMERIC); return; }
       if (m1 - m0 == 1) {
         scale = 1.0 / mx;
         inv[m] = 1.0 / sqrt(sq);
@@ -418,7 +419,7 @@ __global__ void inverse_iteration(int n, const double2* __restrict__ dv, const d
         for (int i = 0; i < n; ++i) x[(long long)i * ld] -= dt * y[(long long)i * ld];
       }
       const double nr = normalise(n, x, ld);
-      if (!(nr > 0.0) || !isfinite(nr)) { atomicExch(status, MB_ERR_NUMERIC); return; }
+      if (!(nr > 0.0) || !isfinite(nr)) { atomicCAS(status, MB_OK, MB_ERR_NUMERIC); return; }
       inv[m] = 1.0;
     }
   }
@@ -553,6 +554,12 @@ __global__ void transpose_kernel(int n, const double* __restrict__ X, const doub
 
 }  // namespace
 
+extern "C" int mb_eigh_status(int status) {
+  if (status == MB_OK) return MB_OK;
+  if (status == MB_ERR_TIMEOUT) return mb_set_error(MB_ERR_TIMEOUT, "eigensolver: a wait between CTAs gave up");
+  return mb_set_error(MB_ERR_NUMERIC, "eigensolver: inverse iteration failed");
+}
+
 extern "C" size_t mb_eigh_ws_bytes(int n) { return sizeof(double) * eigh::ws_doubles(n) + 256; }
 
 extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
@@ -624,7 +631,7 @@ extern "C" int mb_eigh_packed_dev(int n, double* fpacked, double* c, double* eig
     ce = cudaMemcpyAsync(&hst, st, sizeof(int), cudaMemcpyDeviceToHost, stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);
     if (ce != cudaSuccess) rc = mb_set_cuda_error(ce, "eigh status", __FILE__, __LINE__);
-    else if (hst != 0) rc = mb_set_error(MB_ERR_NUMERIC, "eigensolver: inverse iteration failed");
+    else rc = mb_eigh_status(hst);
   }
   cudaFree(ws);
   cudaFree(st);

@@ -58,6 +58,10 @@ inline Ws carve(int n, void* ws) {
 
 }  // namespace eigh
 
+// eigen.cu: the caller's return code for a solve's status word, with its message.
+// The word holds the first failure: MB_ERR_TIMEOUT (a bounded wait gave up) or
+// MB_ERR_NUMERIC.
+extern "C" int mb_eigh_status(int status);
 // eigen_panel.cu
 extern "C" int mb_eigh_panels(int n, int cols, const eigh::Ws* w, cudaStream_t stream, int* done);
 extern "C" int mb_eigh_back(int n, const eigh::Ws* w, double* c, cudaStream_t stream);

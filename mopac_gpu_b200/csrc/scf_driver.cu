@@ -26,6 +26,7 @@ extern "C" int mb_helect_ws(int n, const double* p, const double* h, const doubl
 extern "C" int mb_cnvg_ws(int norbs, double* pnew, double* p, double* p1, int niter, double* pl_out, double* ws,
                           cudaStream_t stream);
 extern "C" size_t mb_eigh_ws_bytes(int n);
+extern "C" int mb_eigh_status(int status);
 extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
                           cudaStream_t stream);
 extern "C" int mb_eigh_ordered_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws,
@@ -625,7 +626,7 @@ static int full_diag(mb_ctx* c, double* fpacked, double* eig_homo, double* eig_l
   MB_CUDA(cudaMemcpyAsync(hl, c->eigs + (ihomo - 1), sizeof(double) * (ihomo < n ? 2 : 1), cudaMemcpyDeviceToHost,
                           c->stream));
   MB_CUDA(cudaStreamSynchronize(c->stream));
-  if (st != 0) return mb_set_error(MB_ERR_NUMERIC, "eigensolver failed (inverse iteration)");
+  MB_TRY(mb_eigh_status(st));
   *eig_homo = hl[0];
   *eig_lumo = hl[1];
   return MB_OK;
@@ -703,6 +704,8 @@ static int exit_block_diag(mb_ctx* c, double* fpacked, double* eig_homo, double*
   double hl[2] = {0.0, 0.0};
   MB_CUDA(cudaMemcpyAsync(hl, c->eigs + (no - 1), sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
   MB_CUDA(cudaStreamSynchronize(s));
+  for (int q : st)
+    if (q == MB_ERR_TIMEOUT) return mb_eigh_status(q);  // not a reason to decline the split
   const double gap = hl[1] - hl[0];
   if (st[0] != 0 || st[1] != 0 || !(gap > 0.0) || !(b2 <= tol_ev * gap)) {
     mb_kstat_mark(MB_KSTAT_EIGH, s, false);

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(CT, 1) tridiag_cluster(ClusterArgs p) {
     if (lane == 0) ((double*)s_red[0])[warp] = pv;
     __syncthreads();
     if (!ONE && s_fail) {
-      if (tid == 0) atomicExch(p.status, MB_ERR_TIMEOUT);
+      if (tid == 0) atomicCAS(p.status, MB_OK, MB_ERR_TIMEOUT);
       break;
     }
     pv = sum_partials(s_red[0]);
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(GT, 1) tridiag_grid(GridArgs p) {
     if (lane == 0) s_red[0][warp] = pv;
     __syncthreads();
     if (s_fail) {
-      if (tid == 0) atomicExch(p.status, MB_ERR_TIMEOUT);
+      if (tid == 0) atomicCAS(p.status, MB_OK, MB_ERR_TIMEOUT);
       return;
     }
     pv = s_red[0][lane & (GW - 1)];
