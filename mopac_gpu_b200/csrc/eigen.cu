@@ -562,8 +562,9 @@ extern "C" int mb_eigh_status(int status) {
 
 extern "C" size_t mb_eigh_ws_bytes(int n) { return sizeof(double) * eigh::ws_doubles(n) + 256; }
 
-extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
-                          cudaStream_t stream) {
+// cluster_max: the largest order that the cluster kernel reduces.
+extern "C" int mb_eigh_cluster_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws,
+                                  int* status_dev, int cluster_max, cudaStream_t stream) {
   const size_t nn = (size_t)n * n;
   const eigh::Ws w = eigh::carve(n, ws);
   MB_CUDA(cudaMemsetAsync(status_dev, 0, sizeof(int), stream));
@@ -580,7 +581,7 @@ extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double
   double* inv = w.wvec;  // the eigenvectors' norms, after the panels have used it
   double* weig = w.e2;   // eigenvalues of the scaled T
   // one launch up to the order whose columns fit in the registers of 16 CTAs
-  const bool small = n <= mb_tridiag_cluster_max();
+  const bool small = n <= cluster_max;
   if (small) {
     mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, true);
     MB_TRY(mb_tridiag_cluster(n, fpacked, perturb, w.V, w.d, w.e, w.tau, status_dev, stream));
@@ -616,6 +617,11 @@ extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double
   transpose_kernel<<<g, blk, 0, stream>>>(n, w.X, inv, w.Z);
   MB_LAUNCH_CHECK();
   return mb_eigh_back(n, &w, c, stream);
+}
+
+extern "C" int mb_eigh_ws(int n, double* fpacked, int perturb, double* c, double* eigs, void* ws, int* status_dev,
+                          cudaStream_t stream) {
+  return mb_eigh_cluster_ws(n, fpacked, perturb, c, eigs, ws, status_dev, mb_tridiag_cluster_max(), stream);
 }
 
 extern "C" int mb_eigh_packed_dev(int n, double* fpacked, double* c, double* eigs, cudaStream_t stream) {

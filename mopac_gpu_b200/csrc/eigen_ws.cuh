@@ -66,6 +66,7 @@ extern "C" int mb_eigh_status(int status);
 extern "C" int mb_eigh_panels(int n, int cols, const eigh::Ws* w, cudaStream_t stream, int* done);
 extern "C" int mb_eigh_back(int n, const eigh::Ws* w, double* c, cudaStream_t stream);
 // tridiag.cu
+extern "C" int mb_tridiag_cluster_orders(int clusters16);
 extern "C" int mb_tridiag_cluster_max(void);
 extern "C" int mb_tridiag_cluster(int n, double* pk, int perturb, double* vall, double* d, double* e, double* tau,
                                   int* status, cudaStream_t stream);

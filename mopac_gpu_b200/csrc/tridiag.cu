@@ -33,6 +33,9 @@
 // 608 in 1.4.
 #include <cooperative_groups.h>
 
+#include <map>
+#include <mutex>
+
 #include "mb_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -563,8 +566,38 @@ __global__ void __launch_bounds__(GT, 1) tridiag_grid(GridArgs p) {
 // Shared memory of a CTA of the grid kernel; its static part is below 4 KB.
 static const size_t kMaxSmem = 232448;
 
-// Orders the cluster kernel takes.
-extern "C" int mb_tridiag_cluster_max(void) { return 608; }
+// Orders the cluster kernel takes on a device that can (or cannot) hold a cluster of
+// 16 CTAs, which is beyond the portable size of 8.
+extern "C" int mb_tridiag_cluster_orders(int clusters16) { return clusters16 > 0 ? 608 : 320; }
+
+// The same on the current device; asked once per device.
+extern "C" int mb_tridiag_cluster_max(void) {
+  static std::mutex mu;
+  static std::map<int, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return mb_tridiag_cluster_orders(0);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(16);
+  cfg.blockDim = dim3(CT);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 16;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const void* fn = (const void*)tridiag_cluster<19, 5, false>;
+  int count = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&count, fn, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    count = 0;
+  }
+  return known[dev] = mb_tridiag_cluster_orders(count);
+}
 
 extern "C" int mb_tridiag_cluster(int n, double* pk, int perturb, double* vall, double* d, double* e, double* tau,
                                   int* status, cudaStream_t stream) {
@@ -575,7 +608,6 @@ extern "C" int mb_tridiag_cluster(int n, double* pk, int perturb, double* vall, 
              : n <= 160 ? (void*)tridiag_cluster<5, 5, false>
              : n <= 320 ? (void*)tridiag_cluster<10, 5, false>
                         : (void*)tridiag_cluster<19, 5, false>;
-  if (cs > 8) MB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   ClusterArgs a{n, perturb, pk, vall, d, e, tau, status};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs);
