@@ -325,6 +325,19 @@ int dmma_tile(long long tiles128, long long tiles64) {
   return t64 <= t128 ? 64 : 128;
 }
 
+// The tile of an m x n product in nz slices of k, and of a packed SYRK of order n.
+int gemm_tile(int m, int n, int nz) {
+  auto tiles = [&](int t) { return (long long)nz * ((m + t - 1) / t) * ((n + t - 1) / t); };
+  return dmma_tile(tiles(128), tiles(64));
+}
+int syrk_tile(int n) {
+  auto tiles = [&](int t) {
+    const long long q = (n + t - 1) / t;
+    return q * (q + 1) / 2;
+  };
+  return dmma_tile(tiles(128), tiles(64));
+}
+
 bool dmma_pairs(const double* x, int ld) { return ((uintptr_t)x & 15) == 0 && ld % 2 == 0; }
 
 template <int TILE, bool TA, bool TB, int V>
@@ -341,8 +354,7 @@ int dmma_launch(int m, int n, int k, int nz, double alpha, const double* a, int 
 template <bool TA, bool TB>
 int dmma_gemm(int m, int n, int k, int nz, double alpha, const double* a, int lda, const double* b, int ldb,
               double beta, double* out, int ldc, cudaStream_t stream) {
-  auto tiles = [&](int t) { return (long long)nz * ((m + t - 1) / t) * ((n + t - 1) / t); };
-  const bool small = dmma_tile(tiles(128), tiles(64)) == 64;
+  const bool small = gemm_tile(m, n, nz) == 64;
   // a slice starts at an even k, or its pairs along k are off their boundary
   const bool even = nz == 1 || (k + nz - 1) / nz % 2 == 0;
   const bool pairs = even && dmma_pairs(a, lda) && dmma_pairs(b, ldb);
@@ -365,11 +377,7 @@ int syrk_launch(int n, int k, double alpha, const double* a, int lda, double* p,
 }
 
 int dmma_syrk(int n, int k, double alpha, const double* a, int lda, double* p, int acc, cudaStream_t stream) {
-  auto tiles = [&](int t) {
-    const long long q = (n + t - 1) / t;
-    return q * (q + 1) / 2;
-  };
-  const bool small = dmma_tile(tiles(128), tiles(64)) == 64, pairs = dmma_pairs(a, lda);
+  const bool small = syrk_tile(n) == 64, pairs = dmma_pairs(a, lda);
   if (small) return pairs ? syrk_launch<64, 2>(n, k, alpha, a, lda, p, acc, stream)
                           : syrk_launch<64, 1>(n, k, alpha, a, lda, p, acc, stream);
   return pairs ? syrk_launch<128, 2>(n, k, alpha, a, lda, p, acc, stream)
@@ -418,7 +426,34 @@ __global__ void add_diag_kernel(int n, double cst, double* __restrict__ p) {
   if (i < n) p[mb_tri(i, i)] = cst + p[mb_tri(i, i)];
 }
 
+// DMMA engine for all but skinny outputs.
+bool gemm_wide(int m, int n) { return m > BM && n > BN; }
+
+// Slices of k, counted in 128- or 64-wide tiles, whatever tile then runs: the sums'
+// order stays the same.
+int gemm_slices(int m, int n, int k, size_t ws_elems) {
+  const bool wide = gemm_wide(m, n);
+  const int t = wide ? 128 : BM;
+  const int tiles = ((n + t - 1) / t) * ((m + t - 1) / t);
+  const int target = wide ? 148 : 296;
+  int nz = 1;
+  if (k >= 512 && tiles < target) {
+    nz = (target + tiles - 1) / tiles;
+    if (nz > k / 128) nz = k / 128;
+    if (nz > 32) nz = 32;
+    while (nz > 1 && (size_t)nz * m * n > ws_elems) --nz;
+  }
+  return nz;
+}
+
 }  // namespace
+
+// Which tile a product takes, given the elements of its workspace (0: none), and a
+// packed SYRK: 64 or 128, 0 for the FFMA engine.
+extern "C" int mb_dgemm_tile(int m, int n, int k, size_t ws_elems) {
+  return gemm_wide(m, n) ? gemm_tile(m, n, gemm_slices(m, n, k, ws_elems)) : 0;
+}
+extern "C" int mb_syrk_tile(int n) { return n > BM ? syrk_tile(n) : 0; }
 
 // GEMM with optional split-K: when the output has too few 64x64 tiles to fill
 // the GPU and k is long, the k loop is cut into slices whose partial sums go to
@@ -430,19 +465,8 @@ extern "C" int mb_dgemm_ws(char transa, char transb, int m, int n, int k, double
   if (m == 0 || n == 0) return MB_OK;
   bool ta = (transa == 'T' || transa == 't' || transa == 'C' || transa == 'c');
   bool tb = (transb == 'T' || transb == 't' || transb == 'C' || transb == 'c');
-  const bool wide = m > BM && n > BN;  // DMMA engine for all but skinny outputs
-  // slices of k are counted in 128- or 64-wide tiles, whatever tile then runs:
-  // the sums' order stays the same
-  const int tb_ = wide ? 128 : BM;
-  const int tiles = ((n + tb_ - 1) / tb_) * ((m + tb_ - 1) / tb_);
-  const int target = wide ? 148 : 296;
-  int nz = 1;
-  if (ws && k >= 512 && tiles < target) {
-    nz = (target + tiles - 1) / tiles;
-    if (nz > k / 128) nz = k / 128;
-    if (nz > 32) nz = 32;
-    while (nz > 1 && (size_t)nz * m * n > ws_elems) --nz;
-  }
+  const bool wide = gemm_wide(m, n);
+  const int nz = ws ? gemm_slices(m, n, k, ws_elems) : 1;
   double* out = nz > 1 ? ws : c;
   if (wide) {
     if (!ta && !tb) MB_TRY((dmma_gemm<false, false>(m, n, k, nz, alpha, a, lda, b, ldb, beta, out, ldc, stream)));
