@@ -529,7 +529,7 @@ def run_mine(args):
     # ---- timed region (device-resident inputs)
     clocks = ClockSampler(local)
     barrier()
-    for kid in range(5):  # drop anything recorded before the timed region
+    for kid in range(len(KSTATS)):  # drop anything recorded before the timed region
         L.mb_kstats_read(kid, None, None)
     L.mb_kstats_enable(1)
     clocks.start()
@@ -547,7 +547,7 @@ def run_mine(args):
     clk = clocks.stop()
     L.mb_kstats_enable(0)
     kst = {}
-    for kid, name in enumerate(["tridiag_panel", "fock2", "density", "eigensolve", "pseudo_diag"]):
+    for kid, name in enumerate(KSTATS):
         cnt, tot = ctypes.c_longlong(0), ctypes.c_double(0.0)
         L.mb_kstats_read(kid, ctypes.byref(cnt), ctypes.byref(tot))
         kst[name] = {"launches": cnt.value, "total_ms": tot.value}
@@ -580,7 +580,10 @@ def run_mine(args):
                "d2h_bytes_per_step": 8 * ctx.mpack, "scf_wall_s": te}
     # ---- rooflines: the dominant kernel (Householder panel) from the events
     # recorded on its stream inside the timed region, and the Fock build
-    roof = panel_roofline(ctx, kst, eigh_sizes(ctx, results))
+    reduced = reductions(ctx, results, pseudo)
+    panelled = [(m, cols) for m, cols in reduced if cols > 0]
+    roof = panel_roofline(ctx, kst, [m for m, _ in panelled], [cols for _, cols in panelled])
+    roof_onchip = onchip_reduction(kst, [m - cols for m, cols in reduced if m - cols > 1])
     roof_fock = fock_roofline(ctx)
     # ---- the plain FP64 GPU path on the same input (reference point of the
     # metric) and |dHf| of the timed SCF against FP64
@@ -683,6 +686,7 @@ def run_mine(args):
             "clocks": clk,
             "roofline": roof,
             "roofline_fock": roof_fock,
+            "onchip_reduction": roof_onchip,
             "kernel_ms": {k: v["total_ms"] / max(1, args.steps) for k, v in kst.items()},
             "cpu_baseline": cpu,
             "parity_vs_oracle": parity,
@@ -717,32 +721,76 @@ def eigh_sizes(ctx, results):
     return sizes
 
 
-def panel_roofline(ctx, kst, sizes):
-    """Householder reduction: each reduced column reads its trailing matrix
-    once for p = A22 v, 8*(m-j-1)^2 bytes for an eigensolve of order m; summed
-    over the columns of every eigensolve of the timed region (sizes) and
-    divided by the reduction kernels' total time there.  launches_expected
-    counts panels of 32 columns; a reduction that ends in shared memory or
-    registers (order 2048 and below) takes the rest in one launch."""
+# Kernel families of mb_kstats_read, by id.
+KSTATS = ["tridiag_panel", "fock2", "density", "eigensolve", "pseudo_diag", "tridiag_onchip"]
+# The largest order whose reduction stays on the chip (148 SMs); a larger one is
+# taken down to it in panels of 32 columns.
+ONCHIP_MAX, PANEL = 2048, 32
+
+
+def reductions(ctx, results, pseudo):
+    """(order, columns reduced in panels) of every Householder reduction of the
+    timed SCFs.  Pseudo-diagonalising and split-precision iterations take the
+    blocked solver, all panels; the exit diagonalisation never does."""
+    def entry(m):
+        return m, PANEL * max(0, -(-(m - ONCHIP_MAX) // PANEL))
+
+    n, no = ctx.norbs, ctx.nclose
+    out = []
+    for r in results:
+        loop = r.n_full_diag - (0 if r.exit_split else 1)
+        blocked = loop if pseudo else min(loop, r.n_split)
+        out += [(n, n - 1)] * blocked + [entry(n)] * (loop - blocked)
+        out += [entry(no), entry(n - no)] if r.exit_split else [entry(n)]
+    return out
+
+
+def panel_roofline(ctx, kst, sizes, columns=None):
+    """Householder panels: each reduced column reads its trailing matrix once
+    for p = A22 v, 8*(m-j-1)^2 bytes for an eigensolve of order m; summed over
+    the columns that eigensolves of orders `sizes` reduced in panels (columns;
+    all m - 1 of them by default) and divided by the panels' total time."""
     st = kst["tridiag_panel"]
     if st["launches"] == 0 or not sizes:
         return None
-    algo_total = sum(8.0 * (m - 1) * m * (2 * m - 1) / 6.0 for m in sizes)
-    panels = sum((m - 2) // 32 + 1 for m in sizes if m > 1)
+    columns = columns or [m - 1 for m in sizes]
+
+    def squares(m):  # 1 + 4 + ... + (m - 1)^2
+        return (m - 1) * m * (2 * m - 1) / 6.0
+
+    algo_total = sum(8.0 * (squares(m) - squares(m - c)) for m, c in zip(sizes, columns))
+    panels = sum((c - 1) // PANEL + 1 for c in columns if c > 0)
     ms = st["total_ms"] / st["launches"]
     peaks, src = _peaks()
     peak = peaks.get("hbm_gbs", 6650.0)
     ach = algo_total / (st["total_ms"] * 1e-3) / 1e9
     n = ctx.norbs
-    return {"kernel": "tridiag_panel, tridiag_grid, tridiag_cluster (Householder reduction: column updates, reflectors, p = A22 v)",
+    return {"kernel": "tridiag_panel (Householder panel: column updates, reflectors, p = A22 v)",
             "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
             "traffic": PANEL_DRAM_BYTES * (algo_total / st["launches"]) / PANEL_ALGO_BYTES_3072,
             "ms_per_launch": ms, "algorithmic_bytes": algo_total / st["launches"],
             "launches": st["launches"], "launches_expected": panels, "eigensolve_orders": sorted(set(sizes)),
             "peak_source": src,
-            "note": "algorithmic bytes: one read of the trailing matrix per column, over every eigensolve "
-                    f"of the timed region (orders {sorted(set(sizes))}); the matrix ({8 * n * n / 1e6:.0f} MB "
+            "note": "algorithmic bytes: one read of the trailing matrix per column, over every column reduced in "
+                    f"panels in the timed region (orders {sorted(set(sizes))}); the matrix ({8 * n * n / 1e6:.0f} MB "
                     "at the full order) is L2-resident, so DRAM traffic is far below it"}
+
+
+def onchip_reduction(kst, orders):
+    """Householder reductions that keep the matrix in registers (tridiag_cluster,
+    to order 608) or shared memory (tridiag_grid, to 2048): bound by the latency of
+    a column's chain, so the rate is columns and FP64 operations a second; the
+    memory sees one read of the matrix and one write of the reflectors."""
+    st = kst["tridiag_onchip"]
+    if st["launches"] == 0 or not orders:
+        return None
+    cols = sum(m - 1 for m in orders)
+    return {"kernel": "tridiag_grid, tridiag_cluster (Householder reduction on the chip)",
+            "bound": "latency of a column (exchange, two block sums, square root, division)",
+            "us_per_column": st["total_ms"] * 1e3 / cols,
+            "achieved": sum(4.0 * m ** 3 / 3.0 for m in orders) / (st["total_ms"] * 1e-3) / 1e12, "unit": "TFLOP/s",
+            "bytes_per_launch": sum(2 * 8.0 * m * m for m in orders) / len(orders),
+            "launches": st["launches"], "launches_expected": len(orders), "orders": sorted(set(orders))}
 
 
 # DRAM bytes (read + write) of the average tridiag_panel launch at n = 3072:

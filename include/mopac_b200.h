@@ -55,7 +55,8 @@ int mb_version(void);                 /* 10000*major + 100*minor + patch       *
 long long mb_launch_count(void);      /* kernels this library has launched     */
 /* Opt-in CUDA-event timing per kernel family, recorded on the launching
  * stream: 0 Householder panel, 1 Fock build, 2 density, 3 full eigensolve,
- * 4 pseudo-diagonalisation.  mb_kstats_read syncs, returns and clears id. */
+ * 4 pseudo-diagonalisation, 5 Householder reduction on the chip (registers of
+ * a cluster or the SMs' shared memory).  mb_kstats_read syncs, returns and clears id. */
 void mb_kstats_enable(int on);
 int mb_kstats_read(int id, long long* count, double* total_ms);
 const char* mb_last_error(void);      /* thread-local text of the last failure */

@@ -583,9 +583,9 @@ extern "C" int mb_eigh_cluster_ws(int n, double* fpacked, int perturb, double* c
   // one launch up to the order whose columns fit in the registers of 16 CTAs
   const bool small = n <= cluster_max;
   if (small) {
-    mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, true);
+    mb_kstat_mark(MB_KSTAT_ONCHIP, stream, true);
     MB_TRY(mb_tridiag_cluster(n, fpacked, perturb, w.V, w.d, w.e, w.tau, status_dev, stream));
-    mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, false);
+    mb_kstat_mark(MB_KSTAT_ONCHIP, stream, false);
   } else {
     MB_TRY(mb_unpack_dev(n, fpacked, w.A, n, perturb, fpacked, stream));
     MB_CUDA(cudaMemsetAsync(w.V, 0, sizeof(double) * nn, stream));
@@ -595,9 +595,9 @@ extern "C" int mb_eigh_cluster_ws(int n, double* fpacked, int perturb, double* c
     int k = 0;
     MB_TRY(mb_eigh_panels(n, n - mb_tridiag_grid_max(sms), &w, stream, &k));
     const size_t o = (size_t)k * n + k;
-    mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, true);
+    mb_kstat_mark(MB_KSTAT_ONCHIP, stream, true);
     MB_TRY(mb_tridiag_grid(n - k, sms, w.A + o, n, w.V + o, w.d + k, w.e + k, w.tau + k, w.U0, status_dev, stream));
-    mb_kstat_mark(MB_KSTAT_TRIDIAG, stream, false);
+    mb_kstat_mark(MB_KSTAT_ONCHIP, stream, false);
   }
   tri_bounds<<<1, 1024, 0, stream>>>(n, w.d, w.e, de, dv, w.bnd);
   MB_LAUNCH_CHECK();

@@ -32,6 +32,7 @@ void mb_count_launch();
 #define MB_KSTAT_DENSITY 2   // one packed SYRK (density) launch
 #define MB_KSTAT_EIGH 3      // one full eigensolve
 #define MB_KSTAT_PSEUDO 4    // one pseudo-diagonalisation
+#define MB_KSTAT_ONCHIP 5    // one tridiag_cluster or tridiag_grid launch
 #define MB_KSTAT_IDS 8
 void mb_kstat_mark(int id, cudaStream_t s, bool begin);
 
