@@ -973,9 +973,10 @@ extern "C" int mb_scf_run(mb_ctx* c, const mb_scf_opts* opts_in, mb_scf_result* 
       res->n_pulay++;
     }
     t_diag.start();
+    const bool pseudo = opts.pseudo && !(halfe || camkin);  // this SCF pseudo-diagonalises once newdg is set
     if (interpolated) {
       // the density of the interpolated vectors
-    } else if (newdg && opts.pseudo && !(halfe || camkin)) {
+    } else if (newdg && pseudo) {
       if (res->n_finish > 0 && !refreshed) {
         // the finish's rotation angles use the energies of the current vectors
         MB_TRY(mb_orbital_energies_ws(n, c->f, c->c, c->eigs, c->eig_ws, s));
@@ -991,7 +992,7 @@ extern "C" int mb_scf_run(mb_ctx* c, const mb_scf_opts* opts_in, mb_scf_result* 
       mb_kstat_mark(MB_KSTAT_PSEUDO, s, false);
       res->n_pseudo_diag++;
     } else {
-      MB_TRY(full_diag(c, c->f, &eig_homo, &eig_lumo, ihomo, 1, opts.pseudo != 0 || use_split));
+      MB_TRY(full_diag(c, c->f, &eig_homo, &eig_lumo, ihomo, 1, pseudo || use_split));
       res->n_full_diag++;
     }
     t_diag.stop();
