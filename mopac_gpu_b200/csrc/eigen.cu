@@ -4,9 +4,9 @@
 //
 //   1. i*1e-10 added to diagonal element i of the packed input (the
 //      reference's parity-critical perturbation, eigenvectors_LAPACK.F90:53-55).
-//   2. Householder tridiagonalisation.  Up to order 608 and up to 2048 the
-//      matrix stays in the registers of one cluster or in the SMs' shared
-//      memory (tridiag.cu).  A larger one is first taken down to that size
+//   2. Householder tridiagonalisation.  Up to order 608 (320 on a device without
+//      clusters of 16 CTAs) and up to 2048 the matrix stays in the registers of one
+//      cluster or in the SMs' shared memory (tridiag.cu).  A larger one is first taken down to that size
 //      in panels (eigen_panel.cu): a cooperative kernel forms 32 reflectors (two
 //      grid barriers per column), and the trailing matrix gets the rank-64
 //      update A -= V W^T + W V^T as FP64 GEMM.
@@ -21,10 +21,10 @@
 //      reflectors, Z -= V (T (V^T Z)), as FP64 GEMMs (eigen_panel.cu).
 // Eigenvalues ascend; eigenvectors are the columns of C.
 //
-// Whole eigensolve on the Fock matrix of a water lattice (ms, one B200),
-// against the blocked form of eigen_panel.cu: order 38 0.10 (0.57), 144 0.37
-// (2.15), 320 0.85 (4.6), 600 2.1 (9.4), 1026 6.8 (17.2), 1501 11.0 (26.6),
-// 2048 17.6 (39.0), 3072 48.7 (72.4).
+// Whole eigensolve on the Fock matrix of a water lattice (ms, one B200, medians of
+// nine in a caller's workspace), in brackets the blocked form of eigen_panel.cu on
+// the same box: order 38 0.10 (0.57), 144 0.36 (2.1), 320 0.84 (4.6), 600 2.1 (9.0),
+// 1026 6.4 (16.4), 1501 10.7 (25.7), 2048 17.1 (37.7), 3072 46.5 (69.5).
 #include "eigen_ws.cuh"
 #include "mb_common.cuh"
 

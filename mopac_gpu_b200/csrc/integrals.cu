@@ -1137,9 +1137,11 @@ __device__ __forceinline__ void pair_of(long long q, int* ii, int* jj) {
 // two heavy atoms (KIND 0), mixed (1; the light partners of a heavy atom in a
 // row), two light ones (2), so that the loops have constant lengths and the lanes
 // of a warp take the same branches.  The W block of two heavy atoms (100
-// numbers) is in shared memory, everything else in registers.  Bound by the FP64
-// pipe's latency, a few hundred square roots and quotients an energy, at 8 to 12
-// warps an SM.  (H2O)200, one B200: 0.25 ms; a thread per pair, with the kinds mixed
+// numbers) is in shared memory.  The rest is in registers, of which two heavy atoms
+// take all 255 and spill (1.1 KB of stores and 1.2 of loads a thread); the other
+// kinds do not (149 and 80).  Bound by the FP64 pipe's latency, a few hundred square
+// roots and quotients an energy, at 8, 11 and 18 warps an SM.  (H2O)200, one B200:
+// 0.25 ms; a thread per pair, with the kinds mixed
 // in a warp and the arrays in local memory, took 3.4, that split by kind and
 // geometry alone 1.0.
 template <int KIND>
