@@ -228,7 +228,8 @@ int mb_dcart_dev(const int* nat_d, const double* coord_d, const MbAtomsDev* at, 
                  const double* p, double* dxyz_dev, void* ws, size_t ws_bytes, cudaStream_t stream);
 
 /* --------------------------------------------- device-pointer kernels */
-/* Atom layout on the device from host nfirst/nlast (1-based). */
+/* Atom layout on the device from host nfirst/nlast (1-based): one or four orbitals
+ * an atom, in ascending order; they need not begin at 1 and may leave gaps. */
 int mb_atoms_create(int numat, const int* nfirst, const int* nlast, MbAtomsDev* out);
 int mb_atoms_destroy(MbAtomsDev* atoms);
 
